@@ -13,7 +13,11 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libpenguin_b200.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVFLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2", "--expt-relaxed-constexpr"]
-SOURCES = ["pg_host.cpp", "pg_kernels.cu", "pg_kernels32.cu", "pg_run.cu", "pg_batch.cu", "pg_serve.cpp", "pg_noalloc.cu"]
+SOURCES = ["pg_host.cpp", "pg_kernels.cu", "pg_sweep.cu", "pg_run.cu", "pg_batch.cu", "pg_serve.cpp", "pg_noalloc.cu"]
+
+
+# the sweeps write their fused multiply-adds out (pg_warp.cuh)
+SOURCE_FLAGS = {"pg_sweep.cu": ["-fmad=false"]}
 
 
 def _newer(out, deps):
@@ -35,7 +39,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
         objs.append(o)
         if not force and _newer(o, [s] + headers):
             continue
-        cmd = ["nvcc", *ARCH, *NVFLAGS, "-c", s, "-o", o]
+        cmd = ["nvcc", *ARCH, *NVFLAGS, *SOURCE_FLAGS.get(src, []), "-c", s, "-o", o]
         if src.endswith(".cpp"):
             cmd = ["nvcc", "-x", "c++", *NVFLAGS, "-c", s, "-o", o]
         if verbose:

@@ -43,9 +43,9 @@ __global__ void kb_status(pgd::DevClock *const *clks, int n, pg_batch_member *ou
 struct Group {
   std::vector<pg_run *> members;
   pgd::BatchRun *d_runs = nullptr;
-  int *d_start = nullptr;          // [4][n+1]: radial tiles, azimuthal tiles, rings, short radial tiles
+  int *d_start = nullptr;          // [3][n+1]: radial tiles, azimuthal tiles, rings
   size_t cap = 0;
-  pgd::BatchQueue qx{}, qy{}, qr{}, qxs{};
+  pgd::BatchQueue qx{}, qy{}, qr{};
   pg_batch_shape shape{0, 0, 8, 0};
 };
 
@@ -114,11 +114,11 @@ static int rebuild(pg_batch *b) {
       g.d_start = nullptr;
       size_t cap = std::max<size_t>(n, 16);
       BK(cudaMalloc(&g.d_runs, cap * sizeof(pgd::BatchRun)));
-      BK(cudaMalloc(&g.d_start, 4 * (cap + 1) * sizeof(int)));
+      BK(cudaMalloc(&g.d_start, 3 * (cap + 1) * sizeof(int)));
       g.cap = cap;
     }
     std::vector<pgd::BatchRun> h(n);
-    std::vector<int> st(4 * (n + 1), 0);
+    std::vector<int> st(3 * (n + 1), 0);
     for (size_t i = 0; i < n; i++) {
       pg_run *r = g.members[i];
       if (int e = pgi::run_batch_desc(r, &h[i])) return bfail(b, e, pg_last_error(r));
@@ -127,7 +127,6 @@ static int rebuild(pg_batch *b) {
       st[i + 1] = st[i] + sh.tiles_x;
       st[(n + 1) + i + 1] = st[(n + 1) + i] + sh.tiles_y;
       st[2 * (n + 1) + i + 1] = st[2 * (n + 1) + i] + sh.nr;
-      st[3 * (n + 1) + i + 1] = st[3 * (n + 1) + i] + sh.tiles_xs;
     }
     if (n) {
       BK(cudaMemcpy(g.d_runs, h.data(), n * sizeof(pgd::BatchRun), cudaMemcpyHostToDevice));
@@ -137,7 +136,6 @@ static int rebuild(pg_batch *b) {
     g.qx = {g.d_runs, g.d_start, ni, st[n]};
     g.qy = {g.d_runs, g.d_start + (n + 1), ni, st[(n + 1) + n]};
     g.qr = {g.d_runs, g.d_start + 2 * (n + 1), ni, st[2 * (n + 1) + n]};
-    g.qxs = {g.d_runs, g.d_start + 3 * (n + 1), ni, st[3 * (n + 1) + n]};
   }
   size_t n = b->runs.size();
   if (n > b->status_cap) {
@@ -166,19 +164,17 @@ static void enqueue_group_step(pg_batch *b, int gi, int64_t *nk) {
   if (!n) return;
   pgk::batch_prestep(g.d_runs, n, s);
   if (gi == 1) {
-    pgk::batch_sweep_x32(g.qx, g.shape.grid_x, g.shape.minb, s);
-    pgk::batch_sweep_x32_short(g.qxs, s);
-    pgk::batch_sweep_y32(g.qy, g.shape.grid_y, g.shape.minb, s);
+    pgk::batch_sweep_x<float>(g.qx, g.shape.grid_x, s);
+    pgk::batch_sweep_y<float>(g.qy, g.shape.grid_y, s);
   } else {
-    pgk::batch_sweep_x(g.qx, g.shape.grid_x, g.shape.minb, s);
-    pgk::batch_sweep_x_short(g.qxs, s);
-    pgk::batch_sweep_y(g.qy, g.shape.grid_y, g.shape.minb, s);
+    pgk::batch_sweep_x<double>(g.qx, g.shape.grid_x, s);
+    pgk::batch_sweep_y<double>(g.qy, g.shape.grid_y, s);
   }
   pgk::batch_poststep(g.d_runs, n, s);
   pgk::batch_reduce(g.qr, gi, 0, s);
   pgk::batch_reduce(g.qr, gi, 9, s);
   pgk::batch_record(g.d_runs, n, s);
-  *nk += 8 + (g.qxs.total > 0 ? 1 : 0);
+  *nk += 7;
 }
 
 // one step of every member, on the batch stream
@@ -211,7 +207,6 @@ int pg_batch_create(int device, pg_batch **out) {
   if (cudaSetDevice(device) != cudaSuccess) return PG_ERR_CUDA;
   pg_batch *b = new pg_batch();
   b->dev = device;
-  b->g[1].shape.minb = 4;   // the FP32 sweeps keep ~80 registers
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&b->d_halted, sizeof(int)) != cudaSuccess ||
       cudaHostAlloc(&b->h_halted, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
@@ -400,8 +395,8 @@ int pg_batch_tune(pg_batch *b, int trial_steps) {
   for (int gi = 0; gi < 2 && rc == PG_OK; gi++) {
     Group &g = b->g[gi];
     if (g.members.empty()) continue;
-    // candidates: CTAs per SM the sweeps are compiled for, and one CTA per
-    // tile or a persistent grid of 1 or 2 waves walking the tile queue
+    // candidates: one CTA per tile, or a persistent grid of 1 or 2 times 8 or
+    // 4 CTAs per SM walking the tile queue
     std::vector<pg_batch_shape> cand;
     for (int minb : {8, 4})
       for (int waves : {0, 1, 2}) {

@@ -14,9 +14,7 @@ struct RunShape {
   int moving;              // plnt_flag 2: the planet feels the disk (own step sequence)
   int eos;                 // EOS 1: isentropic sweeps (own step sequence)
   int nr, nphi, nk;
-  int tiles_x, tiles_y;    // 2D pencil chunks of the radial and azimuthal sweeps
-  int tiles_xs;            // radial last chunks of at most 64 cells, 4 columns per tile
-                           // (then not counted in tiles_x)
+  int tiles_x, tiles_y;    // CTAs of the radial and azimuthal sweeps
 };
 int run_shape(const pg_run *run, RunShape *out);
 

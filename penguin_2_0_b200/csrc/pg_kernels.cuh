@@ -27,19 +27,17 @@ __host__ __device__ inline Chunking make_chunking(int n) {
 // "ring" index rk = k*nrg + row.
 struct Tables {
   int nr, nphi, nk, nrg;
-  int occ8;                                     // 128-thread sweeps capped at 64 registers (8 CTAs/SM)
-  int zpack;                                    // polar pencils per CTA when nk is one chunk (0: one per CTA)
-  int xpack;                                    // radial columns per CTA of the full chunks (1, 2 or 4)
   Chunking cx, cy, cz;
   const double *rx, *rdx, *rxvol, *rxc;         // [nrg]
+  const double *irdx, *irxc;                    // [nrg]: 1/rdx, 1/rxc (k_tables)
   const double *radc, *cs2, *nu;                // [nk*nrg]
-  const double *gp;                             // [nk*nrg] ghost-ring pressure
+  const double *irc, *snd;                      // [nk*nrg]: 1/radc, sqrt(gam cs2) (k_tables)
   const double *y, *dy, *yvol, *yc;             // [nphi]
+  const double *idy, *cyc, *syc;                // [nphi]: 1/dy, cos(yc), sin(yc) (k_tables)
   const double *z, *dz, *zvol, *zc;             // [nk + 12]: 6 ghost layers each side
-  const double *szc, *czc;                      // [nk + 12]: sin(zc), cos(zc) (k_tables)
-  const double *szf, *czf;                      // [nk + 12]: sin(z), cos(z) of the layer faces
-  const double *iszc, *iszf, *idz;              // [nk + 12]: 1/sin(zc), 1/sin(z), 1/dz (polar sweep)
-  const double *zpar;                           // [5 (nk + 12)]: Eulerian paraset c0..c4 per layer (k_tables)
+  const double *szc, *idz;                      // [nk + 12]: sin(zc), 1/dz (k_tables)
+  const double *csg;                            // [12 nr]: cs2 of the fixed polar ghost layers (as nug)
+  const double *ax[3];                          // per axis: what a chunk's cells need of the grid (pg_warp.cuh)
   const double *nug;                            // [12 nr]: nu of the polar ghost layers (6 below, 6 above) per ring
   const double *val_r, *val_u, *val_v;          // [nk*nrg] damping / FARGO targets
   const double *damp_g, *damp_pw;               // [nk*nrg] zone factor, r^-1.5
@@ -50,17 +48,16 @@ struct Tables {
   int *inc_j, *rot_j;                           // [nk*nrg]
 };
 
-struct Planes {
-  const double *r, *u, *v, *w;
-  double *ro, *uo, *vo, *wo;
-  const double *p0;   // non-null: pressure of a freshly loaded dump (first sweep only)
+// State planes a sweep reads and writes: FP64 Sigma, v_r, v_phi, v_theta, or
+// FP32 dS = Sigma - S_bg, v_r, dv = v_phi - v_bg, v_theta
+template <class RT>
+struct PlanesT {
+  const RT *r = nullptr, *u = nullptr, *v = nullptr, *w = nullptr;
+  RT *ro = nullptr, *uo = nullptr, *vo = nullptr, *wo = nullptr;
+  const double *p0 = nullptr;   // non-null: pressure of a freshly loaded dump (first sweep only, FP64)
 };
-
-// FP32 planes: dS = Sigma - S_bg, v_r, dv = v_phi - v_bg, v_theta
-struct Planes32 {
-  const float *r, *u, *v, *w;
-  float *ro, *uo, *vo, *wo;
-};
+using Planes = PlanesT<double>;
+using Planes32 = PlanesT<float>;
 
 // The device-resident clock of the fused loop (main.cu:270-441).
 struct DevClock {
@@ -120,64 +117,100 @@ struct BatchQueue {
   int total;
 };
 
+// ---- small device functions the sweeps and the kernels around them share ----
+// Operations are written out, so that a value has the same bits wherever it
+// is formed (the fused epilogue and the separate kernels must agree).
+__device__ __forceinline__ int wrap1(int j, int n) {
+  if (j < 0) j += n;
+  if (j >= n) j -= n;
+  return j;
+}
+__device__ __forceinline__ int wrapm(int j, int n) {
+  j %= n;
+  return j < 0 ? j + n : j;
+}
+// a density or azimuthal velocity from and to its plane (FP32: less the ring's background)
+template <class RT>
+__device__ __forceinline__ double load_r(RT x, double bg) {
+  return sizeof(RT) == 4 ? bg + (double)x : (double)x;
+}
+template <class RT>
+__device__ __forceinline__ RT store_r(double x, double bg) {
+  return sizeof(RT) == 4 ? (RT)(x - bg) : (RT)x;
+}
+__device__ __forceinline__ double damped(double x, double target, double f) { return __fma_rn(f, __dsub_rn(target, x), x); }
+__device__ __forceinline__ double sound_speed(double r, double p, const Phys &ph) { return sqrt(__dmul_rn(ph.gam, p) / r); }
+// dt_lv1's rate of a cell (timestep.cu:36-57): 1/dr, azimuthal velocity less
+// the ring's frame, 1/(r dphi), 1/(r dtheta)
+template <bool THREED>
+__device__ __forceinline__ double cfl_rate(double cs, double u, double irdx, double v, double iwy, double w, double iwz) {
+  const double t0 = __dmul_rn(__dadd_rn(fabs(u), cs), irdx), t1 = __dmul_rn(__dadd_rn(fabs(v), cs), iwy);
+  if (!THREED) return fmax(t0, t1);
+  return max3(t0, t1, __dmul_rn(__dadd_rn(fabs(w), cs), iwz));
+}
+// the run of tile t of a batch queue, by bisection in its prefix sums
+__device__ __forceinline__ int batch_find(const BatchQueue &q, int t) {
+  int lo = 0, hi = q.nruns;   // q.start[lo] <= t < q.start[hi]
+  while (hi - lo > 1) {
+    int mid = (lo + hi) >> 1;
+    if (q.start[mid] <= t) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
 }  // namespace pgd
 
-// launchers (pg_kernels.cu)
+// launchers (pg_kernels.cu; the sweeps in pg_sweep.cu)
 namespace pgk {
 using namespace pgd;
 void tables(const Tables &T, const Phys &ph, int ndim, double kill_rin, double kill_rout, double xmin,
             double xmax, cudaStream_t s);
-void sweep_x(const Tables &T, const Planes &P, const Phys &ph, const SweepCtl &c, int ndim, cudaStream_t s);
-void sweep_y(const Tables &T, const Planes &P, const Phys &ph, const SweepCtl &c, int ndim, cudaStream_t s);
-void sweep_z(const Tables &T, const Planes &P, const Phys &ph, const SweepCtl &c, int ntop, cudaStream_t s);
-int sweep_launches(const Chunking &ch);
+template <class RT>
+void sweep_x(const Tables &T, const PlanesT<RT> &P, const Phys &ph, const SweepCtl &c, int ndim, cudaStream_t s);
+template <class RT>
+void sweep_y(const Tables &T, const PlanesT<RT> &P, const Phys &ph, const SweepCtl &c, int ndim, cudaStream_t s);
+template <class RT>
+void sweep_z(const Tables &T, const PlanesT<RT> &P, const Phys &ph, const SweepCtl &c, int ntop, cudaStream_t s);
 // per-device kernel attributes (dynamic shared memory limits); 0 on success
 int setup_device();
-int setup_device32();
-void cfl_full(const Tables &T, const double *r, const double *u, const double *v, const double *w,
-              const double *p0, const Phys &ph, double frrot, int ndim, unsigned long long *out,
-              cudaStream_t s);
+// CTAs of a run's radial and azimuthal sweep (batch queues)
+int tiles_x(const Tables &T);
+int tiles_y(const Tables &T);
+// the grid's axis tables (Tables::ax), and the doubles one takes
+void axis_tables(const Tables &T, int ndim, cudaStream_t s);
+size_t axis_table_elems(const Chunking &ch);
+// CFL rate max of the planes (p0: the pressure of a freshly loaded dump, or
+// null) into *out; with clk, the device loop's: FrRot, target and halt flag
+// from the clock, the step's shift still pending when rot_pending
+template <class RT>
+void cfl(const Tables &T, const RT *r, const RT *u, const RT *v, const RT *w, const double *p0, const Phys &ph,
+         double frrot, int ndim, unsigned long long *out, DevClock *clk, int rot_pending, cudaStream_t s);
 void index_shift(const Tables &T, double dt, double frrot, int fargo, const DevClock *clk, cudaStream_t s);
 void rotate(const Tables &T, const DevClock *clk, cudaStream_t s);
-void damp(const Tables &T, double *r, double *u, double *v, double *w, double dt, int ndim, cudaStream_t s);
+// damping by dt, or by the clock's step
+template <class RT>
+void damp(const Tables &T, RT *r, RT *u, RT *v, RT *w, double dt, const DevClock *clk, int ndim, cudaStream_t s);
 void reduce(const Tables &T, const double *r, const Body &pl, const DevClock *clk, double exclude,
             int mode, int plnt, double p_alpha, int ndim, double *ring_part, unsigned int *counter,
             double *out, double *hist_row, cudaStream_t s);
 void reduce32(const Tables &T, const float *r, const Body &pl, const DevClock *clk, double exclude, int mode,
               int plnt, double p_alpha, int ndim, double *ring_part, unsigned int *counter, double *out,
               cudaStream_t s);
-// FP32 sweeps (pg_kernels32.cu)
-void sweep_x32(const Tables &T, const Planes32 &P, const Phys &ph, const SweepCtl &c, int ndim, cudaStream_t s);
-void sweep_y32(const Tables &T, const Planes32 &P, const Phys &ph, const SweepCtl &c, int ndim, cudaStream_t s);
-void sweep_z32(const Tables &T, const Planes32 &P, const Phys &ph, const SweepCtl &c, int ntop, cudaStream_t s);
-void cfl32(const Tables &T, const Planes32 &cur, const Phys &ph, double frrot, int ndim, int rot_pending,
-           unsigned long long *out, int *status, cudaStream_t s);
-void damp32(const Tables &T, const Planes32 &cur, double dt, const DevClock *clk, int ndim, cudaStream_t s);
-void cfl32_clk(const Tables &T, const Planes32 &cur, const Phys &ph, int ndim, DevClock *clk, cudaStream_t s,
-               int rot_pending = 1);
 // batched 2D steps over many runs (one launch per phase for all runs)
 void batch_prestep(const BatchRun *runs, int nruns, cudaStream_t s);
 void batch_poststep(const BatchRun *runs, int nruns, cudaStream_t s);
 void batch_record(const BatchRun *runs, int nruns, cudaStream_t s);
 void batch_reduce(const BatchQueue &rings, int fp32, int mode, cudaStream_t s);
-void batch_sweep_x(const BatchQueue &q, int grid, int minb, cudaStream_t s);
-void batch_sweep_x_short(const BatchQueue &q, cudaStream_t s);
-void batch_sweep_x32_short(const BatchQueue &q, cudaStream_t s);
-void batch_sweep_y(const BatchQueue &q, int grid, int minb, cudaStream_t s);
-void batch_sweep_x32(const BatchQueue &q, int grid, int minb, cudaStream_t s);
-void batch_sweep_y32(const BatchQueue &q, int grid, int minb, cudaStream_t s);
-void damp_clk(const Tables &T, double *r, double *u, double *v, double *w, const DevClock *clk,
-              cudaStream_t s);
-void cfl_clk(const Tables &T, const double *r, const double *u, const double *v, const double *w,
-             const Phys &ph, DevClock *clk, cudaStream_t s);
+template <class RT>
+void batch_sweep_x(const BatchQueue &q, int grid, cudaStream_t s);
+template <class RT>
+void batch_sweep_y(const BatchQueue &q, int grid, cudaStream_t s);
 void prestep(DevClock *clk, const Tables &T, int fargo, cudaStream_t s);
 // moving planet (plnt_flag 2): the step's end split around the disk-force reductions
 void poststep_drift(DevClock *clk, const Tables &T, cudaStream_t s);
 void poststep_kick(DevClock *clk, cudaStream_t s);
 void reduce_forces(const Tables &T, const void *r, int fp32, DevClock *clk, double p_alpha, int ndim,
                    double *ring_part, unsigned int *counter, cudaStream_t s);
-void cfl_clk_after(const Tables &T, const double *r, const double *u, const double *v, const double *w,
-                   const Phys &ph, DevClock *clk, int ndim, cudaStream_t s);
 void poststep(DevClock *clk, const Tables &T, cudaStream_t s);
 // dump <-> planes: stage holds the dump's field arrays ring by ring ([nr*nk][5][nphi]
 // for unpack, whole 72*nphi+96-byte ring records for pack); err bit 1: a density

@@ -122,6 +122,14 @@ static int check_launch(pg_run *run, int n) {
   return PG_OK;
 }
 
+// doubles of a run's table block (pg_create lays it out)
+static size_t table_elems(size_t nr, size_t nphi, size_t nk) {
+  const size_t nrg = nr + 2 * NPAD, nring = nk * nrg, nz = nk + 2 * NPAD;
+  size_t n = 6 * nrg + 11 * nring + 7 * nphi + 6 * nz + 6 * (size_t)2 * NPAD * nr;
+  for (size_t len : {nr, nphi, nk}) n += pgk::axis_table_elems(pgd::make_chunking((int)len));
+  return n;
+}
+
 static pgd::Planes32 planes32_fwd(pg_run *run, int src) {
   pgd::Planes32 p;
   p.r = run->p32[src][0]; p.u = run->p32[src][1]; p.v = run->p32[src][2]; p.w = run->p32[src][3];
@@ -129,15 +137,6 @@ static pgd::Planes32 planes32_fwd(pg_run *run, int src) {
   p.wo = run->p32[1 - src][3];
   return p;
 }
-// the current FP32 planes as both source and target (in-place kernels)
-static pgd::Planes32 planes32_cur(pg_run *run) {
-  pgd::Planes32 p;
-  int c = run->cur;
-  p.r = p.ro = run->p32[c][0]; p.u = p.uo = run->p32[c][1]; p.v = p.vo = run->p32[c][2];
-  p.w = p.wo = run->p32[c][3];
-  return p;
-}
-
 static pgd::Planes planes_fwd(pg_run *run, int src, const double *p0) {
   pgd::Planes p;
   p.r = run->planes[src][0]; p.u = run->planes[src][1]; p.v = run->planes[src][2]; p.w = run->planes[src][3];
@@ -145,6 +144,91 @@ static pgd::Planes planes_fwd(pg_run *run, int src, const double *p0) {
   p.wo = run->planes[1 - src][3];
   p.p0 = p0;
   return p;
+}
+
+// One step of main.cu:343-441 as device work on the run's stream.
+template <class RT>
+static RT **planes_of(pg_run *run, int copy) {
+  if constexpr (sizeof(RT) == 4) return run->p32[copy];
+  else return run->planes[copy];
+}
+template <class RT>
+static pgd::PlanesT<RT> fwd(pg_run *run, int src, const double *p0) {
+  if constexpr (sizeof(RT) == 4) return planes32_fwd(run, src);
+  else return planes_fwd(run, src, p0);
+}
+
+template <class RT>
+static int enqueue_step_t(pg_run *run, bool first_p0) {
+  const pg_params &P = run->P;
+  cudaStream_t s = run->stream;
+  pgd::SweepCtl c{};
+  c.clk = run->clk;
+  c.fuse = 0;
+  c.shift = 0;
+  int a = run->cur;
+  int n = 0;
+  const bool tm = run->timing;
+  size_t e_step = 0, e_k = 0;
+  if (tm && ev_pair(run, 3, e_step)) return fail(run, PG_ERR_CUDA, "event record");
+  pgk::prestep(run->clk, run->T, P.FARGO_flag, s); n++;
+  if (tm && ev_pair(run, 0, e_k)) return fail(run, PG_ERR_CUDA, "event record");
+  pgk::sweep_x<RT>(run->T, fwd<RT>(run, a, first_p0 ? run->p0 : nullptr), run->ph, c, P.ndim, s); n++;
+  if (tm && ev_close(run, e_k)) return fail(run, PG_ERR_CUDA, "event record");
+  const bool moving = P.plnt_flag == 2;
+  if (P.ndim == 2) {
+    c.fuse = 1;
+    c.shift = 1;
+    c.nocfl = moving;
+  }
+  if (tm && ev_pair(run, 1, e_k)) return fail(run, PG_ERR_CUDA, "event record");
+  pgk::sweep_y<RT>(run->T, fwd<RT>(run, 1 - a, nullptr), run->ph, c, P.ndim, s); n++;
+  if (tm && ev_close(run, e_k)) return fail(run, PG_ERR_CUDA, "event record");
+  if (P.ndim == 3) {
+    // the polar sweep applies the FARGO shift; damping and the CFL rate are
+    // fused into its store when its chunks are never idle
+    if (tm && ev_pair(run, 2, e_k)) return fail(run, PG_ERR_CUDA, "event record");
+    c.shift = 1;
+    const bool fuse_z = !run->T.cz.stuck;
+    c.fuse = fuse_z;
+    c.nocfl = moving;
+    pgk::sweep_z<RT>(run->T, fwd<RT>(run, a, nullptr), run->ph, c, P.ntop, s); n++;
+    if (tm && ev_close(run, e_k)) return fail(run, PG_ERR_CUDA, "event record");
+    RT **cp = planes_of<RT>(run, 1 - a);
+    if (!fuse_z) {
+      pgk::damp<RT>(run->T, cp[0], cp[1], cp[2], cp[3], 0.0, run->clk, 3, s); n++;
+      if (!moving) {
+        pgk::cfl<RT>(run->T, cp[0], cp[1], cp[2], cp[3], nullptr, run->ph, 0.0, 3, nullptr, run->clk, 1, s); n++;
+      }
+    }
+    run->cur = 1 - a;
+  }
+  RT **cp = planes_of<RT>(run, run->cur);
+  if (moving) {
+    // moving planet (planet.cu:54-93): drift, the disk's forces on the
+    // drifted planet (reductions 8 and 9), kick; FrRot is then known and the
+    // next get_dt's CFL runs on the stored state
+    pgk::poststep_drift(run->clk, run->T, s); n++;
+    pgk::reduce_forces(run->T, cp[0], run->fp32, run->clk, P.p_alpha, P.ndim, run->ring_part, run->counter, s); n += 2;
+    pgk::poststep_kick(run->clk, s); n++;
+    pgk::cfl<RT>(run->T, cp[0], cp[1], cp[2], cp[3], nullptr, run->ph, 0.0, P.ndim, nullptr, run->clk, 0, s); n++;
+  } else {
+    pgk::poststep(run->clk, run->T, s); n++;
+  }
+  auto sum = [&](int mode, int plnt, double *out) {
+    if constexpr (sizeof(RT) == 4)
+      pgk::reduce32(run->T, cp[0], pgd::Body{}, run->clk, 0.0, mode, plnt, P.p_alpha, P.ndim, run->ring_part,
+                    run->counter, out, s);
+    else
+      pgk::reduce(run->T, cp[0], pgd::Body{}, run->clk, 0.0, mode, plnt, P.p_alpha, P.ndim, run->ring_part,
+                  run->counter, out, nullptr, s);
+    n++;
+  };
+  sum(0, P.plnt_flag > 0, &run->clk->mass);
+  if (P.plnt_flag > 0 && P.ndim == 2) sum(9, 1, &run->clk->torque);
+  pgk::record(run->clk, s); n++;
+  if (tm && ev_close(run, e_step)) return fail(run, PG_ERR_CUDA, "event record");
+  return check_launch(run, n);
 }
 
 extern "C" {
@@ -190,49 +274,32 @@ int pg_create(const pg_params *p, int device, pg_run **out) {
   int nrg = run->nrg, nphi = run->nphi, nk = run->nk, nr = run->nr;
   size_t nring = (size_t)nk * nrg;
   size_t nz = (size_t)nk + 2 * NPAD;
-  run->tab_elems = 4 * (size_t)nrg + 10 * nring + 4 * (size_t)nphi + 16 * nz + (size_t)2 * NPAD * nr * 4 +
-                   (size_t)2 * NPAD * nr;
+  run->tab_elems = table_elems(nr, nphi, nk);
   if (cudaMalloc(&run->tab, run->tab_elems * sizeof(double)) != cudaSuccess) return bail(PG_ERR_NOMEM);
   if (cudaMalloc(&run->itab, 2 * nring * sizeof(int)) != cudaSuccess) return bail(PG_ERR_NOMEM);
   double *t = run->tab;
   pgd::Tables &T = run->T;
   T.nr = nr; T.nphi = nphi; T.nk = nk; T.nrg = nrg;
-  {
-    // 64-register sweeps (8 CTAs of 128 per SM) by default: ~14% faster on
-    // large 2D grids, same arithmetic; PG_SWEEP_OCC=6 keeps ~76 registers
-    const char *occ = std::getenv("PG_SWEEP_OCC");
-    T.occ8 = (occ && std::atoi(occ) == 6) ? 0 : 1;
-    // short chunks packed several per CTA by default: a radial last chunk of
-    // at most 64 cells 4 per CTA, an FP64 polar pencil of one chunk 8 per CTA
-    // up to 44 cells and 4 above, an FP32 one 4 per CTA (PG_POLAR_PACK=0: one
-    // per CTA); same arithmetic per cell either way
-    const char *zp = std::getenv("PG_POLAR_PACK");
-    T.zpack = (zp && std::atoi(zp) == 0) ? 0 : 4;
-    // full radial chunks: 2 adjacent azimuth columns per CTA by default
-    // (PG_RADIAL_PACK 1 or 4 for one or four); same arithmetic per cell.
-    // Measured on the 128x1024x32 disk: radial 0.727 ms with one column per
-    // CTA, 0.660 with two, 0.697 with four
-    const char *xp = std::getenv("PG_RADIAL_PACK");
-    T.xpack = xp ? std::atoi(xp) : 2;
-    if (T.xpack != 2 && T.xpack != 4) T.xpack = 1;
-  }
   T.cx = pgd::make_chunking(nr);
   T.cy = pgd::make_chunking(nphi);
   T.cz = pgd::make_chunking(nk);
+  // the axis tables first: their chunks start on 16-byte boundaries
+  for (int a = 0; a < 3; a++) {
+    T.ax[a] = t;
+    t += pgk::axis_table_elems(a == 0 ? T.cx : a == 1 ? T.cy : T.cz);
+  }
   T.rx = t; t += nrg; T.rdx = t; t += nrg; T.rxvol = t; t += nrg; T.rxc = t; t += nrg;
-  T.radc = t; t += nring; T.cs2 = t; t += nring; T.nu = t; t += nring; T.gp = t; t += nring;
+  T.irdx = t; t += nrg; T.irxc = t; t += nrg;
+  T.radc = t; t += nring; T.cs2 = t; t += nring; T.nu = t; t += nring; T.irc = t; t += nring; T.snd = t; t += nring;
   T.val_r = t; t += nring; T.val_u = t; t += nring; T.val_v = t; t += nring;
   T.damp_g = t; t += nring; T.damp_pw = t; t += nring;
   T.res_v = t; t += nring;
-  // rot_v shares the block below (10th ring table)
+  // rot_v has a block of its own below
   T.y = t; t += nphi; T.dy = t; t += nphi; T.yvol = t; t += nphi; T.yc = t; t += nphi;
-  T.z = t; t += nz; T.dz = t; t += nz; T.zvol = t; t += nz; T.zc = t; t += nz;
-  // szc, czc, szf, czf, iszc, iszf, idz consecutive at stride nz: the polar
-  // sweep reads them as lay[0], lay[nz], ... from one pointer per layer
-  T.szc = t; t += nz; T.czc = t; t += nz; T.szf = t; t += nz; T.czf = t; t += nz;
-  T.iszc = t; t += nz; T.iszf = t; t += nz; T.idz = t; t += nz;
-  T.zpar = t; t += 5 * nz;
+  T.idy = t; t += nphi; T.cyc = t; t += nphi; T.syc = t; t += nphi;
+  T.z = t; t += nz; T.dz = t; t += nz; T.zvol = t; t += nz; T.zc = t; t += nz; T.szc = t; t += nz; T.idz = t; t += nz;
   T.nug = t; t += (size_t)2 * NPAD * nr;
+  T.csg = t; t += (size_t)2 * NPAD * nr;
   T.tg = t; t += (size_t)2 * NPAD * nr * 4;
   if (cudaMalloc(&T.rot_v, nring * sizeof(double)) != cudaSuccess) return bail(PG_ERR_NOMEM);
   if (cudaMalloc(&run->vbg, nring * sizeof(double)) != cudaSuccess) return bail(PG_ERR_NOMEM);
@@ -321,7 +388,7 @@ int pg_load_rings(pg_run *run, const void *rings, size_t bytes) {
   const size_t nring = (size_t)nk * nrg, nz = (size_t)nk + 2 * NPAD;
   // host images of the tables
   std::vector<double> rx(nrg), rdx(nrg), rxvol(nrg), rxc(nrg);
-  std::vector<double> gp(nring, 0.0), vr(nring, 0.0), vu(nring, 0.0), vv(nring, 0.0);
+  std::vector<double> vr(nring, 0.0), vu(nring, 0.0), vv(nring, 0.0);
   std::vector<double> res_v(nring, 0.0), rot_v(nring, 0.0), vbg(nring, 0.0), sbg(nring, 0.0);
   std::vector<int> inc_j(nring, 0), rot_j(nring, 0);
   std::vector<double> z(nz, 0.0), dz(nz, 0.0), zvol(nz, 0.0), zc(nz, 0.0);
@@ -339,8 +406,8 @@ int pg_load_rings(pg_run *run, const void *rings, size_t bytes) {
   for (int k = 0; k < nk; k++) {
     for (int i = 0; i < NPAD; i++) {
       size_t a = (size_t)k * nrg + i, c = (size_t)k * nrg + nr + NPAD + i;
-      gp[a] = lft[i + NPAD * k].p; rot_v[a] = lft[i + NPAD * k].rot_v; vbg[a] = lft[i + NPAD * k].v; sbg[a] = lft[i + NPAD * k].r;
-      gp[c] = rgh[i + NPAD * k].p; rot_v[c] = rgh[i + NPAD * k].rot_v; vbg[c] = rgh[i + NPAD * k].v; sbg[c] = rgh[i + NPAD * k].r;
+      rot_v[a] = lft[i + NPAD * k].rot_v; vbg[a] = lft[i + NPAD * k].v; sbg[a] = lft[i + NPAD * k].r;
+      rot_v[c] = rgh[i + NPAD * k].rot_v; vbg[c] = rgh[i + NPAD * k].v; sbg[c] = rgh[i + NPAD * k].r;
     }
     for (int i = 0; i < nr; i++) {
       size_t rk = (size_t)k * nrg + i + NPAD;
@@ -390,7 +457,7 @@ int pg_load_rings(pg_run *run, const void *rings, size_t bytes) {
     return cudaMemcpyAsync((void *)dst, src.data(), src.size() * sizeof(double), cudaMemcpyHostToDevice, s);
   };
   CK(up(T.rx, rx)); CK(up(T.rdx, rdx)); CK(up(T.rxvol, rxvol)); CK(up(T.rxc, rxc));
-  CK(up(T.gp, gp)); CK(up(T.val_r, vr)); CK(up(T.val_u, vu)); CK(up(T.val_v, vv));
+  CK(up(T.val_r, vr)); CK(up(T.val_u, vu)); CK(up(T.val_v, vv));
   CK(up(T.res_v, res_v)); CK(up(T.rot_v, rot_v)); CK(up(T.vbg, vbg)); CK(up(T.sbg, sbg));
   CK(cudaMemcpyAsync(T.inc_j, inc_j.data(), nring * sizeof(int), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(T.rot_j, rot_j.data(), nring * sizeof(int), cudaMemcpyHostToDevice, s));
@@ -440,7 +507,7 @@ int pg_load_rings(pg_run *run, const void *rings, size_t bytes) {
   if (herr & 2) return fail(run, PG_ERR_STATE, "2D dump with nonzero w");
   run->launches += 2;
   pgk::tables(T, run->ph, P.ndim, P.kill_rin, P.kill_rout, P.xmin, P.xmax, s);
-  if (int e = check_launch(run, 1)) return e;
+  if (int e = check_launch(run, P.ndim == 3 ? 4 : 3)) return e;
   CK(cudaStreamSynchronize(s));
   run->cur = 0;
   run->p0_live = !run->fp32;
@@ -535,12 +602,13 @@ int pg_get_dt(pg_run *run, double dt_old, double frrot, double *dt_out) {
   CK(cudaSetDevice(run->dev));
   cudaStream_t s = run->stream;
   double **cp = run->planes[run->cur];
+  float **fp = run->p32[run->cur];
   CK(cudaMemsetAsync(run->cfl, 0, sizeof(unsigned long long), s));
   if (run->fp32)
-    pgk::cfl32(run->T, planes32_cur(run), run->ph, frrot, run->P.ndim, 0, run->cfl, nullptr, s);
+    pgk::cfl<float>(run->T, fp[0], fp[1], fp[2], fp[3], nullptr, run->ph, frrot, run->P.ndim, run->cfl, nullptr, 0, s);
   else
-    pgk::cfl_full(run->T, cp[0], cp[1], cp[2], cp[3], run->p0_live ? run->p0 : nullptr, run->ph, frrot,
-                  run->P.ndim, run->cfl, s);
+    pgk::cfl<double>(run->T, cp[0], cp[1], cp[2], cp[3], run->p0_live ? run->p0 : nullptr, run->ph, frrot,
+                     run->P.ndim, run->cfl, nullptr, 0, s);
   if (int e = check_launch(run, 1)) return e;
   unsigned long long bits = 0;
   CK(cudaMemcpyAsync(&bits, run->cfl, sizeof(bits), cudaMemcpyDeviceToHost, s));
@@ -574,10 +642,6 @@ static pgd::SweepCtl host_ctl(double dt, const pg_body *pl, double frrot) {
   return c;
 }
 
-static int nx(pg_run *run) { return pgk::sweep_launches(run->T.cx); }
-static int ny(pg_run *run) { return pgk::sweep_launches(run->T.cy); }
-static int nz(pg_run *run) { return pgk::sweep_launches(run->T.cz); }
-
 // On a 3D run this is what the reference's bundle_sweep2D does on a 3D
 // build: the radial and azimuthal sweeps of every polar layer (sweepx takes
 // the layer from blockIdx.y, ppm.cu:33; sweepy folds it into the ring index,
@@ -590,17 +654,17 @@ int pg_sweep2d(pg_run *run, double dt, const pg_body *planet, double frrot) {
   cudaStream_t s = run->stream;
   const int nd = run->P.ndim;
   if (run->fp32) {
-    pgk::sweep_x32(run->T, planes32_fwd(run, run->cur), run->ph, c, nd, s);
+    pgk::sweep_x<float>(run->T, planes32_fwd(run, run->cur), run->ph, c, nd, s);
     c.shift = 1;
-    pgk::sweep_y32(run->T, planes32_fwd(run, 1 - run->cur), run->ph, c, nd, s);
+    pgk::sweep_y<float>(run->T, planes32_fwd(run, 1 - run->cur), run->ph, c, nd, s);
   } else {
-    pgk::sweep_x(run->T, planes_fwd(run, run->cur, run->p0_live ? run->p0 : nullptr), run->ph, c, nd, s);
+    pgk::sweep_x<double>(run->T, planes_fwd(run, run->cur, run->p0_live ? run->p0 : nullptr), run->ph, c, nd, s);
     c.shift = 1;
-    pgk::sweep_y(run->T, planes_fwd(run, 1 - run->cur, nullptr), run->ph, c, nd, s);
+    pgk::sweep_y<double>(run->T, planes_fwd(run, 1 - run->cur, nullptr), run->ph, c, nd, s);
   }
   if (run->P.FARGO_flag > 0) pgk::rotate(run->T, nullptr, s);
   run->p0_live = false;
-  return check_launch(run, nx(run) + ny(run) + (run->P.FARGO_flag > 0 ? 1 : 0));
+  return check_launch(run, 2 + (run->P.FARGO_flag > 0 ? 1 : 0));
 }
 
 int pg_sweep3d(pg_run *run, double dt, const pg_body *planet, double frrot) {
@@ -612,20 +676,20 @@ int pg_sweep3d(pg_run *run, double dt, const pg_body *planet, double frrot) {
   cudaStream_t s = run->stream;
   int a = run->cur;
   if (run->fp32) {
-    pgk::sweep_x32(run->T, planes32_fwd(run, a), run->ph, c, 3, s);
-    pgk::sweep_y32(run->T, planes32_fwd(run, 1 - a), run->ph, c, 3, s);
+    pgk::sweep_x<float>(run->T, planes32_fwd(run, a), run->ph, c, 3, s);
+    pgk::sweep_y<float>(run->T, planes32_fwd(run, 1 - a), run->ph, c, 3, s);
     c.shift = 1;
-    pgk::sweep_z32(run->T, planes32_fwd(run, a), run->ph, c, run->P.ntop, s);
+    pgk::sweep_z<float>(run->T, planes32_fwd(run, a), run->ph, c, run->P.ntop, s);
   } else {
-    pgk::sweep_x(run->T, planes_fwd(run, a, run->p0_live ? run->p0 : nullptr), run->ph, c, 3, s);
-    pgk::sweep_y(run->T, planes_fwd(run, 1 - a, nullptr), run->ph, c, 3, s);
+    pgk::sweep_x<double>(run->T, planes_fwd(run, a, run->p0_live ? run->p0 : nullptr), run->ph, c, 3, s);
+    pgk::sweep_y<double>(run->T, planes_fwd(run, 1 - a, nullptr), run->ph, c, 3, s);
     c.shift = 1;   // the polar sweep is the last one: it applies the FARGO shift
-    pgk::sweep_z(run->T, planes_fwd(run, a, nullptr), run->ph, c, run->P.ntop, s);
+    pgk::sweep_z<double>(run->T, planes_fwd(run, a, nullptr), run->ph, c, run->P.ntop, s);
   }
   if (run->P.FARGO_flag > 0) pgk::rotate(run->T, nullptr, s);
   run->cur = 1 - a;
   run->p0_live = false;
-  return check_launch(run, nx(run) + ny(run) + nz(run) + (run->P.FARGO_flag > 0 ? 1 : 0));
+  return check_launch(run, 3 + (run->P.FARGO_flag > 0 ? 1 : 0));
 }
 
 int pg_sweep_axis(pg_run *run, int axis, double dt, const pg_body *planet, double frrot) {
@@ -640,19 +704,19 @@ int pg_sweep_axis(pg_run *run, int axis, double dt, const pg_body *planet, doubl
   // polar in 3D.  The dump's p is used only by a leading radial sweep.
   int n = 0;
   if (axis == 0) {
-    if (run->fp32) pgk::sweep_x32(run->T, planes32_fwd(run, a), run->ph, c, run->P.ndim, s);
-    else pgk::sweep_x(run->T, planes_fwd(run, a, run->p0_live ? run->p0 : nullptr), run->ph, c, run->P.ndim, s);
-    n = nx(run);
+    if (run->fp32) pgk::sweep_x<float>(run->T, planes32_fwd(run, a), run->ph, c, run->P.ndim, s);
+    else pgk::sweep_x<double>(run->T, planes_fwd(run, a, run->p0_live ? run->p0 : nullptr), run->ph, c, run->P.ndim, s);
+    n = 1;
   } else if (axis == 1) {
     c.shift = run->P.ndim == 2;
-    if (run->fp32) pgk::sweep_y32(run->T, planes32_fwd(run, a), run->ph, c, run->P.ndim, s);
-    else pgk::sweep_y(run->T, planes_fwd(run, a, nullptr), run->ph, c, run->P.ndim, s);
-    n = ny(run);
+    if (run->fp32) pgk::sweep_y<float>(run->T, planes32_fwd(run, a), run->ph, c, run->P.ndim, s);
+    else pgk::sweep_y<double>(run->T, planes_fwd(run, a, nullptr), run->ph, c, run->P.ndim, s);
+    n = 1;
   } else {
     c.shift = 1;
-    if (run->fp32) pgk::sweep_z32(run->T, planes32_fwd(run, a), run->ph, c, run->P.ntop, s);
-    else pgk::sweep_z(run->T, planes_fwd(run, a, nullptr), run->ph, c, run->P.ntop, s);
-    n = nz(run);
+    if (run->fp32) pgk::sweep_z<float>(run->T, planes32_fwd(run, a), run->ph, c, run->P.ntop, s);
+    else pgk::sweep_z<double>(run->T, planes_fwd(run, a, nullptr), run->ph, c, run->P.ntop, s);
+    n = 1;
   }
   run->cur = 1 - a;
   run->p0_live = false;
@@ -672,10 +736,11 @@ int pg_damp(pg_run *run, double dt) {
   if (!run->loaded) return fail(run, PG_ERR_STATE, "no state loaded");
   CK(cudaSetDevice(run->dev));
   if (run->fp32) {
-    pgk::damp32(run->T, planes32_cur(run), dt, nullptr, run->P.ndim, run->stream);
+    float **fp = run->p32[run->cur];
+    pgk::damp<float>(run->T, fp[0], fp[1], fp[2], fp[3], dt, nullptr, run->P.ndim, run->stream);
   } else {
     double **cp = run->planes[run->cur];
-    pgk::damp(run->T, cp[0], cp[1], cp[2], cp[3], dt, run->P.ndim, run->stream);
+    pgk::damp<double>(run->T, cp[0], cp[1], cp[2], cp[3], dt, nullptr, run->P.ndim, run->stream);
   }
   return check_launch(run, 1);
 }
@@ -804,11 +869,12 @@ int pg_clock_reset(pg_run *run, int startat) {
   CK(cudaMemcpyAsync(run->clk, &c, sizeof(c), cudaMemcpyHostToDevice, s));
   // first get_dt's CFL rate (the fused loop takes later ones from sweepy)
   double **cp = run->planes[run->cur];
+  float **fp = run->p32[run->cur];
   if (run->fp32)
-    pgk::cfl32(run->T, planes32_cur(run), run->ph, fr, P.ndim, 0, &run->clk->cfl_bits, nullptr, s);
+    pgk::cfl<float>(run->T, fp[0], fp[1], fp[2], fp[3], nullptr, run->ph, fr, P.ndim, &run->clk->cfl_bits, nullptr, 0, s);
   else
-    pgk::cfl_full(run->T, cp[0], cp[1], cp[2], cp[3], run->p0_live ? run->p0 : nullptr, run->ph, fr, P.ndim,
-                  &run->clk->cfl_bits, s);
+    pgk::cfl<double>(run->T, cp[0], cp[1], cp[2], cp[3], run->p0_live ? run->p0 : nullptr, run->ph, fr, P.ndim,
+                     &run->clk->cfl_bits, nullptr, 0, s);
   if (int e = check_launch(run, 1)) return e;
   CK(cudaStreamSynchronize(s));
   run->clock_ready = true;
@@ -834,128 +900,8 @@ int pg_clock_get(pg_run *run, pg_clock *out, pg_body *planet) {
   return PG_OK;
 }
 
-// one step of main.cu:343-441 as device work on the run's stream
-// One step of the device-resident loop on the FP32 planes: the same launch
-// sequence as the FP64 step below, with the float sweeps.
-static int enqueue_step32(pg_run *run, pgd::SweepCtl c, int n, size_t e_step) {
-  const pg_params &P = run->P;
-  cudaStream_t s = run->stream;
-  const bool tm = run->timing;
-  size_t e_k = 0;
-  int a = run->cur;
-  if (tm && ev_pair(run, 0, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-  pgk::sweep_x32(run->T, planes32_fwd(run, a), run->ph, c, P.ndim, s); n += nx(run);
-  if (tm && ev_close(run, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-  const bool moving = P.plnt_flag == 2;
-  if (P.ndim == 2) {
-    c.fuse = 1;
-    c.shift = 1;
-    c.nocfl = moving;
-    if (tm && ev_pair(run, 1, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-    pgk::sweep_y32(run->T, planes32_fwd(run, 1 - a), run->ph, c, 2, s); n += ny(run);
-    if (tm && ev_close(run, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-  } else {
-    if (tm && ev_pair(run, 1, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-    pgk::sweep_y32(run->T, planes32_fwd(run, 1 - a), run->ph, c, 3, s); n += ny(run);
-    if (tm && ev_close(run, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-    if (tm && ev_pair(run, 2, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-    c.shift = 1;
-    pgk::sweep_z32(run->T, planes32_fwd(run, a), run->ph, c, P.ntop, s); n += nz(run);
-    if (tm && ev_close(run, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-    run->cur = 1 - a;
-    pgk::damp32(run->T, planes32_cur(run), 0.0, run->clk, 3, s); n++;
-    if (!moving) { pgk::cfl32_clk(run->T, planes32_cur(run), run->ph, 3, run->clk, s); n++; }
-  }
-  if (moving) {
-    // drift, disk forces on the drifted planet, kick; then the next CFL
-    pgk::poststep_drift(run->clk, run->T, s); n++;
-    pgk::reduce_forces(run->T, run->p32[run->cur][0], 1, run->clk, P.p_alpha, P.ndim, run->ring_part,
-                       run->counter, s); n += 2;
-    pgk::poststep_kick(run->clk, s); n++;
-    pgk::cfl32_clk(run->T, planes32_cur(run), run->ph, P.ndim, run->clk, s, 0); n++;
-  } else {
-    pgk::poststep(run->clk, run->T, s); n++;
-  }
-  pgk::reduce32(run->T, run->p32[run->cur][0], pgd::Body{}, run->clk, 0.0, 0, P.plnt_flag > 0, P.p_alpha, P.ndim,
-                run->ring_part, run->counter, &run->clk->mass, s); n++;
-  if (P.plnt_flag > 0 && P.ndim == 2) {
-    pgk::reduce32(run->T, run->p32[run->cur][0], pgd::Body{}, run->clk, 0.0, 9, 1, P.p_alpha, P.ndim,
-                  run->ring_part, run->counter, &run->clk->torque, s); n++;
-  }
-  pgk::record(run->clk, s); n++;
-  if (tm && ev_close(run, e_step)) return fail(run, PG_ERR_CUDA, "event record");
-  return check_launch(run, n);
-}
-
 static int enqueue_step(pg_run *run, bool first_p0) {
-  const pg_params &P = run->P;
-  cudaStream_t s = run->stream;
-  pgd::SweepCtl c{};
-  c.clk = run->clk;
-  c.fuse = 0;
-  c.shift = 0;
-  int a = run->cur;
-  int n = 0;
-  const bool tm = run->timing;
-  size_t e_step = 0, e_k = 0;
-  if (tm && ev_pair(run, 3, e_step)) return fail(run, PG_ERR_CUDA, "event record");
-  pgk::prestep(run->clk, run->T, P.FARGO_flag, s); n++;
-  if (run->fp32) return enqueue_step32(run, c, n, e_step);
-  if (tm && ev_pair(run, 0, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-  pgk::sweep_x(run->T, planes_fwd(run, a, first_p0 ? run->p0 : nullptr), run->ph, c, P.ndim, s); n += nx(run);
-  if (tm && ev_close(run, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-  const bool moving = P.plnt_flag == 2;
-  if (P.ndim == 2) {
-    c.fuse = 1;
-    c.shift = 1;
-    c.nocfl = moving;
-    if (tm && ev_pair(run, 1, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-    pgk::sweep_y(run->T, planes_fwd(run, 1 - a, nullptr), run->ph, c, 2, s); n += ny(run);
-    if (tm && ev_close(run, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-  } else {
-    if (tm && ev_pair(run, 1, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-    pgk::sweep_y(run->T, planes_fwd(run, 1 - a, nullptr), run->ph, c, 3, s); n += ny(run);
-    if (tm && ev_close(run, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-    // 3D: the polar sweep applies the FARGO shift; damping and the CFL rate
-    // are fused into its store when its chunks are never idle
-    if (tm && ev_pair(run, 2, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-    c.shift = 1;
-    const bool fuse_z = !run->T.cz.stuck;
-    c.fuse = fuse_z;
-    c.nocfl = moving;
-    pgk::sweep_z(run->T, planes_fwd(run, a, nullptr), run->ph, c, P.ntop, s); n += nz(run);
-    if (tm && ev_close(run, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-    double **cp = run->planes[1 - a];
-    if (!fuse_z) {
-      pgk::damp_clk(run->T, cp[0], cp[1], cp[2], cp[3], run->clk, s); n++;
-      if (!moving) { pgk::cfl_clk(run->T, cp[0], cp[1], cp[2], cp[3], run->ph, run->clk, s); n++; }
-    }
-    run->cur = 1 - a;
-  }
-  if (moving) {
-    // moving planet (planet.cu:54-93): drift, the disk's forces on the
-    // drifted planet (reductions 8 and 9), kick; FrRot is then known and the
-    // next get_dt's CFL runs on the stored state
-    double **cp = run->planes[run->cur];
-    pgk::poststep_drift(run->clk, run->T, s); n++;
-    pgk::reduce_forces(run->T, cp[0], 0, run->clk, P.p_alpha, P.ndim, run->ring_part, run->counter, s); n += 2;
-    pgk::poststep_kick(run->clk, s); n++;
-    pgk::cfl_clk_after(run->T, cp[0], cp[1], cp[2], cp[3], run->ph, run->clk, P.ndim, s); n++;
-  } else {
-    pgk::poststep(run->clk, run->T, s); n++;
-  }
-  if (P.plnt_flag > 0 || true) {
-    double **cp = run->planes[run->cur];
-    pgk::reduce(run->T, cp[0], pgd::Body{}, run->clk, 0.0, 0, P.plnt_flag > 0, P.p_alpha, P.ndim,
-                run->ring_part, run->counter, &run->clk->mass, nullptr, s); n++;
-    if (P.plnt_flag > 0 && P.ndim == 2) {
-      pgk::reduce(run->T, cp[0], pgd::Body{}, run->clk, 0.0, 9, 1, P.p_alpha, P.ndim, run->ring_part,
-                  run->counter, &run->clk->torque, nullptr, s); n++;
-    }
-    pgk::record(run->clk, s); n++;
-  }
-  if (tm && ev_close(run, e_step)) return fail(run, PG_ERR_CUDA, "event record");
-  return check_launch(run, n);
+  return run->fp32 ? enqueue_step_t<float>(run, false) : enqueue_step_t<double>(run, first_p0);
 }
 
 // The device clock halts the loop (end time, a tmovie dump, an error); the
@@ -1179,13 +1125,13 @@ extern "C" size_t pg_run_device_bytes(const pg_params *p) {
   if (!p) return 0;
   auto up = [](size_t b) { return (b + 511) & ~(size_t)511; };
   size_t nr = (size_t)p->imax, nphi = (size_t)p->jmax, nk = (size_t)p->kmax, nrg = nr + 2 * NPAD;
-  size_t nring = nk * nrg, nz = nk + 2 * NPAD;
+  size_t nring = nk * nrg;
   size_t pe = nring * nphi;
   int nf = (p->ndim == 3) ? 4 : 3;
   size_t es = (p->precision == 1) ? sizeof(float) : sizeof(double);
   size_t b = 2 * (size_t)nf * up(pe * es);
   if (p->precision != 1) b += up(pe * sizeof(double));                         // p0
-  b += up((4 * nrg + 10 * nring + 4 * nphi + 16 * nz + 2 * NPAD * nr * 4 + 2 * NPAD * nr) * sizeof(double));
+  b += up(table_elems(nr, nphi, nk) * sizeof(double));
   b += up(2 * nring * sizeof(int)) + 3 * up(nring * sizeof(double));           // itab, rot_v, vbg, sbg
   b += up(nr * nk * sizeof(double)) + up(4) + up(32) + up(8) + up(sizeof(pgd::DevClock));
   b += up((size_t)4096 * pgd::HIST_COLS * sizeof(double));
@@ -1205,11 +1151,8 @@ int run_shape(const pg_run *run, RunShape *o) {
   o->moving = run->P.plnt_flag == 2 ? 1 : 0;
   o->eos = run->P.EOS;
   o->nr = run->nr; o->nphi = run->nphi; o->nk = run->nk;
-  const pgd::Chunking &cx = run->T.cx;
-  const bool short_last = !cx.stuck && cx.lim_last <= 64;
-  o->tiles_x = run->nphi * (cx.loop - (short_last ? 1 : 0)) * run->nk;
-  o->tiles_xs = short_last ? (run->nphi * run->nk + 3) / 4 : 0;
-  o->tiles_y = run->T.cy.loop * run->nr * run->nk;
+  o->tiles_x = pgk::tiles_x(run->T);
+  o->tiles_y = pgk::tiles_y(run->T);
   return PG_OK;
 }
 

@@ -1,0 +1,1047 @@
+// pg_sweep.cu -- the directional sweeps: each chunk of a pencil is one warp's
+// work (pg_warp.cuh), in FP64 arithmetic on FP64 or FP32 state planes.
+//
+//   k_sweep_x   radial sweep (ppm.cu:26-160)
+//   k_sweep_y   azimuthal sweep (ppm.cu:162-307); FARGO integer shift
+//               (rotate_rings, ppm.cu:309-322) at its store; optional fused
+//               epilogue: wave damping, CFL rate max (dt_lv1,
+//               timestep.cu:12-73), finiteness check into the status word
+//   k_sweep_z   polar sweep (3D), same store and epilogue
+//   kb_sweep_*  the radial and azimuthal sweeps of every 2D member of a batch
+//
+// FP32 planes hold dS = Sigma - S_bg(ring) and dv = v_phi - v_bg(ring); a
+// sweep adds the FP64 ring values at its loads and rounds the differences at
+// its stores, so both plane types run the same chain.
+//
+// A CTA of 4 warps takes one tile.  Radial and polar tiles are 4 P adjacent
+// azimuth columns of one chunk (P pencils per warp: one full chunk, or as
+// many short ones as 32 lanes hold); the CTA moves them between global and
+// shared memory with neighbouring threads on neighbouring columns, where a
+// lane that read its own rows would use 8 of each 32-byte sector.  Azimuthal
+// pencils lie along the rows: each warp reads its cells directly and passes
+// its results through shared memory, so that a store instruction covers 256
+// contiguous bytes.
+//
+// What bounds them and what they measured (B200, event-timed per sweep, FP64):
+// instruction issue at 2.1-2.3 of 4 per cycle and SM, FP64 pipe 40-45 %, DRAM
+// below 20 %.  Against one thread per cell, the chain through shared memory
+// and 22 CTA barriers per chunk:
+//   128x1024x32  radial 628 -> 284 us, azimuthal 554 -> 207, polar 698 -> 470
+//   1536x4608    radial 836 -> 369 us, azimuthal 906 -> 338
+//   256x768      radial  46 ->  22 us, azimuthal  37 ->  21
+// 4 warps per CTA, 4 CTAs per SM at 128 registers (some 100 bytes of spills):
+// 3 CTAs at 168 registers without spills ran 0-13 % longer, 2 CTAs at 230
+// registers 25-50 %; 8 warps per CTA 5 %, 16 warps 30 %.  Loading the tile in
+// one go before the first use took the radial sweep from 344 to 328 us, cutting
+// the workspace from 11 to 9 slots (which leaves L1 room for the axis tables)
+// from 308 to 284.
+#include "pg_warp.cuh"
+
+namespace pgd {
+
+constexpr int NW = 4;                    // warps per CTA
+constexpr int NT = 32 * NW;
+constexpr int MINB = 4;                  // CTAs per SM
+
+struct StepIn {
+  double dt, frrot, frrot_next;
+  Body pl;
+};
+// the step's dt, planet and frame rotation: launch arguments or the device clock
+__device__ __forceinline__ bool load_step(const SweepCtl &c, StepIn &s) {
+  if (c.clk) {
+    // all loads at once: one round trip to L2
+    s.dt = c.clk->dt_step;
+    s.frrot = c.clk->frrot;
+    s.frrot_next = c.clk->frrot_next;
+    s.pl = c.clk->planet;
+    return !c.clk->halted;
+  } else {
+    s.dt = c.dt;
+    s.frrot = c.frrot;
+    s.frrot_next = c.frrot;
+    s.pl = c.planet;
+  }
+  return true;
+}
+
+// The planet's constants and the cosine and sine of its azimuth, formed by
+// one thread while the others load.
+struct PlanetShm { PlanetC p; double cy, sy; };
+template <bool THREED>
+__device__ __forceinline__ void planet_shm(PlanetShm &S, const StepIn &st, const Phys &ph) {
+  if (threadIdx.x == NT - 32) {
+    S.p = planet_consts<THREED>(st.pl, ph);
+    sincos(st.pl.y, &S.sy, &S.cy);
+  }
+}
+
+// lanes per pencil and pencils per warp of a chunk of lim cells
+struct LaneMap {
+  int G, P;
+  __device__ __forceinline__ LaneMap(int lim, int C) : G((lim + C - 1) / C), P(32 / ((lim + C - 1) / C)) {}
+};
+
+// ---------------------------------------------------------------------------
+// axis tables (pg_warp.cuh AxisEntry): chunk l of an axis holds A_COUNT
+// arrays of ARR entries, cell n = C g + c stored so that a lane's C entries
+// are read in whole lines by the warp (table_pos)
+__device__ __forceinline__ int table_pos(int n, int C, int G) {
+  const int g = n / C, c = n % C;
+  return C == 4 ? (c >> 1) * 2 * G + 2 * g + (c & 1) : c * G + g;
+}
+
+__global__ void k_axis_table(Tables T, int axis, int C, double *out) {
+  const Chunking &ch = axis == 0 ? T.cx : axis == 1 ? T.cy : T.cz;
+  const int nn = axis == 0 ? T.nr : axis == 1 ? T.nphi : T.nk;
+  const int l = blockIdx.x, n = threadIdx.x, N = nn + 2 * NPAD;
+  const int lim = l == ch.loop - 1 ? ch.lim_last : ARR;
+  const int G = (lim + C - 1) / C;
+  if (n >= C * G) return;
+  auto clampe = [&](int e) { return e < 0 ? 0 : e >= N ? N - 1 : e; };
+  auto turn = [&](int e) { return e < NPAD ? -1 : e >= nn + NPAD ? 1 : 0; };
+  auto face = [&](int e) {
+    e = clampe(e);
+    if (axis == 0) return T.rx[e];
+    if (axis == 2) return T.z[e];
+    return T.y[e - NPAD - turn(e) * nn] + turn(e) * kTwoPi;
+  };
+  auto width = [&](int e) {
+    e = clampe(e);
+    if (axis == 0) return T.rdx[e];
+    if (axis == 2) return T.dz[e];
+    return T.dy[e - NPAD - turn(e) * nn];
+  };
+  const int e = clampe(REAL * l + n);
+  const double xm = width(e - 1), x = width(e), xp = width(e + 1), xpp = width(e + 2);
+  const double a = x + xp, b = a + x, c = a + xp, am = xm + x, ap = xp + xpp;
+  const double d = 1.0 / (am + ap);
+  double o[A_COUNT] = {};
+  o[A_XF] = face(e);
+  o[A_IW] = 1.0 / x;
+  o[A_C0] = x / a * (1.0 + 2.0 * d * xp * (am / b - ap / c));
+  o[A_C1] = -d * x * am / b;
+  o[A_C2] = d * xp * ap / c;
+  const double h = x / (am + xp);
+  o[A_C3] = h * (am + xm) / a;
+  o[A_C4] = h * c / am;
+  // derivs (viscosity.cu:2-18) on faces at distances f1 to the left and f2 to
+  // the right: first = (f1/f2 D+ + f2/f1 D-)/(f1+f2), second = 2 (D+/f2 - D-/f1)/(f1+f2)
+  const double f1 = face(e) - face(e - 1), f2 = face(e + 1) - face(e), fs = f1 + f2;
+  if (f1 > 0.0 && f2 > 0.0) {
+    o[A_VA] = f1 / (f2 * fs);
+    o[A_VB] = f2 / (f1 * fs);
+    o[A_VC] = 2.0 / (f2 * fs);
+    o[A_VD] = 2.0 / (f1 * fs);
+  }
+  o[A_VOL] = axis == 0 ? T.rxvol[e] : axis == 2 ? T.zvol[e] : T.yvol[e - NPAD - turn(e) * nn];
+  o[A_IVOL] = 1.0 / o[A_VOL];
+  o[A_XC] = axis == 0 ? T.rxc[e] : axis == 2 ? T.zc[e] : T.yc[e - NPAD - turn(e) * nn] + turn(e) * kTwoPi;
+  if (axis == 0) {
+    o[A_E0] = 1.0 / o[A_XF];
+    o[A_E1] = 1.0 / o[A_XC];
+  } else {
+    const bool az = axis == 1;
+    sincos(o[A_XF], &o[az ? A_E1 : A_E0], &o[az ? A_E0 : A_E1]);
+    sincos(o[A_XC], &o[az ? A_E3 : A_E2], &o[az ? A_E2 : A_E3]);
+    if (!az) {
+      o[A_E4] = 1.0 / o[A_E0];
+      o[A_E5] = 1.0 / o[A_E2];
+    }
+  }
+  double *q = out + (size_t)l * A_COUNT * ARR + table_pos(n, C, G);
+  for (int i = 0; i < A_COUNT; i++) q[i * ARR] = o[i];
+}
+
+// ---------------------------------------------------------------------------
+// Shared block of a radial or polar tile: the warps' workspaces and the
+// per-row values
+struct __align__(16) TileShm {
+  double ws[NW][WS];
+  double row[R_COUNT][ARR];
+  PlanetShm pl;
+};
+// Place of cell n of column cl of a tile in a slot of its warp's workspace
+struct ColMap {
+  int w, l0;                             // the column's warp and first lane
+  __device__ __forceinline__ ColMap(const LaneMap &M, int cl) : w(cl / M.P), l0((cl - cl / M.P * M.P) * M.G) {}
+  template <int C>
+  __device__ __forceinline__ int at(int n) const {
+    const int g = n / C, c = n - g * C;
+    return ws_lane<C>(l0 + g) + (C == 4 ? (c >> 1) * PIECE<4> + (c & 1) : c * PIECE<3>);
+  }
+};
+// Threads of a tile's loads and stores: thread t keeps column t % cols and
+// takes rows t / cols, t / cols + step, ...; threads past the last whole row idle.
+struct TileWalk {
+  int cl, n, step;
+  __device__ __forceinline__ TileWalk(int cols, int tid) : cl(tid % cols), n(tid / cols), step(NT / cols) {
+    if (n >= step) n = 1 << 20;
+  }
+};
+
+// The lane's place in a chunk of lim cells.  Lanes past the warp's last pencil
+// compute on a uniform state of their own, out of every range.
+template <int C, bool HAS_P = true>
+__device__ __forceinline__ int place_lane(Lane<C> &L, const LaneMap &M, int lim, const double *tab, const double *row,
+                                          double *ws, int lane) {
+  const int pw = min(lane / M.G, M.P - 1), g = min(lane - pw * M.G, M.G - 1);
+  const bool idle = lane >= M.P * M.G;
+  L.n0 = idle ? 1 << 20 : C * g;
+  L.lim = lim;
+  L.tab = tab + (C == 4 ? 2 * g : g);
+  L.row = row + (C == 4 ? 2 * g : g);
+  L.half = C == 4 ? 2 * M.G : M.G;
+  L.ws = ws + ws_lane<C>(lane);
+  if (idle) {
+    double one[C], zero[C];
+    PG_CELLS {
+      one[c] = 1.0;
+      zero[c] = 0.0;
+    }
+    put<C>(L, W_R, one);
+    if (HAS_P) put<C>(L, W_P, one);
+    put<C>(L, W_U, zero);
+    put<C>(L, W_V, zero);
+    put<C>(L, W_W, zero);
+  }
+  return C * g;
+}
+
+// ---------------------------------------------------------------------------
+// radial sweep: tile t of the run
+template <class RT, bool THREED, int EOS>
+__device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const PlanesT<RT> &P, const Phys &ph,
+                                             const StepIn &st, int t) {
+  constexpr int C = 4;
+  const int nphi = T.nphi, nrg = T.nrg, full = T.cx.loop - 1, tid = threadIdx.x;
+  int l, k, j0;
+  const int nfull = full * ((nphi + NW - 1) / NW) * T.nk;
+  if (t < nfull) {
+    const int ng = (nphi + NW - 1) / NW;
+    j0 = (t % ng) * NW;
+    l = (t / ng) % full;
+    k = t / (ng * full);
+  } else {
+    const int w = NW * LaneMap(T.cx.stuck ? ARR : T.cx.lim_last, C).P, ng = (nphi + w - 1) / w;
+    t -= nfull;
+    j0 = (t % ng) * w;
+    l = full;
+    k = t / ng;
+  }
+  const bool last = l == full;
+  if (last && T.cx.stuck) {
+    // ppm.cu:48 gives this chunk lim = 12: its rings keep their values
+#pragma unroll 1
+    for (int q = tid; q < REAL * NW; q += NT) {
+      const int i = REAL * l + q / NW, j = j0 + q % NW;
+      if (i >= T.nr || j >= nphi) continue;
+      const size_t o = ((size_t)k * nrg + i + NPAD) * nphi + j;
+      P.ro[o] = P.r[o]; P.uo[o] = P.u[o]; P.vo[o] = P.v[o];
+      if (THREED) P.wo[o] = P.w[o];
+    }
+    return;
+  }
+  const int lim = last ? T.cx.lim_last : ARR, row0 = REAL * l;
+  const LaneMap M(lim, C);
+  const int cols = NW * M.P, rows = C * M.G;
+  const TileWalk W(cols, tid);
+  const ColMap cm(M, W.cl);
+  double *const cw = S.ws[cm.w];
+  // every load of the tile in flight before the first is used
+  RT a[4][4];
+  double rc[4], cs2[4], p0[4], bs[4], bv[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int n = W.n + i * W.step;
+    if (n >= rows) break;
+    const int rk = k * nrg + min(row0 + n, nrg - 1);
+    const size_t o = (size_t)rk * nphi + min(j0 + W.cl, nphi - 1);
+    a[i][0] = __ldcg(&P.r[o]);
+    a[i][1] = __ldcg(&P.u[o]);
+    a[i][2] = __ldcg(&P.v[o]);
+    if (THREED) a[i][3] = __ldcg(&P.w[o]);
+    if (P.p0) p0[i] = P.p0[o];
+    rc[i] = T.radc[rk];
+    cs2[i] = T.cs2[rk];
+    if (sizeof(RT) == 4) {
+      bs[i] = T.sbg[rk];
+      bv[i] = T.vbg[rk];
+    }
+  }
+  if (tid < rows) {
+    const int rk = k * nrg + min(row0 + tid, nrg - 1);
+    const double snd = T.snd[rk], nu = T.nu[rk], r = T.radc[rk], irc = T.irc[rk], res = T.res_v[rk];
+    const int q = table_pos(tid, C, M.G);
+    S.row[R_SND][q] = snd;
+    double sh, ch;
+    sincos_near(0.5 * st.dt * (res * irc - st.pl.vy), sh, ch);
+    S.row[R_CH][q] = ch;
+    S.row[R_SH][q] = sh;
+    S.row[R_NU][q] = nu;
+    S.row[R_RC][q] = r;
+    S.row[R_IRC][q] = irc;
+  }
+  planet_shm<THREED>(S.pl, st, ph);
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int n = W.n + i * W.step;
+    if (n >= rows) break;
+    const int s = cm.at<C>(n);
+    const double r = load_r(a[i][0], bs[i]);
+    cw[W_R * SLOT + s] = r;
+    cw[W_U * SLOT + s] = (double)a[i][1];
+    cw[W_V * SLOT + s] = load_r(a[i][2], bv[i]) * rc[i];
+    if (THREED) cw[W_W * SLOT + s] = (double)a[i][3];
+    cw[W_P * SLOT + s] = P.p0 ? p0[i] : EOS == 0 ? r * cs2[i] : cs2[i] * pow_call(r, ph.gam) / ph.gam;
+  }
+  __syncthreads();
+  {
+    const int lane = tid & 31, wid = tid >> 5;
+    const PlanetC pl = S.pl.p;
+    Lane<C> L;
+    place_lane<C>(L, M, lim, T.ax[0] + (size_t)l * A_COUNT * ARR, S.row[0], S.ws[wid], lane);
+    L.dt = st.dt;
+    {
+      // cos and sin of the column's azimuth less the planet's
+      const int j = min(j0 + wid * M.P + min(lane / M.G, M.P - 1), nphi - 1);
+      const double cy = T.cyc[j], sy = T.syc[j];
+      L.sp = THREED ? T.szc[k + NPAD] : 1.0;
+      L.isp2 = THREED ? 1.0 / (L.sp * L.sp) : 1.0;
+      L.c0 = fma(cy, S.pl.cy, sy * S.pl.sy) * L.sp;
+      L.s0 = fma(sy, S.pl.cy, -(cy * S.pl.sy)) * L.sp;
+    }
+    if (THREED) {
+      double x[C], w[C];
+      ld<C>(L, A_XC, x);
+      get<C>(L, W_W, w);
+      PG_CELLS w[c] *= x[c];
+      put<C>(L, W_W, w);
+    }
+    {
+      double cs[C];
+      ld<C>(L, A_IW, cs);
+      if (EOS == 0 && !P.p0) {
+        double snd[C];
+        ld_row<C>(L, R_SND, snd);
+        PG_CELLS cs[c] = 0.5 * st.dt * snd[c] * cs[c];
+      } else {
+        double p[C], r[C];
+        get<C>(L, W_P, p);
+        get<C>(L, W_R, r);
+        PG_CELLS {
+          const double x = ph.gam * p[c] * rcp(r[c]);
+          cs[c] = 0.5 * st.dt * (x * rsq(x)) * cs[c];
+        }
+      }
+      warp_chain<0, THREED, EOS, C>(L, pl, ph, cs);
+    }
+    // device_viscosity_r viscosity.cu:370-421; the stored v_phi is v / r_cyl
+    double irc[C], rc[C], v[C];
+    ld_row<C>(L, R_IRC, irc);
+    ld_row<C>(L, R_RC, rc);
+    get<C>(L, W_V, v);
+    PG_CELLS v[c] = quot(v[c], rc[c], irc[c]);
+    if (ph.visc) {
+      double a[C], nr[C], n1[C], d1[C], d2[C], dtr[C];
+      Deriv<C> D;
+      D.load(L);
+      get<C>(L, W_R, a);
+      ld_row<C>(L, R_NU, nr);
+      PG_CELLS {
+        nr[c] *= a[c];
+        dtr[c] = st.dt * rcp(a[c]);
+      }
+      D.of(nr, n1, d2);
+      get<C>(L, W_U, a);
+      D.of(a, d1, d2);
+      PG_CELLS a[c] = fma(2.0 * dtr[c], fma(nr[c], fma(irc[c], fma(-a[c], irc[c], d1[c]), d2[c]), n1[c] * d1[c]), a[c]);
+      put<C>(L, W_U, a);
+      PG_CELLS a[c] = v[c] * irc[c];
+      D.of(a, d1, d2);
+      PG_CELLS {
+        const double x = fma(rc[c], fma(nr[c], d2[c], n1[c] * d1[c]), 3.0 * nr[c] * d1[c]);
+        v[c] = fma(dtr[c], x, v[c]);
+      }
+      if (THREED) {
+        get<C>(L, W_W, a);
+        D.of(a, d1, d2);
+        PG_CELLS a[c] = fma(dtr[c], fma(nr[c], fma(d1[c], irc[c], d2[c]), n1[c] * d1[c]), a[c]);
+        put<C>(L, W_W, a);
+      }
+    }
+    put<C>(L, W_V, v);
+    if (THREED) {
+      double w[C], x[C], ix[C];
+      get<C>(L, W_W, w);
+      ld<C>(L, A_XC, x);
+      ld<C>(L, A_E1, ix);
+      PG_CELLS w[c] = quot(w[c], x[c], ix[c]);
+      put<C>(L, W_W, w);
+    }
+  }
+  __syncthreads();
+  if (j0 + W.cl < nphi) {
+#pragma unroll 2
+    for (int n = W.n + NPAD; n < lim - NPAD; n += W.step) {
+      const int rk = k * nrg + row0 + n;
+      const size_t o = (size_t)rk * nphi + j0 + W.cl;
+      const double bs = sizeof(RT) == 4 ? T.sbg[rk] : 0.0, bv = sizeof(RT) == 4 ? T.vbg[rk] : 0.0;
+      const int s = cm.at<C>(n);
+      P.ro[o] = store_r<RT>(cw[W_R * SLOT + s], bs);
+      P.uo[o] = (RT)cw[W_U * SLOT + s];
+      P.vo[o] = store_r<RT>(cw[W_V * SLOT + s], bv);
+      if (THREED) P.wo[o] = (RT)cw[W_W * SLOT + s];
+    }
+  }
+}
+
+template <class RT, bool THREED, int EOS>
+__global__ void __launch_bounds__(NT, MINB) k_sweep_x(Tables T, PlanesT<RT> P, Phys ph, SweepCtl ctl) {
+  extern __shared__ __align__(16) unsigned char shm[];
+  StepIn st;
+  if (!load_step(ctl, st)) return;
+  sweep_x_tile<RT, THREED, EOS>(*reinterpret_cast<TileShm *>(shm), T, P, ph, st, blockIdx.x);
+}
+
+// ---------------------------------------------------------------------------
+// The last sweep's epilogue on one finished cell of ring rk, layer k: damping
+// on the stored state, the next get_dt's CFL rate and the finiteness check.
+// Values are those that the separate kernels (k_damp, k_cfl) form.
+template <class RT>
+struct Finish {
+  double f, tr, tu, tv;                  // damping factor (0: none) and targets
+  double cs, irdx, off, irc, iwz;        // sound speed (EOS 0), 1/dr, frame offset, 1/r_cyl, 1/(r dtheta)
+  double bs, bv, cs2;
+  int rot;                               // rot_j after the step's shift
+  __device__ __forceinline__ void ring(const Tables &T, const SweepCtl &ctl, const StepIn &st, int rk, int row, int kz, int inc) {
+    bs = sizeof(RT) == 4 ? T.sbg[rk] : 0.0;
+    bv = sizeof(RT) == 4 ? T.vbg[rk] : 0.0;
+    f = 0.0;
+    if (!ctl.fuse) return;
+    const double g = T.damp_g[rk];
+    if (g > 0.0) {
+      f = g * (st.dt * T.damp_pw[rk]);
+      tr = T.val_r[rk]; tu = T.val_u[rk]; tv = T.val_v[rk];
+    }
+    cs2 = T.cs2[rk];
+    cs = T.snd[rk];
+    irdx = T.irdx[row];
+    irc = T.irc[rk];
+    off = fma(st.frrot_next, T.radc[rk], T.rot_v[rk]);
+    iwz = kz >= 0 ? T.idz[kz] * T.irxc[row] : 0.0;
+    rot = wrapm(T.rot_j[rk] + inc, T.nphi);
+  }
+  // stores the cell at offset o (azimuth column jo) and returns its CFL rate
+  template <bool THREED, int EOS>
+  __device__ __forceinline__ double cell(const Tables &T, const PlanesT<RT> &P, const SweepCtl &ctl, const Phys &ph, size_t o,
+                                         int jo, double r, double u, double v, double w, bool &bad) const {
+    RT sr = store_r<RT>(r, bs), su = (RT)u, sv = store_r<RT>(v, bv), sw = (RT)w;
+    double rate = 0.0;
+    if (ctl.fuse) {
+      if (f > 0.0) {
+        sr = store_r<RT>(damped(load_r(sr, bs), tr, f), bs);
+        su = (RT)damped((double)su, tu, f);
+        sv = store_r<RT>(damped(load_r(sv, bv), tv, f), bv);
+        if (THREED) sw = (RT)damped((double)sw, 0.0, f);
+      }
+      r = load_r(sr, bs);
+      v = load_r(sv, bv);
+      if (!ctl.nocfl) {
+        const double a = EOS == 0 ? cs : sound_speed(r, eos_p<EOS>(r, cs2, ph), ph);
+        int js = jo - rot;
+        if (js < 0) js += T.nphi;
+        rate = cfl_rate<THREED>(a, (double)su, irdx, v - off, T.idy[js] * irc, (double)sw, iwz);
+      }
+      if (!(r > 0.0) || !isfinite(r) || !isfinite((double)su) || !isfinite(v)) bad = true;
+    }
+    P.ro[o] = sr; P.uo[o] = su; P.vo[o] = sv;
+    if (THREED) P.wo[o] = sw;
+    return rate;
+  }
+};
+
+// a warp's CFL maximum and failure flag into the clock
+__device__ __forceinline__ void report(const SweepCtl &ctl, double rate, bool bad) {
+  for (int o = 16; o > 0; o >>= 1) {
+    const double x = __shfl_down_sync(0xffffffffu, rate, o);
+    rate = (x > rate || x != x) ? x : rate;
+  }
+  bad = __any_sync(0xffffffffu, bad);
+  if ((threadIdx.x & 31) == 0) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(rate);
+    // NaN sorts above every number; most warps are below the maximum so far
+    if ((rate > 0.0 || rate != rate) && b > *(volatile unsigned long long *)&ctl.clk->cfl_bits)
+      atomicMax(&ctl.clk->cfl_bits, b);
+    if (bad) atomicExch(&ctl.clk->status, 3);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// azimuthal sweep: warp task t of the run
+template <int EOS>
+struct __align__(16) YShm {
+  double ws[NW][EOS ? WS : WS_ISO_Y];
+  PlanetShm pl;
+};
+template <class RT, bool THREED, int EOS>
+__device__ __forceinline__ void sweep_y_task(double *ws, const PlanetShm &SP, const Tables &T, const PlanesT<RT> &P,
+                                             const Phys &ph, const SweepCtl &ctl, const StepIn &st, int t) {
+  constexpr int C = 4;
+  const int nphi = T.nphi, nrg = T.nrg, full = T.cy.loop - 1, rings = T.nr * T.nk, lane = threadIdx.x & 31;
+  int l = full, ring, lim = T.cy.lim_last;
+  // the tasks of full chunks fill whole CTAs, so that a CTA's warps take the
+  // chain's barriers together; tasks past the last ring compute and store nothing
+  const int nfull = (rings + NW - 1) / NW * NW;
+  if (t < full * nfull) {
+    // rings of one chunk side by side: the warps of an SM share its tables
+    l = t / nfull;
+    ring = t % nfull;
+    lim = ARR;
+  } else if (T.cy.stuck) {
+    ring = t - full * nfull;
+    if (ring >= rings) return;
+    // ppm.cu:196 gives this chunk lim = 12: its cells keep their values and
+    // only move with the ring's rotation
+    const int k = ring / T.nr, row = ring % T.nr + NPAD, rk = k * nrg + row;
+    const size_t base = (size_t)rk * nphi;
+    const int inc = ctl.shift ? wrapm(T.inc_j[rk], nphi) : 0;
+    Finish<RT> F;
+    F.ring(T, ctl, st, rk, row, THREED ? k + NPAD : -1, ctl.shift ? T.inc_j[rk] : 0);
+    double rate = 0.0;
+    bool bad = false;
+#pragma unroll 1
+    for (int j = REAL * l + lane; j < nphi; j += 32) {
+      int jo = j + inc;
+      if (jo >= nphi) jo -= nphi;
+      const size_t s = base + j;
+      const double x = F.template cell<THREED, EOS>(T, P, ctl, ph, base + jo, jo, load_r(P.r[s], F.bs), (double)P.u[s],
+                                                    load_r(P.v[s], F.bv), THREED ? (double)P.w[s] : 0.0, bad);
+      rate = (x > rate || x != x) ? x : rate;
+    }
+    if (ctl.fuse) report(ctl, rate, bad);
+    return;
+  } else {
+    ring = (t - full * nfull) * LaneMap(lim, C).P;
+  }
+  const LaneMap M(lim, C);
+  {
+    const int q = min(ring + min(lane / M.G, M.P - 1), rings - 1), k = q / T.nr, row = q % T.nr + NPAD, rk = k * nrg + row;
+    Lane<C> L;
+    const int n0 = place_lane<C, (EOS != 0)>(L, M, lim, T.ax[1] + (size_t)l * A_COUNT * ARR, ws, ws, lane);
+    // all loads in flight before the first is used; the four cells of a lane
+    // share their sectors in L1
+    const size_t base = (size_t)rk * nphi;
+    RT x[4][C];
+    PG_CELLS {
+      int j = REAL * l - NPAD + n0 + c;
+      j = j < 0 ? j + nphi : j >= nphi ? j - nphi : j;
+      x[0][c] = P.r[base + j];
+      x[1][c] = P.v[base + j];
+      if (THREED) x[2][c] = P.w[base + j];
+      x[3][c] = P.u[base + j];
+    }
+    const double bs = sizeof(RT) == 4 ? T.sbg[rk] : 0.0, bv = sizeof(RT) == 4 ? T.vbg[rk] : 0.0;
+    L.dt = st.dt;
+    L.frrot = st.frrot;
+    L.rad = T.radc[rk];
+    L.irad = T.irc[rk];
+    L.sp = THREED ? T.szc[k + NPAD] : 1.0;
+    L.vr = T.res_v[rk] * L.irad;
+    L.cs2 = T.cs2[rk];
+    const double snd = T.snd[rk], rs = T.rxc[row];
+    // the planet's constants, formed meanwhile by the CTA's last warp
+    __syncthreads();
+    const PlanetC pl = SP.p;
+    {
+      L.bq = fma(rs, rs, pl.b2);         // the planet's distance sees the spherical radius in 3D
+      const double a = 0.5 * st.dt * (L.vr - pl.vy);
+      double s, c;
+      L.ca = SP.cy; L.sa = -SP.sy;
+      sincos_near(a, s, c);
+      L.cb = fma(L.ca, c, -(L.sa * s)); L.sb = fma(L.sa, c, L.ca * s);
+      L.cc = fma(L.cb, c, -(L.sb * s)); L.sc = fma(L.sb, c, L.cb * s);
+    }
+    {
+      double q[C];
+      PG_CELLS q[c] = load_r(x[0][c], bs);
+      put<C>(L, W_R, q);
+      PG_CELLS q[c] = load_r(x[1][c], bv);
+      put<C>(L, W_U, q);
+      if (THREED) {
+        PG_CELLS q[c] = (double)x[2][c];
+        put<C>(L, W_V, q);
+      }
+      PG_CELLS q[c] = (double)x[3][c];
+      put<C>(L, W_W, q);
+    }
+    double cs[C];
+    {
+      ld<C>(L, A_IW, cs);
+      if (EOS == 0) {
+        L.ciso = L.cs2 * rsq(L.cs2);
+        L.low = max(kTiny, __double2hiint(1.0e-14 * rcp(L.cs2)) + 1);
+        const double a = 0.5 * st.dt * snd * L.irad;
+        PG_CELLS cs[c] *= a;
+      } else {
+        double p[C], r[C];
+        get<C>(L, W_R, r);
+        PG_CELLS {
+          p[c] = L.cs2 * pow_call(r[c], ph.gam) / ph.gam;
+          const double x2 = ph.gam * p[c] * rcp(r[c]);
+          cs[c] *= 0.5 * st.dt * (x2 * rsq(x2)) * L.irad;
+        }
+        put<C>(L, W_P, p);
+      }
+    }
+    warp_chain<1, THREED, EOS, C>(L, pl, ph, cs);
+    // device_viscosity_p viscosity.cu:423-472 on x = r_cyl phi
+    if (ph.visc) {
+      const double nu = T.nu[rk], ir = L.irad;
+      double a[C], nr[C], n1[C], d1[C], d2[C], dtr[C];
+      Deriv<C> D;
+      D.load(L);
+      get<C>(L, W_R, a);
+      PG_CELLS {
+        nr[c] = nu * a[c];
+        dtr[c] = st.dt * (ir * ir) * rcp(a[c]);
+      }
+      D.of(nr, n1, d2);
+#pragma unroll 1
+      for (int f = W_U; f <= W_W; f++) {
+        if (!THREED && f == W_V) continue;
+        const double two = f == W_U ? 2.0 : 1.0;
+        get<C>(L, f, a);
+        D.of(a, d1, d2);
+        PG_CELLS a[c] = fma(two * dtr[c], fma(nr[c], d2[c], n1[c] * d1[c]), a[c]);
+        put<C>(L, f, a);
+      }
+    }
+  }
+  __syncwarp();
+  double rate = 0.0;
+  bool bad = false;
+  const int len = lim - 2 * NPAD;
+#pragma unroll 1
+  for (int b = 0; b < M.P && ring + b < rings; b++) {
+    const int q = ring + b, k = q / T.nr, row = q % T.nr + NPAD, rk = k * nrg + row;
+    const size_t base = (size_t)rk * nphi;
+    const int inc = ctl.shift ? T.inc_j[rk] : 0, im = wrapm(inc, nphi);
+    const ColMap cm(M, b);
+    Finish<RT> F;
+    F.ring(T, ctl, st, rk, row, THREED ? k + NPAD : -1, inc);
+#pragma unroll 1
+    for (int m = lane; m < len; m += 32) {
+      const int s = cm.at<C>(m + NPAD);
+      int jo = REAL * l + m + im;
+      if (jo >= nphi) jo -= nphi;
+      const double x = F.template cell<THREED, EOS>(T, P, ctl, ph, base + jo, jo, ws[W_R * SLOT + s], ws[W_W * SLOT + s],
+                                                    ws[W_U * SLOT + s], THREED ? ws[W_V * SLOT + s] : 0.0, bad);
+      rate = (x > rate || x != x) ? x : rate;
+    }
+  }
+  if (ctl.fuse) report(ctl, rate, bad);
+}
+
+template <class RT, bool THREED, int EOS>
+__global__ void __launch_bounds__(NT, MINB) k_sweep_y(Tables T, PlanesT<RT> P, Phys ph, SweepCtl ctl) {
+  extern __shared__ __align__(16) unsigned char shm[];
+  YShm<EOS> &S = *reinterpret_cast<YShm<EOS> *>(shm);
+  StepIn st;
+  if (!load_step(ctl, st)) return;
+  planet_shm<THREED>(S.pl, st, ph);
+  const int wid = threadIdx.x >> 5;
+  sweep_y_task<RT, THREED, EOS>(S.ws[wid], S.pl, T, P, ph, ctl, st, blockIdx.x * NW + wid);
+}
+
+// ---------------------------------------------------------------------------
+// polar-angle sweep (3D, ngeomz 5): no reference kernel exists
+// (bundle_sweep3D is called at main.cu:376 and never defined).  Modelled on
+// the radial sweep: pencils along k for one (i, phi column), fixed lower
+// layers (init.cpp:415-476) and a reflecting midplane (boundary.cu:412-418,
+// mirror with v_theta negated) or fixed upper layers.  Slots: u <- v_theta,
+// v <- v_r, w <- r sin(theta) v_phi (so get_fz's w^2 cos/(r sin)^3 is the
+// centrifugal term); viscosity follows device_viscosity_p's pattern on the
+// arc length r*theta.  A tile is 4 P columns of one ring, so its row values
+// (one layer per row) are shared by the whole CTA.
+template <class RT, int EOS, int C>
+__device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const PlanesT<RT> &P, const Phys &ph,
+                                             const SweepCtl &ctl, const StepIn &st, int ntop, int t) {
+  const int nphi = T.nphi, nrg = T.nrg, nk = T.nk, full = T.cz.loop - 1, tid = threadIdx.x;
+  int l, i, j0;
+  const int nfull = full * ((nphi + NW - 1) / NW) * T.nr;
+  if (t < nfull) {
+    const int ng = (nphi + NW - 1) / NW;
+    j0 = (t % ng) * NW;
+    i = (t / ng) % T.nr;
+    l = t / (ng * T.nr);
+  } else {
+    const int w = NW * LaneMap(T.cz.stuck ? ARR : T.cz.lim_last, C).P, ng = (nphi + w - 1) / w;
+    t -= nfull;
+    j0 = (t % ng) * w;
+    i = t / ng;
+    l = full;
+  }
+  const int row = i + NPAD;
+  const bool last = l == full;
+  if (last && T.cz.stuck) {
+#pragma unroll 1
+    for (int q = tid; q < REAL * NW; q += NT) {
+      const int k = REAL * l + q / NW, j = j0 + q % NW;
+      if (k >= nk || j >= nphi) continue;
+      const int rk = k * nrg + row;
+      int jo = j + (ctl.shift ? wrapm(T.inc_j[rk], nphi) : 0);
+      if (jo >= nphi) jo -= nphi;
+      const size_t s = (size_t)rk * nphi + j, o = (size_t)rk * nphi + jo;
+      P.ro[o] = P.r[s]; P.uo[o] = P.u[s]; P.vo[o] = P.v[s]; P.wo[o] = P.w[s];
+    }
+    return;
+  }
+  const int lim = last ? T.cz.lim_last : ARR, k0 = REAL * l - NPAD;
+  const LaneMap M(lim, C);
+  const int cols = NW * M.P, rows = C * M.G;
+  const double rad = T.rxc[row];
+  const TileWalk W(cols, tid);
+  const ColMap cm(M, W.cl);
+  double *const cw = S.ws[cm.w];
+  // every load of the tile in flight before the first is used; a ghost layer
+  // below or a fixed one above comes from the ghost tables (no FARGO
+  // residual), a mirrored one from its mirror image
+  RT a[4][4];
+  double rc[4], cs2[4], bs[4], bv[4];
+#pragma unroll
+  for (int i4 = 0; i4 < 4; i4++) {
+    const int n = W.n + i4 * W.step;
+    if (n >= rows) break;
+    const int kr = min(k0 + n, nk + NPAD - 1);
+    rc[i4] = (kr >= 0 && kr < nk) ? T.radc[kr * nrg + row] : rad * T.szc[kr + NPAD];
+    if (kr >= 0 && (kr < nk || ntop == 0)) {
+      const int km = kr >= nk ? 2 * nk - 1 - kr : kr, rk = km * nrg + row;
+      const size_t o = (size_t)rk * nphi + min(j0 + W.cl, nphi - 1);
+      a[i4][0] = __ldcg(&P.r[o]);
+      a[i4][1] = __ldcg(&P.u[o]);
+      a[i4][2] = __ldcg(&P.v[o]);
+      a[i4][3] = __ldcg(&P.w[o]);
+      cs2[i4] = T.cs2[rk];
+      bs[i4] = sizeof(RT) == 4 ? T.sbg[rk] : 0.0;
+      bv[i4] = sizeof(RT) == 4 ? T.vbg[rk] : 0.0;
+    }
+  }
+  if (tid < rows) {
+    const int kr = min(k0 + tid, nk + NPAD - 1);
+    const bool fixed = kr < 0 || (kr >= nk && ntop != 0);
+    const int km = kr >= nk ? 2 * nk - 1 - kr : kr, rk = km * nrg + row;
+    const int gq = (kr < 0 ? kr + NPAD : kr - nk + NPAD) * T.nr + i;
+    const int q = table_pos(tid, C, M.G);
+    S.row[R_SND][q] = fixed ? sqrt(ph.gam * T.csg[gq]) : T.snd[rk];
+    double sh, ch;
+    sincos_near(0.5 * st.dt * ((fixed ? 0.0 : T.res_v[rk] * T.irc[rk]) - st.pl.vy), sh, ch);
+    S.row[R_CH][q] = ch;
+    S.row[R_SH][q] = sh;
+    S.row[R_NU][q] = (kr >= 0 && kr < nk) ? T.nu[rk] : T.nug[gq];
+  }
+  planet_shm<true>(S.pl, st, ph);
+#pragma unroll
+  for (int i4 = 0; i4 < 4; i4++) {
+    const int n = W.n + i4 * W.step;
+    if (n >= rows) break;
+    const int kr = min(k0 + n, nk + NPAD - 1), s = cm.at<C>(n);
+    double r, p, vt, vr, vp;
+    if (kr < 0 || (kr >= nk && ntop != 0)) {
+      const double *g = T.tg + ((size_t)(kr < 0 ? kr + NPAD : NPAD + kr - nk) * T.nr + i) * 4;
+      r = g[0]; p = g[1]; vr = g[2]; vp = g[3];
+      vt = 0.0;
+    } else {
+      r = load_r(a[i4][0], bs[i4]);
+      vr = (double)a[i4][1];
+      vp = load_r(a[i4][2], bv[i4]);
+      vt = kr >= nk ? -(double)a[i4][3] : (double)a[i4][3];
+      p = EOS == 0 ? r * cs2[i4] : cs2[i4] * pow_call(r, ph.gam) / ph.gam;
+    }
+    cw[W_R * SLOT + s] = r;
+    cw[W_U * SLOT + s] = vt;
+    cw[W_V * SLOT + s] = vr;
+    cw[W_W * SLOT + s] = vp * rc[i4];
+    cw[W_P * SLOT + s] = p;
+  }
+  __syncthreads();
+  {
+    const int lane = tid & 31, wid = tid >> 5;
+    const PlanetC pl = S.pl.p;
+    Lane<C> L;
+    place_lane<C>(L, M, lim, T.ax[2] + (size_t)l * A_COUNT * ARR, S.row[0], S.ws[wid], lane);
+    L.dt = st.dt;
+    L.rad = rad;
+    L.irad = T.irxc[row];
+    L.bq = fma(rad, rad, pl.b2);
+    {
+      const int j = min(j0 + wid * M.P + min(lane / M.G, M.P - 1), nphi - 1);
+      const double cy = T.cyc[j], sy = T.syc[j];
+      L.c0 = fma(cy, S.pl.cy, sy * S.pl.sy);
+      L.s0 = fma(sy, S.pl.cy, -(cy * S.pl.sy));
+    }
+    {
+      double cs[C];
+      ld<C>(L, A_IW, cs);
+      const double a = 0.5 * st.dt * L.irad;
+      if (EOS == 0) {
+        double snd[C];
+        ld_row<C>(L, R_SND, snd);
+        PG_CELLS cs[c] = a * snd[c] * cs[c];
+      } else {
+        double p[C], r[C];
+        get<C>(L, W_P, p);
+        get<C>(L, W_R, r);
+        PG_CELLS {
+          const double x = ph.gam * p[c] * rcp(r[c]);
+          cs[c] = a * (x * rsq(x)) * cs[c];
+        }
+      }
+      warp_chain<2, true, EOS, C>(L, pl, ph, cs);
+    }
+    if (ph.visc) {
+      double a[C], nr[C], n1[C], d1[C], d2[C], dtr[C];
+      Deriv<C> D;
+      D.load(L);
+      get<C>(L, W_R, a);
+      ld_row<C>(L, R_NU, nr);
+      PG_CELLS {
+        nr[c] *= a[c];
+        dtr[c] = st.dt * (L.irad * L.irad) * rcp(a[c]);
+      }
+      D.of(nr, n1, d2);
+#pragma unroll 1
+      for (int f = W_U; f <= W_V; f++) {
+        const double two = f == W_U ? 2.0 : 1.0;
+        get<C>(L, f, a);
+        D.of(a, d1, d2);
+        PG_CELLS a[c] = fma(two * dtr[c], fma(nr[c], d2[c], n1[c] * d1[c]), a[c]);
+        put<C>(L, f, a);
+      }
+    }
+  }
+  __syncthreads();
+  // the polar sweep is the last of a 3D step: the FARGO integer shift of each
+  // layer (rotate_rings, ppm.cu:309-322) is applied at this store.  What the
+  // epilogue needs of a layer's ring is formed once per row.
+  const int len = lim - 2 * NPAD;
+#pragma unroll 1
+  for (int m = tid; m < len; m += NT) {
+    const int k = k0 + m + NPAD, rk = k * nrg + row, inc = ctl.shift ? T.inc_j[rk] : 0;
+    Finish<RT> F;
+    F.ring(T, ctl, st, rk, row, k + NPAD, inc);
+    S.row[R_F][m] = F.f;
+    S.row[R_TR][m] = F.tr;
+    S.row[R_TU][m] = F.tu;
+    S.row[R_TV][m] = F.tv;
+    S.row[R_OFF][m] = F.off;
+    S.row[R_IWZ][m] = F.iwz;
+    reinterpret_cast<int2 *>(S.row[R_J])[m] = make_int2(wrapm(inc, nphi), F.rot);
+  }
+  __syncthreads();
+  double rate = 0.0;
+  bool bad = false;
+  if (j0 + W.cl < nphi) {
+    Finish<RT> F;
+    F.irdx = T.irdx[row];
+#pragma unroll 1
+    for (int m = W.n; m < len; m += W.step) {
+      const int rk = (k0 + m + NPAD) * nrg + row, s = cm.at<C>(m + NPAD);
+      const int2 sh = reinterpret_cast<const int2 *>(S.row[R_J])[m];
+      F.f = S.row[R_F][m]; F.tr = S.row[R_TR][m]; F.tu = S.row[R_TU][m]; F.tv = S.row[R_TV][m];
+      F.off = S.row[R_OFF][m]; F.iwz = S.row[R_IWZ][m];
+      F.rot = sh.y;
+      F.cs = T.snd[rk];
+      F.cs2 = T.cs2[rk];
+      F.irc = T.irc[rk];
+      F.bs = sizeof(RT) == 4 ? T.sbg[rk] : 0.0;
+      F.bv = sizeof(RT) == 4 ? T.vbg[rk] : 0.0;
+      int jo = j0 + W.cl + sh.x;
+      if (jo >= nphi) jo -= nphi;
+      const double x = F.template cell<true, EOS>(T, P, ctl, ph, (size_t)rk * nphi + jo, jo, cw[W_R * SLOT + s],
+                                                  cw[W_V * SLOT + s], quot(cw[W_W * SLOT + s], T.radc[rk], F.irc),
+                                                  cw[W_U * SLOT + s], bad);
+      rate = (x > rate || x != x) ? x : rate;
+    }
+  }
+  if (ctl.fuse) report(ctl, rate, bad);
+}
+
+template <class RT, int EOS, int C>
+__global__ void __launch_bounds__(NT, MINB) k_sweep_z(Tables T, PlanesT<RT> P, Phys ph, SweepCtl ctl, int ntop) {
+  extern __shared__ __align__(16) unsigned char shm[];
+  StepIn st;
+  if (!load_step(ctl, st)) return;
+  sweep_z_tile<RT, EOS, C>(*reinterpret_cast<TileShm *>(shm), T, P, ph, ctl, st, ntop, blockIdx.x);
+}
+
+// ---------------------------------------------------------------------------
+// Batched 2D sweeps: one launch walks the tiles of every run of a group; CTA
+// b takes tiles b, b + grid, ...  Each tile runs the same code as in the
+// run's own launch, so a run's results depend on neither batch nor grid.
+template <class RT>
+__device__ __forceinline__ const PlanesT<RT> &batch_planes(const BatchRun &b, int y) {
+  if constexpr (sizeof(RT) == 4) return y ? b.QY : b.QX;
+  else return y ? b.PY : b.PX;
+}
+
+template <class RT>
+__global__ void __launch_bounds__(NT, MINB) kb_sweep_x(BatchQueue q) {
+  extern __shared__ __align__(16) unsigned char shm[];
+  for (int t = blockIdx.x; t < q.total; t += gridDim.x) {
+    const int r = batch_find(q, t);
+    const BatchRun &b = q.runs[r];
+    SweepCtl ctl{};
+    ctl.clk = b.clk;
+    StepIn st;
+    if (load_step(ctl, st)) {
+      PlanesT<RT> P = batch_planes<RT>(b, 0);
+      P.p0 = (sizeof(RT) == 8 && b.p0 && b.clk->ncycle == b.p0_cycle) ? b.p0 : nullptr;
+      sweep_x_tile<RT, false, 0>(*reinterpret_cast<TileShm *>(shm), b.T, P, b.ph, st, t - q.start[r]);
+    }
+    __syncthreads();
+  }
+}
+
+template <class RT>
+__global__ void __launch_bounds__(NT, MINB) kb_sweep_y(BatchQueue q) {
+  extern __shared__ __align__(16) unsigned char shm[];
+  YShm<0> &S = *reinterpret_cast<YShm<0> *>(shm);
+  const int wid = threadIdx.x >> 5;
+  for (int t = blockIdx.x; t < q.total; t += gridDim.x) {
+    const int r = batch_find(q, t);
+    const BatchRun &b = q.runs[r];
+    SweepCtl ctl{};
+    ctl.clk = b.clk;
+    ctl.fuse = 1;
+    ctl.shift = 1;
+    StepIn st;
+    if (load_step(ctl, st)) {
+      planet_shm<false>(S.pl, st, b.ph);
+      sweep_y_task<RT, false, 0>(S.ws[wid], S.pl, b.T, batch_planes<RT>(b, 1), b.ph, ctl, st, (t - q.start[r]) * NW + wid);
+    }
+    __syncthreads();
+  }
+}
+
+}  // namespace pgd
+
+// ---------------------------------------------------------------------------
+namespace pgk {
+using namespace pgd;
+
+static int pencils_per_warp(int lim, int C) { return 32 / ((lim + C - 1) / C); }
+
+// Cells per lane of the polar sweep: 3 or 4, whichever leaves fewer of the
+// warp's cell slots empty.  The 32-layer disk's pencils of 44 cells fill 88 of
+// 96 slots with 3 (two pencils of 15 lanes) and 88 of 128 with 4; 28 and 36
+// cells fill 112 and 108 of 128 with 4.  Grids of more than one chunk take 4.
+int polar_cells(const Chunking &ch) {
+  if (ch.loop > 1 || ch.stuck) return 4;
+  const int lim = ch.lim_last;
+  if (lim > 96) return 4;
+  return 4 * pencils_per_warp(lim, 3) > 3 * pencils_per_warp(lim, 4) ? 3 : 4;
+}
+
+static int groups(int n, int w) { return (n + w - 1) / w; }
+static int last_group(const Chunking &ch, int C) { return NW * (ch.stuck ? 1 : pencils_per_warp(ch.lim_last, C)); }
+
+// CTAs of a run's radial, azimuthal and polar sweep
+int tiles_x(const Tables &T) {
+  return T.nk * ((T.cx.loop - 1) * groups(T.nphi, NW) + groups(T.nphi, last_group(T.cx, 4)));
+}
+int tiles_y(const Tables &T) {
+  const int rings = T.nr * T.nk;
+  return (T.cy.loop - 1) * groups(rings, NW) + groups(rings, last_group(T.cy, 4));
+}
+static int tiles_z(const Tables &T, int C) {
+  return T.nr * ((T.cz.loop - 1) * groups(T.nphi, NW) + groups(T.nphi, last_group(T.cz, C)));
+}
+
+// the sweeps take their shared blocks (some 12 KB per warp) as dynamic shared
+// memory, above the 48 KiB default limit: set per device before a launch
+int setup_device() {
+  const void *k[] = {(const void *)k_sweep_x<double, false, 0>, (const void *)k_sweep_x<double, true, 0>,
+                     (const void *)k_sweep_x<double, false, 1>, (const void *)k_sweep_x<double, true, 1>,
+                     (const void *)k_sweep_x<float, false, 0>,  (const void *)k_sweep_x<float, true, 0>,
+                     (const void *)k_sweep_z<double, 0, 3>,     (const void *)k_sweep_z<double, 0, 4>,
+                     (const void *)k_sweep_z<double, 1, 3>,     (const void *)k_sweep_z<double, 1, 4>,
+                     (const void *)k_sweep_z<float, 0, 3>,      (const void *)k_sweep_z<float, 0, 4>,
+                     (const void *)kb_sweep_x<double>,          (const void *)kb_sweep_x<float>,
+                     (const void *)k_sweep_y<double, false, 0>, (const void *)k_sweep_y<double, true, 0>,
+                     (const void *)k_sweep_y<double, false, 1>, (const void *)k_sweep_y<double, true, 1>,
+                     (const void *)k_sweep_y<float, false, 0>,  (const void *)k_sweep_y<float, true, 0>,
+                     (const void *)kb_sweep_y<double>,          (const void *)kb_sweep_y<float>};
+  for (const void *f : k)
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileShm)) != cudaSuccess) return 1;
+  return 0;
+}
+
+void axis_tables(const Tables &T, int ndim, cudaStream_t s) {
+  k_axis_table<<<T.cx.loop, ARR, 0, s>>>(T, 0, 4, const_cast<double *>(T.ax[0]));
+  k_axis_table<<<T.cy.loop, ARR, 0, s>>>(T, 1, 4, const_cast<double *>(T.ax[1]));
+  if (ndim == 3) k_axis_table<<<T.cz.loop, ARR, 0, s>>>(T, 2, polar_cells(T.cz), const_cast<double *>(T.ax[2]));
+}
+size_t axis_table_elems(const Chunking &ch) { return (size_t)ch.loop * A_COUNT * ARR; }
+
+template <class RT>
+void sweep_x(const Tables &T, const PlanesT<RT> &P, const Phys &ph, const SweepCtl &c, int ndim, cudaStream_t s) {
+  const int n = tiles_x(T);
+  if constexpr (sizeof(RT) == 8) {
+    if (ph.eos) {
+      if (ndim == 3) k_sweep_x<RT, true, 1><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c);
+      else k_sweep_x<RT, false, 1><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c);
+      return;
+    }
+  }
+  if (ndim == 3) k_sweep_x<RT, true, 0><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c);
+  else k_sweep_x<RT, false, 0><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c);
+}
+
+template <class RT>
+void sweep_y(const Tables &T, const PlanesT<RT> &P, const Phys &ph, const SweepCtl &c, int ndim, cudaStream_t s) {
+  const int n = tiles_y(T);
+  if constexpr (sizeof(RT) == 8) {
+    if (ph.eos) {
+      if (ndim == 3) k_sweep_y<RT, true, 1><<<n, NT, sizeof(YShm<1>), s>>>(T, P, ph, c);
+      else k_sweep_y<RT, false, 1><<<n, NT, sizeof(YShm<1>), s>>>(T, P, ph, c);
+      return;
+    }
+  }
+  if (ndim == 3) k_sweep_y<RT, true, 0><<<n, NT, sizeof(YShm<0>), s>>>(T, P, ph, c);
+  else k_sweep_y<RT, false, 0><<<n, NT, sizeof(YShm<0>), s>>>(T, P, ph, c);
+}
+
+template <class RT>
+void sweep_z(const Tables &T, const PlanesT<RT> &P, const Phys &ph, const SweepCtl &c, int ntop, cudaStream_t s) {
+  const int C = polar_cells(T.cz), n = tiles_z(T, C);
+  if constexpr (sizeof(RT) == 8) {
+    if (ph.eos) {
+      if (C == 3) k_sweep_z<RT, 1, 3><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c, ntop);
+      else k_sweep_z<RT, 1, 4><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c, ntop);
+      return;
+    }
+  }
+  if (C == 3) k_sweep_z<RT, 0, 3><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c, ntop);
+  else k_sweep_z<RT, 0, 4><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c, ntop);
+}
+
+template <class RT>
+void batch_sweep_x(const BatchQueue &q, int grid, cudaStream_t s) {
+  if (q.total > 0) kb_sweep_x<RT><<<grid > 0 && grid < q.total ? grid : q.total, NT, sizeof(TileShm), s>>>(q);
+}
+template <class RT>
+void batch_sweep_y(const BatchQueue &q, int grid, cudaStream_t s) {
+  if (q.total > 0) kb_sweep_y<RT><<<grid > 0 && grid < q.total ? grid : q.total, NT, sizeof(YShm<0>), s>>>(q);
+}
+
+#define PG_SWEEPS(RT)                                                                                              \
+  template void sweep_x<RT>(const Tables &, const PlanesT<RT> &, const Phys &, const SweepCtl &, int, cudaStream_t); \
+  template void sweep_y<RT>(const Tables &, const PlanesT<RT> &, const Phys &, const SweepCtl &, int, cudaStream_t); \
+  template void sweep_z<RT>(const Tables &, const PlanesT<RT> &, const Phys &, const SweepCtl &, int, cudaStream_t); \
+  template void batch_sweep_x<RT>(const BatchQueue &, int, cudaStream_t);                                            \
+  template void batch_sweep_y<RT>(const BatchQueue &, int, cudaStream_t);
+PG_SWEEPS(double)
+PG_SWEEPS(float)
+
+}  // namespace pgk
