@@ -13,11 +13,11 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libpenguin_b200.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVFLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2", "--expt-relaxed-constexpr"]
-SOURCES = ["pg_host.cpp", "pg_kernels.cu", "pg_sweep.cu", "pg_run.cu", "pg_batch.cu", "pg_serve.cpp", "pg_noalloc.cu"]
+SOURCES = ["pg_host.cpp", "pg_kernels.cu", "pg_sweep.cu", "pg_step.cu", "pg_run.cu", "pg_batch.cu", "pg_serve.cpp", "pg_noalloc.cu"]
 
 
-# the sweeps write their fused multiply-adds out (pg_warp.cuh)
-SOURCE_FLAGS = {"pg_sweep.cu": ["-fmad=false"]}
+# these write their fused multiply-adds out (pg_warp.cuh)
+SOURCE_FLAGS = {"pg_sweep.cu": ["-fmad=false"], "pg_step.cu": ["-fmad=false"]}
 
 
 def _newer(out, deps):

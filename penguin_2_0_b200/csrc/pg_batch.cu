@@ -4,11 +4,9 @@
 // runs (each a pg_run with its own planes, tables, clock and dt) and steps
 // them together:
 //   * 2D members are split by precision into two groups.  For each group a
-//     step is one launch per phase: prestep (one CTA per run: dt, Index_Shift,
-//     half kick), radial sweep and azimuthal sweep (a tile queue over the
-//     pencil chunks of every member; CTA b takes tiles b, b + grid, ...),
-//     poststep, mass and torque reductions (one CTA per ring of every member)
-//     and the history record.
+//     step is one launch per phase: radial sweep and azimuthal sweep (a tile
+//     queue over the pencil chunks of every member; CTA b takes tiles b,
+//     b + grid, ...) and what lies between two steps (a few CTAs per member).
 //   * 3D members, members with a moving planet (plnt_flag 2) and isentropic
 //     members (EOS 1) take their own launch sequence (the per-run fused
 //     step) in the same stream order; the queue kernels are isothermal 2D.
@@ -43,7 +41,7 @@ __global__ void kb_status(pgd::DevClock *const *clks, int n, pg_batch_member *ou
 struct Group {
   std::vector<pg_run *> members;
   pgd::BatchRun *d_runs = nullptr;
-  int *d_start = nullptr;          // [3][n+1]: radial tiles, azimuthal tiles, rings
+  int *d_start = nullptr;          // [3][n+1]: radial tiles, azimuthal tiles, CTAs between steps
   size_t cap = 0;
   pgd::BatchQueue qx{}, qy{}, qr{};
   pg_batch_shape shape{0, 0, 8, 0};
@@ -126,7 +124,7 @@ static int rebuild(pg_batch *b) {
       pgi::run_shape(r, &sh);
       st[i + 1] = st[i] + sh.tiles_x;
       st[(n + 1) + i + 1] = st[(n + 1) + i] + sh.tiles_y;
-      st[2 * (n + 1) + i + 1] = st[2 * (n + 1) + i] + sh.nr;
+      st[2 * (n + 1) + i + 1] = st[2 * (n + 1) + i] + sh.ctas_b;
     }
     if (n) {
       BK(cudaMemcpy(g.d_runs, h.data(), n * sizeof(pgd::BatchRun), cudaMemcpyHostToDevice));
@@ -156,33 +154,27 @@ static int rebuild(pg_batch *b) {
   return PG_OK;
 }
 
-// one step of the members of group gi
-static void enqueue_group_step(pg_batch *b, int gi, int64_t *nk) {
-  cudaStream_t s = b->stream;
-  Group &g = b->g[gi];
-  int n = (int)g.members.size();
-  if (!n) return;
-  pgk::batch_prestep(g.d_runs, n, s);
-  if (gi == 1) {
-    pgk::batch_sweep_x<float>(g.qx, g.shape.grid_x, s);
-    pgk::batch_sweep_y<float>(g.qy, g.shape.grid_y, s);
-  } else {
-    pgk::batch_sweep_x<double>(g.qx, g.shape.grid_x, s);
-    pgk::batch_sweep_y<double>(g.qy, g.shape.grid_y, s);
-  }
-  pgk::batch_poststep(g.d_runs, n, s);
-  pgk::batch_reduce(g.qr, gi, 0, s);
-  pgk::batch_reduce(g.qr, gi, 9, s);
-  pgk::batch_record(g.d_runs, n, s);
-  *nk += 7;
+// one step of the members of group gi (first, last: of the sequence being queued)
+template <class RT>
+static void enqueue_group_step(Group &g, bool first, bool last, cudaStream_t s, int64_t *nk) {
+  if (g.members.empty()) return;
+  if (first) pgk::batch_between<RT>(g.qr, pgd::BETWEEN_PRE, s);
+  pgk::batch_sweep_x<RT>(g.qx, g.shape.grid_x, s);
+  pgk::batch_sweep_y<RT>(g.qy, g.shape.grid_y, s);
+  pgk::batch_between<RT>(g.qr, pgd::BETWEEN_POST | pgd::BETWEEN_DIAG | (last ? 0 : pgd::BETWEEN_PRE), s);
+  *nk += first ? 4 : 3;
+}
+static void enqueue_group_step(pg_batch *b, int gi, bool first, bool last, int64_t *nk) {
+  if (gi == 1) enqueue_group_step<float>(b->g[1], first, last, b->stream, nk);
+  else enqueue_group_step<double>(b->g[0], first, last, b->stream, nk);
 }
 
 // one step of every member, on the batch stream
-static int enqueue_batch_step(pg_batch *b, int64_t *nk) {
+static int enqueue_batch_step(pg_batch *b, bool first, bool last, int64_t *nk) {
   cudaStream_t s = b->stream;
-  for (int gi = 0; gi < 2; gi++) enqueue_group_step(b, gi, nk);
+  for (int gi = 0; gi < 2; gi++) enqueue_group_step(b, gi, first, last, nk);
   for (pg_run *r : b->solo)
-    if (int e = pgi::run_enqueue_on(r, s, nk)) return bfail(b, e, pg_last_error(r));
+    if (int e = pgi::run_enqueue_on(r, s, first, last, nk)) return bfail(b, e, pg_last_error(r));
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return bfail(b, PG_ERR_CUDA, cudaGetErrorString(e));
   return PG_OK;
@@ -300,7 +292,7 @@ int pg_batch_advance(pg_batch *b, int nsteps, int chunk) {
   }
   if (p0_solo) {
     int64_t nk = 0;
-    if (int e = enqueue_batch_step(b, &nk)) return e;
+    if (int e = enqueue_batch_step(b, true, true, &nk)) return e;
     b->launches += nk;
     done = 1;
   }
@@ -318,7 +310,7 @@ int pg_batch_advance(pg_batch *b, int nsteps, int chunk) {
     // an even chunk leaves the 3D members' plane copies where they started
     BK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     for (int i = 0; i < chunk; i++) {
-      if (int e = enqueue_batch_step(b, &nk)) {
+      if (int e = enqueue_batch_step(b, i == 0, i == chunk - 1, &nk)) {
         cudaStreamEndCapture(b->stream, &gr);
         return e;
       }
@@ -345,8 +337,8 @@ int pg_batch_advance(pg_batch *b, int nsteps, int chunk) {
   }
   if (done < nsteps && done + chunk > nsteps) {
     int64_t nk = 0;
-    for (; done < nsteps; done++)
-      if (int e = enqueue_batch_step(b, &nk)) return e;
+    for (bool first = true; done < nsteps; done++, first = false)
+      if (int e = enqueue_batch_step(b, first, done == nsteps - 1, &nk)) return e;
     b->launches += nk;
   }
   for (auto &g : b->g)
@@ -408,9 +400,9 @@ int pg_batch_tune(pg_batch *b, int trial_steps) {
     for (const pg_batch_shape &c : cand) {
       g.shape = c;
       int64_t nk = 0;
-      enqueue_group_step(b, gi, &nk);   // warm-up step
+      enqueue_group_step(b, gi, true, true, &nk);   // warm-up step
       if (cudaEventRecord(e0, b->stream) != cudaSuccess) { rc = PG_ERR_CUDA; break; }
-      for (int i = 0; i < trial_steps; i++) enqueue_group_step(b, gi, &nk);
+      for (int i = 0; i < trial_steps; i++) enqueue_group_step(b, gi, i == 0, i == trial_steps - 1, &nk);
       if (cudaEventRecord(e1, b->stream) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess) {
         rc = PG_ERR_CUDA;
         break;

@@ -15,6 +15,7 @@ struct RunShape {
   int eos;                 // EOS 1: isentropic sweeps (own step sequence)
   int nr, nphi, nk;
   int tiles_x, tiles_y;    // CTAs of the radial and azimuthal sweeps
+  int ctas_b;              // CTAs between two steps
 };
 int run_shape(const pg_run *run, RunShape *out);
 
@@ -22,8 +23,9 @@ int run_shape(const pg_run *run, RunShape *out);
 int run_batch_desc(pg_run *run, pgd::BatchRun *d);
 // The batch enqueued steps of this run: the p0 plane is used up, count launches.
 void run_batched(pg_run *run, int64_t launches);
-// One step of the device-resident loop of this run, enqueued on stream s.
-int run_enqueue_on(pg_run *run, cudaStream_t s, int64_t *launches);
+// One step of the device-resident loop of this run, enqueued on stream s
+// (first, last: of the sequence being queued).
+int run_enqueue_on(pg_run *run, cudaStream_t s, bool first, bool last, int64_t *launches);
 // Device clock of the run.
 pgd::DevClock *run_clock(pg_run *run);
 // which of the two plane copies is current (3D steps flip it)

@@ -29,7 +29,7 @@ struct Tables {
   int nr, nphi, nk, nrg;
   Chunking cx, cy, cz;
   const double *rx, *rdx, *rxvol, *rxc;         // [nrg]
-  const double *irdx, *irxc;                    // [nrg]: 1/rdx, 1/rxc (k_tables)
+  const double *irdx, *irxc, *rpa;              // [nrg]: 1/rdx, 1/rxc, rxc^-p_alpha (k_tables)
   const double *radc, *cs2, *nu;                // [nk*nrg]
   const double *irc, *snd;                      // [nk*nrg]: 1/radc, sqrt(gam cs2) (k_tables)
   const double *y, *dy, *yvol, *yc;             // [nphi]
@@ -86,6 +86,10 @@ struct SweepCtl {
   int shift;          // store at (j + inc_j) mod jmax: the last sweep of a step
   int nocfl;          // with fuse: no CFL rate (a moving planet's FrRot is known only after the step)
 };
+
+// parts of what happens between two steps (pg_step.cu): the end of one with a
+// fixed planet, its diagnostics, the start of the next
+constexpr int BETWEEN_POST = 1, BETWEEN_DIAG = 2, BETWEEN_PRE = 4;
 
 // Planes a dump is unpacked into / packed from (pg_load_rings, pg_save_rings).
 struct DumpPlanes {
@@ -181,37 +185,40 @@ void axis_tables(const Tables &T, int ndim, cudaStream_t s);
 size_t axis_table_elems(const Chunking &ch);
 // CFL rate max of the planes (p0: the pressure of a freshly loaded dump, or
 // null) into *out; with clk, the device loop's: FrRot, target and halt flag
-// from the clock, the step's shift still pending when rot_pending
+// from the clock, the step's shift still pending when rot_pending; with hout,
+// *out goes to *hout (host memory) and is cleared (counter: 0 between launches)
 template <class RT>
 void cfl(const Tables &T, const RT *r, const RT *u, const RT *v, const RT *w, const double *p0, const Phys &ph,
-         double frrot, int ndim, unsigned long long *out, DevClock *clk, int rot_pending, cudaStream_t s);
-void index_shift(const Tables &T, double dt, double frrot, int fargo, const DevClock *clk, cudaStream_t s);
-void rotate(const Tables &T, const DevClock *clk, cudaStream_t s);
+         double frrot, int ndim, unsigned long long *out, DevClock *clk, int rot_pending, unsigned *counter,
+         unsigned long long *hout, cudaStream_t s);
 // damping by dt, or by the clock's step
 template <class RT>
 void damp(const Tables &T, RT *r, RT *u, RT *v, RT *w, double dt, const DevClock *clk, int ndim, cudaStream_t s);
-void reduce(const Tables &T, const double *r, const Body &pl, const DevClock *clk, double exclude,
-            int mode, int plnt, double p_alpha, int ndim, double *ring_part, unsigned int *counter,
-            double *out, double *hist_row, cudaStream_t s);
-void reduce32(const Tables &T, const float *r, const Body &pl, const DevClock *clk, double exclude, int mode,
-              int plnt, double p_alpha, int ndim, double *ring_part, unsigned int *counter, double *out,
-              cudaStream_t s);
-// batched 2D steps over many runs (one launch per phase for all runs)
-void batch_prestep(const BatchRun *runs, int nruns, cudaStream_t s);
-void batch_poststep(const BatchRun *runs, int nruns, cudaStream_t s);
-void batch_record(const BatchRun *runs, int nruns, cudaStream_t s);
-void batch_reduce(const BatchQueue &rings, int fp32, int mode, cudaStream_t s);
+// the step around the sweeps (pg_step.cu)
+void index_shift(const Tables &T, double dt, double frrot, int fargo, cudaStream_t s);
+void rotate(const Tables &T, cudaStream_t s);
+// disk mass (mode 0), radial force (8) or torque (9) on the planet into *out;
+// part: 2 nr nk doubles, counter: 0 between launches
+template <class RT>
+void reduce(const Tables &T, const RT *r, const Body &pl, double exclude, int mode, int plnt, double p_alpha, int ndim,
+            double *part, unsigned *counter, double *out, cudaStream_t s);
+// between two steps: any of the parts BETWEEN_*
+template <class RT>
+void between(const Tables &T, const RT *r, DevClock *clk, double *part, unsigned *counter, double p_alpha, int fargo,
+             int plnt, int ndim, int fl, cudaStream_t s);
+// moving planet (plnt_flag 2): a step's end up to the kick
+template <class RT>
+void moving(const Tables &T, const RT *r, DevClock *clk, double *part, unsigned *counter, double p_alpha, int ndim,
+            cudaStream_t s);
+// between() of every member of a batch; CTAs of a member
+template <class RT>
+void batch_between(const BatchQueue &q, int fl, cudaStream_t s);
+int between_ctas(int rings);
+// batched 2D sweeps over many runs
 template <class RT>
 void batch_sweep_x(const BatchQueue &q, int grid, cudaStream_t s);
 template <class RT>
 void batch_sweep_y(const BatchQueue &q, int grid, cudaStream_t s);
-void prestep(DevClock *clk, const Tables &T, int fargo, cudaStream_t s);
-// moving planet (plnt_flag 2): the step's end split around the disk-force reductions
-void poststep_drift(DevClock *clk, const Tables &T, cudaStream_t s);
-void poststep_kick(DevClock *clk, cudaStream_t s);
-void reduce_forces(const Tables &T, const void *r, int fp32, DevClock *clk, double p_alpha, int ndim,
-                   double *ring_part, unsigned int *counter, cudaStream_t s);
-void poststep(DevClock *clk, const Tables &T, cudaStream_t s);
 // dump <-> planes: stage holds the dump's field arrays ring by ring ([nr*nk][5][nphi]
 // for unpack, whole 72*nphi+96-byte ring records for pack); err bit 1: a density
 // that is not finite and positive, bit 2: nonzero w in a 2D dump
@@ -225,5 +232,4 @@ void pack_dump(const Tables &T, const DumpPlanes &D, const Phys &ph, int ndim, i
 // (ab[2i], ab[2i+1]), torque on a planet at r = 1 per ring (ring_out[k*nr+i])
 void post_harmonic(const Tables &T, const void *r, int fp32, double m, double *ab, cudaStream_t s);
 void post_torque(const Tables &T, const void *r, int fp32, double M_p, double *ring_out, cudaStream_t s);
-void record(DevClock *clk, cudaStream_t s);
 }  // namespace pgk

@@ -51,7 +51,6 @@ struct pg_run {
   // scratch + clock
   double *ring_part = nullptr;
   unsigned int *counter = nullptr;
-  double *dscal = nullptr;
   unsigned long long *cfl = nullptr;
   pgd::DevClock *clk = nullptr;
   double *hist = nullptr;
@@ -65,9 +64,17 @@ struct pg_run {
   int gsteps = 0;
   int gcur = 0;                    // plane copy current when gexec was captured
   int64_t graph_kernels = 0;       // kernels per replay of gexec
-  // early exit of pg_advance*: pinned copies of clk->halted, read a few
-  // launches behind the one being queued
-  int *h_halt = nullptr;
+  // pinned host memory of the run: copies of clk->halted, read a few launches
+  // behind the one being queued (early exit of pg_advance*), results that
+  // kernels write here themselves, and a copy of the clock
+  struct HostPage {
+    int halt[4];
+    double sum;
+    unsigned long long cfl;
+    pgd::DevClock clk;
+  };
+  HostPage *page = nullptr;
+  int64_t ncycle = -1;             // clk->ncycle as far as the host knows it (-1: it does not)
   cudaEvent_t halt_ev[4] = {};
   // event timing
   bool timing = false;
@@ -112,6 +119,23 @@ static int fail(pg_run *run, int code, const std::string &msg) {
   return code;
 }
 
+static int host_page(pg_run *run) {
+  if (run->page) return PG_OK;
+  if (cudaHostAlloc(&run->page, sizeof(pg_run::HostPage), cudaHostAllocDefault) != cudaSuccess) {
+    run->page = nullptr;
+    return fail(run, PG_ERR_NOMEM, "pinned host memory");
+  }
+  return PG_OK;
+}
+// the run's clock, copied to the page; waits for the stream
+static int read_clock(pg_run *run) {
+  if (int e = host_page(run)) return e;
+  CK(cudaMemcpyAsync(&run->page->clk, run->clk, sizeof(pgd::DevClock), cudaMemcpyDeviceToHost, run->stream));
+  CK(cudaStreamSynchronize(run->stream));
+  run->ncycle = run->page->clk.ncycle;
+  return PG_OK;
+}
+
 static int check_launch(pg_run *run, int n) {
   run->launches += n;
   cudaError_t e = cudaGetLastError();
@@ -125,7 +149,7 @@ static int check_launch(pg_run *run, int n) {
 // doubles of a run's table block (pg_create lays it out)
 static size_t table_elems(size_t nr, size_t nphi, size_t nk) {
   const size_t nrg = nr + 2 * NPAD, nring = nk * nrg, nz = nk + 2 * NPAD;
-  size_t n = 6 * nrg + 11 * nring + 7 * nphi + 6 * nz + 6 * (size_t)2 * NPAD * nr;
+  size_t n = 7 * nrg + 11 * nring + 7 * nphi + 6 * nz + 6 * (size_t)2 * NPAD * nr;
   for (size_t len : {nr, nphi, nk}) n += pgk::axis_table_elems(pgd::make_chunking((int)len));
   return n;
 }
@@ -146,7 +170,9 @@ static pgd::Planes planes_fwd(pg_run *run, int src, const double *p0) {
   return p;
 }
 
-// One step of main.cu:343-441 as device work on the run's stream.
+// One step of main.cu:343-441 as device work on the run's stream.  The step's
+// start (dt, Index_Shift, half kick) is queued with the end of the step before;
+// a sequence queues that of its first step itself and none after its last.
 template <class RT>
 static RT **planes_of(pg_run *run, int copy) {
   if constexpr (sizeof(RT) == 4) return run->p32[copy];
@@ -159,7 +185,7 @@ static pgd::PlanesT<RT> fwd(pg_run *run, int src, const double *p0) {
 }
 
 template <class RT>
-static int enqueue_step_t(pg_run *run, bool first_p0) {
+static int enqueue_step_t(pg_run *run, bool first_p0, bool first, bool last) {
   const pg_params &P = run->P;
   cudaStream_t s = run->stream;
   pgd::SweepCtl c{};
@@ -171,11 +197,16 @@ static int enqueue_step_t(pg_run *run, bool first_p0) {
   const bool tm = run->timing;
   size_t e_step = 0, e_k = 0;
   if (tm && ev_pair(run, 3, e_step)) return fail(run, PG_ERR_CUDA, "event record");
-  pgk::prestep(run->clk, run->T, P.FARGO_flag, s); n++;
+  const bool moving = P.plnt_flag == 2;
+  auto between = [&](int fl) {
+    pgk::between<RT>(run->T, planes_of<RT>(run, run->cur)[0], run->clk, run->ring_part, run->counter, P.p_alpha,
+                     P.FARGO_flag, P.plnt_flag > 0, P.ndim, fl, s);
+    n++;
+  };
+  if (first) between(pgd::BETWEEN_PRE);
   if (tm && ev_pair(run, 0, e_k)) return fail(run, PG_ERR_CUDA, "event record");
   pgk::sweep_x<RT>(run->T, fwd<RT>(run, a, first_p0 ? run->p0 : nullptr), run->ph, c, P.ndim, s); n++;
   if (tm && ev_close(run, e_k)) return fail(run, PG_ERR_CUDA, "event record");
-  const bool moving = P.plnt_flag == 2;
   if (P.ndim == 2) {
     c.fuse = 1;
     c.shift = 1;
@@ -198,35 +229,22 @@ static int enqueue_step_t(pg_run *run, bool first_p0) {
     if (!fuse_z) {
       pgk::damp<RT>(run->T, cp[0], cp[1], cp[2], cp[3], 0.0, run->clk, 3, s); n++;
       if (!moving) {
-        pgk::cfl<RT>(run->T, cp[0], cp[1], cp[2], cp[3], nullptr, run->ph, 0.0, 3, nullptr, run->clk, 1, s); n++;
+        pgk::cfl<RT>(run->T, cp[0], cp[1], cp[2], cp[3], nullptr, run->ph, 0.0, 3, nullptr, run->clk, 1,
+                     nullptr, nullptr, s); n++;
       }
     }
     run->cur = 1 - a;
   }
-  RT **cp = planes_of<RT>(run, run->cur);
   if (moving) {
     // moving planet (planet.cu:54-93): drift, the disk's forces on the
     // drifted planet (reductions 8 and 9), kick; FrRot is then known and the
     // next get_dt's CFL runs on the stored state
-    pgk::poststep_drift(run->clk, run->T, s); n++;
-    pgk::reduce_forces(run->T, cp[0], run->fp32, run->clk, P.p_alpha, P.ndim, run->ring_part, run->counter, s); n += 2;
-    pgk::poststep_kick(run->clk, s); n++;
-    pgk::cfl<RT>(run->T, cp[0], cp[1], cp[2], cp[3], nullptr, run->ph, 0.0, P.ndim, nullptr, run->clk, 0, s); n++;
-  } else {
-    pgk::poststep(run->clk, run->T, s); n++;
+    RT **cp = planes_of<RT>(run, run->cur);
+    pgk::moving<RT>(run->T, cp[0], run->clk, run->ring_part, run->counter, P.p_alpha, P.ndim, s); n++;
+    pgk::cfl<RT>(run->T, cp[0], cp[1], cp[2], cp[3], nullptr, run->ph, 0.0, P.ndim, nullptr, run->clk, 0, nullptr,
+                 nullptr, s); n++;
   }
-  auto sum = [&](int mode, int plnt, double *out) {
-    if constexpr (sizeof(RT) == 4)
-      pgk::reduce32(run->T, cp[0], pgd::Body{}, run->clk, 0.0, mode, plnt, P.p_alpha, P.ndim, run->ring_part,
-                    run->counter, out, s);
-    else
-      pgk::reduce(run->T, cp[0], pgd::Body{}, run->clk, 0.0, mode, plnt, P.p_alpha, P.ndim, run->ring_part,
-                  run->counter, out, nullptr, s);
-    n++;
-  };
-  sum(0, P.plnt_flag > 0, &run->clk->mass);
-  if (P.plnt_flag > 0 && P.ndim == 2) sum(9, 1, &run->clk->torque);
-  pgk::record(run->clk, s); n++;
+  between((moving ? 0 : pgd::BETWEEN_POST) | pgd::BETWEEN_DIAG | (last ? 0 : pgd::BETWEEN_PRE));
   if (tm && ev_close(run, e_step)) return fail(run, PG_ERR_CUDA, "event record");
   return check_launch(run, n);
 }
@@ -289,7 +307,7 @@ int pg_create(const pg_params *p, int device, pg_run **out) {
     t += pgk::axis_table_elems(a == 0 ? T.cx : a == 1 ? T.cy : T.cz);
   }
   T.rx = t; t += nrg; T.rdx = t; t += nrg; T.rxvol = t; t += nrg; T.rxc = t; t += nrg;
-  T.irdx = t; t += nrg; T.irxc = t; t += nrg;
+  T.irdx = t; t += nrg; T.irxc = t; t += nrg; T.rpa = t; t += nrg;
   T.radc = t; t += nring; T.cs2 = t; t += nring; T.nu = t; t += nring; T.irc = t; t += nring; T.snd = t; t += nring;
   T.val_r = t; t += nring; T.val_u = t; t += nring; T.val_v = t; t += nring;
   T.damp_g = t; t += nring; T.damp_pw = t; t += nring;
@@ -309,13 +327,13 @@ int pg_create(const pg_params *p, int device, pg_run **out) {
 
   T.inc_j = run->itab; T.rot_j = run->itab + nring;
   // scratch
-  if (cudaMalloc(&run->ring_part, (size_t)nr * nk * sizeof(double)) != cudaSuccess) return bail(PG_ERR_NOMEM);
+  if (cudaMalloc(&run->ring_part, 2 * (size_t)nr * nk * sizeof(double)) != cudaSuccess) return bail(PG_ERR_NOMEM);
   if (cudaMalloc(&run->counter, sizeof(unsigned int)) != cudaSuccess) return bail(PG_ERR_NOMEM);
-  if (cudaMalloc(&run->dscal, 4 * sizeof(double)) != cudaSuccess) return bail(PG_ERR_NOMEM);
   if (cudaMalloc(&run->cfl, sizeof(unsigned long long)) != cudaSuccess) return bail(PG_ERR_NOMEM);
   if (cudaMalloc(&run->clk, sizeof(pgd::DevClock)) != cudaSuccess) return bail(PG_ERR_NOMEM);
   if (cudaMalloc(&run->hist, (size_t)run->hist_cap * pgd::HIST_COLS * sizeof(double)) != cudaSuccess) return bail(PG_ERR_NOMEM);
   if (cudaMemsetAsync(run->counter, 0, sizeof(unsigned int), run->stream) != cudaSuccess) return bail(PG_ERR_CUDA);
+  if (cudaMemsetAsync(run->cfl, 0, sizeof(unsigned long long), run->stream) != cudaSuccess) return bail(PG_ERR_CUDA);
   // physics constants
   run->ph.gam = p->gam;
   run->ph.sc2 = p->sc_h * p->sc_h;
@@ -339,7 +357,7 @@ int pg_destroy(pg_run *run) {
   if (run->gexec) cudaGraphExecDestroy(run->gexec);
   for (auto e : run->ev_pool) cudaEventDestroy(e);
   for (auto e : run->halt_ev) if (e) cudaEventDestroy(e);
-  if (run->h_halt) cudaFreeHost(run->h_halt);
+  if (run->page) cudaFreeHost(run->page);
   for (auto &b : run->planes)
     for (auto &f : b) if (f) cudaFree(f);
   for (auto &b : run->p32)
@@ -352,7 +370,6 @@ int pg_destroy(pg_run *run) {
   cudaFree(run->T.rot_v);
   cudaFree(run->ring_part);
   cudaFree(run->counter);
-  cudaFree(run->dscal);
   cudaFree(run->cfl);
   cudaFree(run->clk);
   cudaFree(run->hist);
@@ -601,23 +618,24 @@ int pg_get_dt(pg_run *run, double dt_old, double frrot, double *dt_out) {
   if (!run->loaded) return fail(run, PG_ERR_STATE, "no state loaded");
   CK(cudaSetDevice(run->dev));
   cudaStream_t s = run->stream;
+  if (int e = host_page(run)) return e;
   double **cp = run->planes[run->cur];
   float **fp = run->p32[run->cur];
-  CK(cudaMemsetAsync(run->cfl, 0, sizeof(unsigned long long), s));
+  unsigned long long *h = &run->page->cfl;
   if (run->fp32)
-    pgk::cfl<float>(run->T, fp[0], fp[1], fp[2], fp[3], nullptr, run->ph, frrot, run->P.ndim, run->cfl, nullptr, 0, s);
+    pgk::cfl<float>(run->T, fp[0], fp[1], fp[2], fp[3], nullptr, run->ph, frrot, run->P.ndim, run->cfl, nullptr, 0,
+                    run->counter, h, s);
   else
     pgk::cfl<double>(run->T, cp[0], cp[1], cp[2], cp[3], run->p0_live ? run->p0 : nullptr, run->ph, frrot,
-                     run->P.ndim, run->cfl, nullptr, 0, s);
+                     run->P.ndim, run->cfl, nullptr, 0, run->counter, h, s);
   if (int e = check_launch(run, 1)) return e;
-  unsigned long long bits = 0;
-  CK(cudaMemcpyAsync(&bits, run->cfl, sizeof(bits), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
+  const unsigned long long bits = *h;
   double rate;
   std::memcpy(&rate, &bits, sizeof(rate));
-  double h = run->P.courant / rate;       // dt_lv3 timestep.cu:105
+  double hdt = run->P.courant / rate;     // dt_lv3 timestep.cu:105
   double dt = 1.1 * dt_old;               // timestep.cu:135-141
-  dt = (h < dt) ? h : dt;
+  dt = (hdt < dt) ? hdt : dt;
   *dt_out = dt;
   if (dt / run->P.endtime < 1.0e-12) return fail(run, PG_ERR_DT_COLLAPSE, "time step too small");
   return PG_OK;
@@ -627,7 +645,7 @@ int pg_index_shift(pg_run *run, double dt, double frrot) {
   if (!run) return PG_ERR_ARG;
   if (!run->loaded) return fail(run, PG_ERR_STATE, "no state loaded");
   CK(cudaSetDevice(run->dev));
-  pgk::index_shift(run->T, dt, frrot, run->P.FARGO_flag, nullptr, run->stream);
+  pgk::index_shift(run->T, dt, frrot, run->P.FARGO_flag, run->stream);
   return check_launch(run, 1);
 }
 
@@ -662,7 +680,7 @@ int pg_sweep2d(pg_run *run, double dt, const pg_body *planet, double frrot) {
     c.shift = 1;
     pgk::sweep_y<double>(run->T, planes_fwd(run, 1 - run->cur, nullptr), run->ph, c, nd, s);
   }
-  if (run->P.FARGO_flag > 0) pgk::rotate(run->T, nullptr, s);
+  if (run->P.FARGO_flag > 0) pgk::rotate(run->T, s);
   run->p0_live = false;
   return check_launch(run, 2 + (run->P.FARGO_flag > 0 ? 1 : 0));
 }
@@ -686,7 +704,7 @@ int pg_sweep3d(pg_run *run, double dt, const pg_body *planet, double frrot) {
     c.shift = 1;   // the polar sweep is the last one: it applies the FARGO shift
     pgk::sweep_z<double>(run->T, planes_fwd(run, a, nullptr), run->ph, c, run->P.ntop, s);
   }
-  if (run->P.FARGO_flag > 0) pgk::rotate(run->T, nullptr, s);
+  if (run->P.FARGO_flag > 0) pgk::rotate(run->T, s);
   run->cur = 1 - a;
   run->p0_live = false;
   return check_launch(run, 3 + (run->P.FARGO_flag > 0 ? 1 : 0));
@@ -727,7 +745,7 @@ int pg_rotate(pg_run *run) {
   if (!run) return PG_ERR_ARG;
   if (!run->loaded) return fail(run, PG_ERR_STATE, "no state loaded");
   CK(cudaSetDevice(run->dev));
-  pgk::rotate(run->T, nullptr, run->stream);
+  pgk::rotate(run->T, run->stream);
   return check_launch(run, 1);
 }
 
@@ -753,16 +771,18 @@ int pg_reduce(pg_run *run, const pg_body *planet, double exclude, int mode, doub
   CK(cudaSetDevice(run->dev));
   pgd::Body b{planet->m, planet->x, planet->y, planet->vx, planet->vy, planet->fx, planet->fy, planet->rs};
   exclude *= run->P.sc_h;                                 // device_func.cu:171
+  if (int e = host_page(run)) return e;
+  double *h = &run->page->sum;     // the kernel writes it
+  const int plnt = run->P.plnt_flag > 0;
   if (run->fp32)
-    pgk::reduce32(run->T, run->p32[run->cur][0], b, nullptr, exclude, mode, run->P.plnt_flag > 0,
-                  run->P.p_alpha, run->P.ndim, run->ring_part, run->counter, run->dscal, run->stream);
+    pgk::reduce<float>(run->T, run->p32[run->cur][0], b, exclude, mode, plnt, run->P.p_alpha, run->P.ndim,
+                       run->ring_part, run->counter, h, run->stream);
   else
-    pgk::reduce(run->T, run->planes[run->cur][0], b, nullptr, exclude, mode, run->P.plnt_flag > 0,
-                run->P.p_alpha, run->P.ndim, run->ring_part, run->counter, run->dscal, nullptr, run->stream);
+    pgk::reduce<double>(run->T, run->planes[run->cur][0], b, exclude, mode, plnt, run->P.p_alpha, run->P.ndim,
+                        run->ring_part, run->counter, h, run->stream);
   if (int e = check_launch(run, 1)) return e;
-  CK(cudaMemcpyAsync(out, run->dscal, sizeof(double), cudaMemcpyDeviceToHost, run->stream));
   CK(cudaStreamSynchronize(run->stream));
-  *out = 0.0 + *out;                                       // host sum device_func.cu:195
+  *out = 0.0 + *h;                                         // host sum device_func.cu:195
   return PG_OK;
 }
 
@@ -871,12 +891,13 @@ int pg_clock_reset(pg_run *run, int startat) {
   double **cp = run->planes[run->cur];
   float **fp = run->p32[run->cur];
   if (run->fp32)
-    pgk::cfl<float>(run->T, fp[0], fp[1], fp[2], fp[3], nullptr, run->ph, fr, P.ndim, &run->clk->cfl_bits, nullptr, 0, s);
+    pgk::cfl<float>(run->T, fp[0], fp[1], fp[2], fp[3], nullptr, run->ph, fr, P.ndim, &run->clk->cfl_bits, nullptr, 0, nullptr, nullptr, s);
   else
     pgk::cfl<double>(run->T, cp[0], cp[1], cp[2], cp[3], run->p0_live ? run->p0 : nullptr, run->ph, fr, P.ndim,
-                     &run->clk->cfl_bits, nullptr, 0, s);
+                     &run->clk->cfl_bits, nullptr, 0, nullptr, nullptr, s);
   if (int e = check_launch(run, 1)) return e;
   CK(cudaStreamSynchronize(s));
+  run->ncycle = 0;
   run->clock_ready = true;
   return PG_OK;
 }
@@ -885,9 +906,8 @@ int pg_clock_get(pg_run *run, pg_clock *out, pg_body *planet) {
   if (!run) return PG_ERR_ARG;
   if (!run->clock_ready) return fail(run, PG_ERR_STATE, "clock not reset");
   CK(cudaSetDevice(run->dev));
-  pgd::DevClock c;
-  CK(cudaMemcpyAsync(&c, run->clk, sizeof(c), cudaMemcpyDeviceToHost, run->stream));
-  CK(cudaStreamSynchronize(run->stream));
+  if (int e = read_clock(run)) return e;
+  const pgd::DevClock &c = run->page->clk;
   if (out) {
     out->simtime = c.simtime; out->timem = c.timem; out->dt = c.dt; out->dt_used = c.dt_step;
     out->frrot = c.frrot; out->ncycle = c.ncycle; out->make_pict = c.make_pict; out->done = c.done;
@@ -900,8 +920,8 @@ int pg_clock_get(pg_run *run, pg_clock *out, pg_body *planet) {
   return PG_OK;
 }
 
-static int enqueue_step(pg_run *run, bool first_p0) {
-  return run->fp32 ? enqueue_step_t<float>(run, false) : enqueue_step_t<double>(run, first_p0);
+static int enqueue_step(pg_run *run, bool first_p0, bool first, bool last) {
+  return run->fp32 ? enqueue_step_t<float>(run, false, first, last) : enqueue_step_t<double>(run, first_p0, first, last);
 }
 
 // The device clock halts the loop (end time, a tmovie dump, an error); the
@@ -914,8 +934,8 @@ struct HaltProbe {
   pg_run *run;
   int64_t unit = 0;
   int init() {
-    if (run->h_halt) return PG_OK;
-    if (cudaHostAlloc(&run->h_halt, kDepth * sizeof(int), cudaHostAllocDefault) != cudaSuccess) return PG_ERR_CUDA;
+    if (host_page(run)) return PG_ERR_CUDA;
+    if (run->halt_ev[0]) return PG_OK;
     for (auto &e : run->halt_ev)
       if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return PG_ERR_CUDA;
     return PG_OK;
@@ -925,11 +945,11 @@ struct HaltProbe {
     if (unit < kDepth) return false;
     int slot = (int)(unit % kDepth);
     if (cudaEventSynchronize(run->halt_ev[slot]) != cudaSuccess) return true;   // surfaces in finish_advance
-    return run->h_halt[slot] != 0;
+    return run->page->halt[slot] != 0;
   }
   int post() {
     int slot = (int)(unit % kDepth);
-    if (cudaMemcpyAsync(&run->h_halt[slot], &run->clk->halted, sizeof(int), cudaMemcpyDeviceToHost,
+    if (cudaMemcpyAsync(&run->page->halt[slot], &run->clk->halted, sizeof(int), cudaMemcpyDeviceToHost,
                         run->stream) != cudaSuccess) return PG_ERR_CUDA;
     if (cudaEventRecord(run->halt_ev[slot], run->stream) != cudaSuccess) return PG_ERR_CUDA;
     unit++;
@@ -938,9 +958,8 @@ struct HaltProbe {
 };
 
 static int finish_advance(pg_run *run, int64_t before, int *taken) {
-  pgd::DevClock c;
-  CK(cudaMemcpyAsync(&c, run->clk, sizeof(c), cudaMemcpyDeviceToHost, run->stream));
-  CK(cudaStreamSynchronize(run->stream));
+  if (int e = read_clock(run)) return e;
+  const pgd::DevClock &c = run->page->clk;
   if (taken) *taken = (int)(c.ncycle - before);
   if (c.status != 0) {
     return fail(run, c.status, c.status == PG_ERR_NONFINITE ? "non-finite or non-positive state"
@@ -959,16 +978,15 @@ int pg_advance(pg_run *run, int nsteps, int *taken) {
   if (!run) return PG_ERR_ARG;
   if (!run->clock_ready) return fail(run, PG_ERR_STATE, "call pg_clock_reset first");
   CK(cudaSetDevice(run->dev));
-  pgd::DevClock c;
-  CK(cudaMemcpy(&c, run->clk, sizeof(c), cudaMemcpyDeviceToHost));
-  int64_t before = c.ncycle;
+  if (run->ncycle < 0)
+    if (int e = read_clock(run)) return e;
+  const int64_t before = run->ncycle;
   HaltProbe hp{run};
   if (int e = hp.init()) return fail(run, e, "halt probe set-up");
   const int group = 16;
   for (int i = 0; i < nsteps; i++) {
     if (i % group == 0 && hp.halted_before_next()) break;
-    bool first = run->p0_live;
-    if (int e = enqueue_step(run, first)) return e;
+    if (int e = enqueue_step(run, run->p0_live, i == 0, i == nsteps - 1)) return e;
     run->p0_live = false;
     if ((i + 1) % group == 0 && hp.post()) return fail(run, PG_ERR_CUDA, "halt probe");
   }
@@ -981,12 +999,12 @@ int pg_advance_graph(pg_run *run, int nsteps, int chunk, int *taken) {
   if (chunk < 1) return fail(run, PG_ERR_ARG, "chunk must be >= 1");
   CK(cudaSetDevice(run->dev));
   if (run->P.ndim == 3 && (chunk & 1)) chunk += 1;   // 3D steps alternate the plane copies
-  pgd::DevClock c;
-  CK(cudaMemcpy(&c, run->clk, sizeof(c), cudaMemcpyDeviceToHost));
-  int64_t before = c.ncycle;
+  if (run->ncycle < 0)
+    if (int e = read_clock(run)) return e;
+  const int64_t before = run->ncycle;
   int done = 0;
   if (run->p0_live && nsteps > 0) {
-    if (int e = enqueue_step(run, true)) return e;
+    if (int e = enqueue_step(run, true, true, true)) return e;
     run->p0_live = false;
     done = 1;
   }
@@ -1000,7 +1018,7 @@ int pg_advance_graph(pg_run *run, int nsteps, int chunk, int *taken) {
     cudaGraph_t g;
     CK(cudaStreamBeginCapture(run->stream, cudaStreamCaptureModeThreadLocal));
     for (int i = 0; i < chunk; i++) {
-      int e = enqueue_step(run, false);
+      int e = enqueue_step(run, false, i == 0, i == chunk - 1);
       if (e) { cudaStreamEndCapture(run->stream, &g); run->timing = tm; return e; }
     }
     CK(cudaStreamEndCapture(run->stream, &g));
@@ -1025,8 +1043,8 @@ int pg_advance_graph(pg_run *run, int nsteps, int chunk, int *taken) {
     per++;
     if (hp.post()) return fail(run, PG_ERR_CUDA, "halt probe");
   }
-  for (; done < nsteps; done++) {
-    if (int e = enqueue_step(run, false)) return e;
+  for (bool first = true; done < nsteps; done++, first = false) {
+    if (int e = enqueue_step(run, false, first, done == nsteps - 1)) return e;
   }
   (void)per;
   return finish_advance(run, before, taken);
@@ -1059,9 +1077,8 @@ int pg_history(pg_run *run, double *rows, int max, int *rows_out) {
   if (!run || !rows_out) return PG_ERR_ARG;
   if (!run->clock_ready) return fail(run, PG_ERR_STATE, "clock not reset");
   CK(cudaSetDevice(run->dev));
-  pgd::DevClock c;
-  CK(cudaMemcpyAsync(&c, run->clk, sizeof(c), cudaMemcpyDeviceToHost, run->stream));
-  CK(cudaStreamSynchronize(run->stream));
+  if (int e = read_clock(run)) return e;
+  const pgd::DevClock &c = run->page->clk;
   int n = c.hist_count < max ? c.hist_count : max;
   if (n > 0 && rows)
     CK(cudaMemcpy(rows, run->hist, (size_t)n * pgd::HIST_COLS * sizeof(double), cudaMemcpyDeviceToHost));
@@ -1133,7 +1150,7 @@ extern "C" size_t pg_run_device_bytes(const pg_params *p) {
   if (p->precision != 1) b += up(pe * sizeof(double));                         // p0
   b += up(table_elems(nr, nphi, nk) * sizeof(double));
   b += up(2 * nring * sizeof(int)) + 3 * up(nring * sizeof(double));           // itab, rot_v, vbg, sbg
-  b += up(nr * nk * sizeof(double)) + up(4) + up(32) + up(8) + up(sizeof(pgd::DevClock));
+  b += up(2 * nr * nk * sizeof(double)) + up(4) + up(8) + up(sizeof(pgd::DevClock));
   b += up((size_t)4096 * pgd::HIST_COLS * sizeof(double));
   return b;
 }
@@ -1153,6 +1170,7 @@ int run_shape(const pg_run *run, RunShape *o) {
   o->nr = run->nr; o->nphi = run->nphi; o->nk = run->nk;
   o->tiles_x = pgk::tiles_x(run->T);
   o->tiles_y = pgk::tiles_y(run->T);
+  o->ctas_b = pgk::between_ctas(run->nr * run->nk);
   return PG_OK;
 }
 
@@ -1187,14 +1205,16 @@ int run_batch_desc(pg_run *run, pgd::BatchRun *d) {
 
 void run_batched(pg_run *run, int64_t launches) {
   run->p0_live = false;
+  run->ncycle = -1;
   run->launches += launches;
 }
 
-int run_enqueue_on(pg_run *run, cudaStream_t s, int64_t *launches) {
+int run_enqueue_on(pg_run *run, cudaStream_t s, bool first, bool last, int64_t *launches) {
   cudaStream_t own = run->stream;
   int64_t l0 = run->launches;
   run->stream = s;
-  int st = enqueue_step(run, run->p0_live);
+  int st = enqueue_step(run, run->p0_live, first, last);
+  run->ncycle = -1;
   run->stream = own;
   run->p0_live = false;
   if (launches) *launches += run->launches - l0;
