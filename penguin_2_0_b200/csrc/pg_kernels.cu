@@ -77,6 +77,7 @@ __global__ void k_tables(Tables T, Phys ph, int ndim, double kill_rin, double ki
   double *dg = const_cast<double *>(T.damp_g);
   double *dp = const_cast<double *>(T.damp_pw);
   radc[t] = rc;
+  set_shift(T, t, T.inc_j[t], T.rot_j[t]);
   cs2[t] = ph.sc2 * pow(rc, -ph.p_beta);          // get_cs2 disk_profile.cu:39-42
   const_cast<double *>(T.irc)[t] = 1.0 / rc;
   const_cast<double *>(T.snd)[t] = sqrt(ph.gam * cs2[t]);

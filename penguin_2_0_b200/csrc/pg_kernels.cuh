@@ -22,12 +22,32 @@ __host__ __device__ inline Chunking make_chunking(int n) {
   return c;
 }
 
+// How a sweep lays a chunk of lim cells on warps: G lanes per pencil, P
+// pencils per warp, cols pencils per CTA, step rows per pass of a CTA's loads
+// and stores, ng groups of cols pencils across the grid.  mG, mP, mC: 2^16 / d
+// rounded up, for quotients of small numbers (quot16); mng: 2^40 / ng.
+struct Tile {
+  int lim, G, P, cols, step, ng;
+  unsigned mG, mP, mC;
+  unsigned long long mng;
+};
+
+// The planet of a step as the sweeps' forces use it (forces.cu:23-182):
+// mass (3D with a planet: the reference's reduced mass), distance, 1/x^2,
+// x^2 + rs^2, the star's share of the mass, azimuth and its rate, cos and sin
+// of the azimuth
+struct PlanetC {
+  double m, x, ix2, b2, star, y, vy, cy, sy;
+};
+
 // Geometry and per-ring tables, all device pointers.  A "row" counts radial
 // rings including the 6 fixed ghost rings on each side (row = i + 6); a
 // "ring" index rk = k*nrg + row.
 struct Tables {
   int nr, nphi, nk, nrg;
   Chunking cx, cy, cz;
+  Tile tx[2], ty[2], tz[2];                     // per axis: full chunks, last chunk (pgk::tiles)
+  unsigned long long mnr;                       // 2^40 / nr rounded up
   const double *rx, *rdx, *rxvol, *rxc;         // [nrg]
   const double *irdx, *irxc, *rpa;              // [nrg]: 1/rdx, 1/rxc, rxc^-p_alpha (k_tables)
   const double *radc, *cs2, *nu;                // [nk*nrg]
@@ -46,6 +66,8 @@ struct Tables {
   const double *sbg;                            // [nk*nrg] FP32 runs: Sigma background (val.r / ghost r)
   double *res_v, *rot_v;                        // [nk*nrg]
   int *inc_j, *rot_j;                           // [nk*nrg]
+  int2 *shift;                                  // [nk*nrg]: inc_j and rot_j + inc_j modulo nphi
+  double2 *fin;                                 // [nk*nrg]: this step's damping factor and CFL frame offset (pg_step.cu)
 };
 
 // State planes a sweep reads and writes: FP64 Sigma, v_r, v_phi, v_theta, or
@@ -64,6 +86,7 @@ struct DevClock {
   double simtime, timem, dt, old_dt, dt_step, frrot, frrot_next;
   double endtime, tmovie, courant;
   Body planet;
+  PlanetC pc;                    // of planet, for the step's sweeps
   long long ncycle, ncycp, ncycend;
   int make_pict, prin, done, halted, status, pad;
   unsigned long long cfl_bits;   // max CFL rate as ordered bits (non-negative)
@@ -152,6 +175,17 @@ __device__ __forceinline__ double cfl_rate(double cs, double u, double irdx, dou
   if (!THREED) return fmax(t0, t1);
   return max3(t0, t1, __dmul_rn(__dadd_rn(fabs(w), cs), iwz));
 }
+// a / d for small a (a d < 2^16) from m = 2^16 / d rounded up
+__device__ __forceinline__ int quot16(int a, unsigned m) { return (int)((unsigned)a * m >> 16); }
+// a / d (a d < 2^40) from m = 2^40 / d rounded up
+__device__ __forceinline__ int quot40(int a, int d, unsigned long long m) {
+  const int q = (int)((unsigned long long)(unsigned)a * m >> 40);
+  return q * d > a ? q - 1 : q;
+}
+// the sweeps' copy of a ring's shift
+__device__ __forceinline__ void set_shift(const Tables &T, int rk, int inc, int rot) {
+  T.shift[rk] = make_int2(wrapm(inc, T.nphi), wrapm(rot + inc, T.nphi));
+}
 // the run of tile t of a batch queue, by bisection in its prefix sums
 __device__ __forceinline__ int batch_find(const BatchQueue &q, int t) {
   int lo = 0, hi = q.nruns;   // q.start[lo] <= t < q.start[hi]
@@ -177,6 +211,8 @@ template <class RT>
 void sweep_z(const Tables &T, const PlanesT<RT> &P, const Phys &ph, const SweepCtl &c, int ntop, cudaStream_t s);
 // per-device kernel attributes (dynamic shared memory limits); 0 on success
 int setup_device();
+// the grid's tiles (Tables::tx, ty, tz, mnr)
+void make_tiles(Tables &T);
 // CTAs of a run's radial and azimuthal sweep (batch queues)
 int tiles_x(const Tables &T);
 int tiles_y(const Tables &T);

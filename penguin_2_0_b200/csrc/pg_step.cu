@@ -50,6 +50,14 @@ __device__ __forceinline__ void index_shift_ring(const Tables &T, int t, double 
   T.inc_j[rk] = jp >= 0.0 ? (int)(jp + 0.5) : (int)(jp - 0.5);
   T.res_v[rk] = floor(jp + 0.5) * widthy;
   T.rot_v[rk] = rot_v;
+  set_shift(T, rk, T.inc_j[rk], T.rot_j[rk]);
+}
+// what the device loop's last sweep needs of a ring: this step's damping
+// factor and the frame offset of the next get_dt's azimuthal rate
+__device__ __forceinline__ void finish_ring(const Tables &T, int t, double dt, double frrot_next) {
+  const int rk = t / T.nr * T.nrg + t % T.nr + NPAD;
+  const double g = T.damp_g[rk];
+  T.fin[rk] = make_double2(g > 0.0 ? g * (dt * T.damp_pw[rk]) : 0.0, fma(frrot_next, T.radc[rk], T.rot_v[rk]));
 }
 // rotate_rings ppm.cu:309-322
 __device__ __forceinline__ int rotated(const Tables &T, int rk) { return wrap1(T.rot_j[rk] + T.inc_j[rk], T.nphi); }
@@ -62,7 +70,9 @@ __global__ void k_rotate(Tables T) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T.nr * T.nk) return;
   const int rk = t / T.nr * T.nrg + t % T.nr + NPAD;
-  T.rot_j[rk] = rotated(T, rk);
+  const int rot = rotated(T, rk);
+  T.rot_j[rk] = rot;
+  set_shift(T, rk, T.inc_j[rk], rot);
 }
 
 // ---------------------------------------------------------------------------
@@ -326,6 +336,7 @@ __device__ __forceinline__ bool step_pre(DevClock &c, double &frrot) {
   }
   c.frrot_next = fr;
   c.cfl_bits = 0ull;
+  c.pc = planet_consts(c.planet, c.ndim == 3, c.plnt_flag > 0);
   return true;
 }
 
@@ -399,14 +410,20 @@ __device__ __forceinline__ void between_body(StepShm &S, const Tables &T, const 
         part[rt] = m;
         part[rings + rt] = t;
         T.rot_j[rk] = rot;
-        if (S.run) index_shift_ring(T, rt, S.c.dt_step, S.frrot_pre, fargo);
+        if (S.run) {
+          index_shift_ring(T, rt, S.c.dt_step, S.frrot_pre, fargo);
+          finish_ring(T, rt, S.c.dt_step, S.c.frrot_next);
+        }
       }
     }
   } else {
     for (int rt = b * ST + tid; rt < rings; rt += nb * ST) {
       const int rk = rt / T.nr * T.nrg + rt % T.nr + NPAD;
       if (post) T.rot_j[rk] = rotated(T, rk);
-      if (S.run) index_shift_ring(T, rt, S.c.dt_step, S.frrot_pre, fargo);
+      if (S.run) {
+        index_shift_ring(T, rt, S.c.dt_step, S.frrot_pre, fargo);
+        finish_ring(T, rt, S.c.dt_step, S.c.frrot_next);
+      }
     }
   }
   if (nb > 1 && !last_cta(counter, nb)) return;

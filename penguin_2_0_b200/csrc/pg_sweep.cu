@@ -65,22 +65,18 @@ __device__ __forceinline__ bool load_step(const SweepCtl &c, StepIn &s) {
   return true;
 }
 
-// The planet's constants and the cosine and sine of its azimuth, formed by
-// one thread while the others load.
-struct PlanetShm { PlanetC p; double cy, sy; };
+// The planet's constants into shared memory: from the clock, or (calls with a
+// planet of their own) formed by one thread while the others load.
 template <bool THREED>
-__device__ __forceinline__ void planet_shm(PlanetShm &S, const StepIn &st, const Phys &ph) {
-  if (threadIdx.x == NT - 32) {
-    S.p = planet_consts<THREED>(st.pl, ph);
-    sincos(st.pl.y, &S.sy, &S.cy);
+__device__ __forceinline__ void planet_shm(PlanetC &S, const SweepCtl &ctl, const StepIn &st, const Phys &ph) {
+  constexpr int N = sizeof(PlanetC) / sizeof(double);
+  const int t = (int)threadIdx.x - (NT - 32);
+  if (ctl.clk) {
+    if (t >= 0 && t < N) reinterpret_cast<double *>(&S)[t] = reinterpret_cast<const double *>(&ctl.clk->pc)[t];
+  } else if (t == 0) {
+    S = planet_consts(st.pl, THREED, ph.plnt);
   }
 }
-
-// lanes per pencil and pencils per warp of a chunk of lim cells
-struct LaneMap {
-  int G, P;
-  __device__ __forceinline__ LaneMap(int lim, int C) : G((lim + C - 1) / C), P(32 / ((lim + C - 1) / C)) {}
-};
 
 // ---------------------------------------------------------------------------
 // axis tables (pg_warp.cuh AxisEntry): chunk l of an axis holds A_COUNT
@@ -159,12 +155,12 @@ __global__ void k_axis_table(Tables T, int axis, int C, double *out) {
 struct __align__(16) TileShm {
   double ws[NW][WS];
   double row[R_COUNT][ARR];
-  PlanetShm pl;
+  PlanetC pl;
 };
 // Place of cell n of column cl of a tile in a slot of its warp's workspace
 struct ColMap {
   int w, l0;                             // the column's warp and first lane
-  __device__ __forceinline__ ColMap(const LaneMap &M, int cl) : w(cl / M.P), l0((cl - cl / M.P * M.P) * M.G) {}
+  __device__ __forceinline__ ColMap(const Tile &M, int cl) : w(quot16(cl, M.mP)), l0((cl - w * M.P) * M.G) {}
   template <int C>
   __device__ __forceinline__ int at(int n) const {
     const int g = n / C, c = n - g * C;
@@ -174,21 +170,23 @@ struct ColMap {
 // Threads of a tile's loads and stores: thread t keeps column t % cols and
 // takes rows t / cols, t / cols + step, ...; threads past the last whole row idle.
 struct TileWalk {
-  int cl, n, step;
-  __device__ __forceinline__ TileWalk(int cols, int tid) : cl(tid % cols), n(tid / cols), step(NT / cols) {
-    if (n >= step) n = 1 << 20;
+  int cl, n;
+  __device__ __forceinline__ TileWalk(const Tile &M, int tid) {
+    n = quot16(tid, M.mC);
+    cl = tid - n * M.cols;
+    if (n >= M.step) n = 1 << 20;
   }
 };
 
 // The lane's place in a chunk of lim cells.  Lanes past the warp's last pencil
 // compute on a uniform state of their own, out of every range.
 template <int C, bool HAS_P = true>
-__device__ __forceinline__ int place_lane(Lane<C> &L, const LaneMap &M, int lim, const double *tab, const double *row,
+__device__ __forceinline__ int place_lane(Lane<C> &L, const Tile &M, int pw, const double *tab, const double *row,
                                           double *ws, int lane) {
-  const int pw = min(lane / M.G, M.P - 1), g = min(lane - pw * M.G, M.G - 1);
+  const int g = min(lane - pw * M.G, M.G - 1);
   const bool idle = lane >= M.P * M.G;
   L.n0 = idle ? 1 << 20 : C * g;
-  L.lim = lim;
+  L.lim = M.lim;
   L.tab = tab + (C == 4 ? 2 * g : g);
   L.row = row + (C == 4 ? 2 * g : g);
   L.half = C == 4 ? 2 * M.G : M.G;
@@ -212,29 +210,21 @@ __device__ __forceinline__ int place_lane(Lane<C> &L, const LaneMap &M, int lim,
 // radial sweep: tile t of the run
 template <class RT, bool THREED, int EOS>
 __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const PlanesT<RT> &P, const Phys &ph,
-                                             const StepIn &st, int t) {
+                                             const SweepCtl &ctl, const StepIn &st, int t) {
   constexpr int C = 4;
   const int nphi = T.nphi, nrg = T.nrg, full = T.cx.loop - 1, tid = threadIdx.x;
-  int l, k, j0;
-  const int nfull = full * ((nphi + NW - 1) / NW) * T.nk;
-  if (t < nfull) {
-    const int ng = (nphi + NW - 1) / NW;
-    j0 = (t % ng) * NW;
-    l = (t / ng) % full;
-    k = t / (ng * full);
-  } else {
-    const int w = NW * LaneMap(T.cx.stuck ? ARR : T.cx.lim_last, C).P, ng = (nphi + w - 1) / w;
-    t -= nfull;
-    j0 = (t % ng) * w;
-    l = full;
-    k = t / ng;
-  }
-  const bool last = l == full;
+  const int nfull = full * T.tx[0].ng * T.nk;
+  const bool last = t >= nfull;
+  const Tile &M = T.tx[last];
+  if (last) t -= nfull;
+  int q = quot40(t, M.ng, M.mng);
+  const int j0 = (t - q * M.ng) * M.cols;
+  const int k = last ? q : q / full, l = last ? full : q - k * full;
   if (last && T.cx.stuck) {
     // ppm.cu:48 gives this chunk lim = 12: its rings keep their values
 #pragma unroll 1
-    for (int q = tid; q < REAL * NW; q += NT) {
-      const int i = REAL * l + q / NW, j = j0 + q % NW;
+    for (int e = tid; e < REAL * NW; e += NT) {
+      const int i = REAL * l + e / NW, j = j0 + e % NW;
       if (i >= T.nr || j >= nphi) continue;
       const size_t o = ((size_t)k * nrg + i + NPAD) * nphi + j;
       P.ro[o] = P.r[o]; P.uo[o] = P.u[o]; P.vo[o] = P.v[o];
@@ -242,10 +232,8 @@ __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const 
     }
     return;
   }
-  const int lim = last ? T.cx.lim_last : ARR, row0 = REAL * l;
-  const LaneMap M(lim, C);
-  const int cols = NW * M.P, rows = C * M.G;
-  const TileWalk W(cols, tid);
+  const int lim = M.lim, row0 = REAL * l, rows = C * M.G;
+  const TileWalk W(M, tid);
   const ColMap cm(M, W.cl);
   double *const cw = S.ws[cm.w];
   // every load of the tile in flight before the first is used
@@ -253,7 +241,7 @@ __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const 
   double rc[4], cs2[4], p0[4], bs[4], bv[4];
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    const int n = W.n + i * W.step;
+    const int n = W.n + i * M.step;
     if (n >= rows) break;
     const int rk = k * nrg + min(row0 + n, nrg - 1);
     const size_t o = (size_t)rk * nphi + min(j0 + W.cl, nphi - 1);
@@ -282,10 +270,10 @@ __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const 
     S.row[R_RC][q] = r;
     S.row[R_IRC][q] = irc;
   }
-  planet_shm<THREED>(S.pl, st, ph);
+  planet_shm<THREED>(S.pl, ctl, st, ph);
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    const int n = W.n + i * W.step;
+    const int n = W.n + i * M.step;
     if (n >= rows) break;
     const int s = cm.at<C>(n);
     const double r = load_r(a[i][0], bs[i]);
@@ -297,19 +285,19 @@ __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const 
   }
   __syncthreads();
   {
-    const int lane = tid & 31, wid = tid >> 5;
-    const PlanetC pl = S.pl.p;
+    const int lane = tid & 31, wid = tid >> 5, pw = min(quot16(lane, M.mG), M.P - 1);
+    const PlanetC pl = S.pl;
     Lane<C> L;
-    place_lane<C>(L, M, lim, T.ax[0] + (size_t)l * A_COUNT * ARR, S.row[0], S.ws[wid], lane);
+    place_lane<C>(L, M, pw, T.ax[0] + (size_t)l * A_COUNT * ARR, S.row[0], S.ws[wid], lane);
     L.dt = st.dt;
     {
       // cos and sin of the column's azimuth less the planet's
-      const int j = min(j0 + wid * M.P + min(lane / M.G, M.P - 1), nphi - 1);
+      const int j = min(j0 + wid * M.P + pw, nphi - 1);
       const double cy = T.cyc[j], sy = T.syc[j];
       L.sp = THREED ? T.szc[k + NPAD] : 1.0;
       L.isp2 = THREED ? 1.0 / (L.sp * L.sp) : 1.0;
-      L.c0 = fma(cy, S.pl.cy, sy * S.pl.sy) * L.sp;
-      L.s0 = fma(sy, S.pl.cy, -(cy * S.pl.sy)) * L.sp;
+      L.c0 = fma(cy, pl.cy, sy * pl.sy) * L.sp;
+      L.s0 = fma(sy, pl.cy, -(cy * pl.sy)) * L.sp;
     }
     if (THREED) {
       double x[C], w[C];
@@ -383,7 +371,7 @@ __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const 
   __syncthreads();
   if (j0 + W.cl < nphi) {
 #pragma unroll 2
-    for (int n = W.n + NPAD; n < lim - NPAD; n += W.step) {
+    for (int n = W.n + NPAD; n < lim - NPAD; n += M.step) {
       const int rk = k * nrg + row0 + n;
       const size_t o = (size_t)rk * nphi + j0 + W.cl;
       const double bs = sizeof(RT) == 4 ? T.sbg[rk] : 0.0, bv = sizeof(RT) == 4 ? T.vbg[rk] : 0.0;
@@ -401,7 +389,7 @@ __global__ void __launch_bounds__(NT, MINB) k_sweep_x(Tables T, PlanesT<RT> P, P
   extern __shared__ __align__(16) unsigned char shm[];
   StepIn st;
   if (!load_step(ctl, st)) return;
-  sweep_x_tile<RT, THREED, EOS>(*reinterpret_cast<TileShm *>(shm), T, P, ph, st, blockIdx.x);
+  sweep_x_tile<RT, THREED, EOS>(*reinterpret_cast<TileShm *>(shm), T, P, ph, ctl, st, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -414,23 +402,23 @@ struct Finish {
   double cs, irdx, off, irc, iwz;        // sound speed (EOS 0), 1/dr, frame offset, 1/r_cyl, 1/(r dtheta)
   double bs, bv, cs2;
   int rot;                               // rot_j after the step's shift
-  __device__ __forceinline__ void ring(const Tables &T, const SweepCtl &ctl, const StepIn &st, int rk, int row, int kz, int inc) {
+  __device__ __forceinline__ void ring(const Tables &T, const SweepCtl &ctl, int rk, int row, int kz, int rot_new) {
     bs = sizeof(RT) == 4 ? T.sbg[rk] : 0.0;
     bv = sizeof(RT) == 4 ? T.vbg[rk] : 0.0;
     f = 0.0;
     if (!ctl.fuse) return;
-    const double g = T.damp_g[rk];
-    if (g > 0.0) {
-      f = g * (st.dt * T.damp_pw[rk]);
+    const double2 t = T.fin[rk];
+    f = t.x;
+    off = t.y;
+    if (f > 0.0) {
       tr = T.val_r[rk]; tu = T.val_u[rk]; tv = T.val_v[rk];
     }
     cs2 = T.cs2[rk];
     cs = T.snd[rk];
     irdx = T.irdx[row];
     irc = T.irc[rk];
-    off = fma(st.frrot_next, T.radc[rk], T.rot_v[rk]);
     iwz = kz >= 0 ? T.idz[kz] * T.irxc[row] : 0.0;
-    rot = wrapm(T.rot_j[rk] + inc, T.nphi);
+    rot = rot_new;
   }
   // stores the cell at offset o (azimuth column jo) and returns its CFL rate
   template <bool THREED, int EOS>
@@ -482,32 +470,38 @@ __device__ __forceinline__ void report(const SweepCtl &ctl, double rate, bool ba
 template <int EOS>
 struct __align__(16) YShm {
   double ws[NW][EOS ? WS : WS_ISO_Y];
-  PlanetShm pl;
+  PlanetC pl;
 };
 template <class RT, bool THREED, int EOS>
-__device__ __forceinline__ void sweep_y_task(double *ws, const PlanetShm &SP, const Tables &T, const PlanesT<RT> &P,
+__device__ __forceinline__ void sweep_y_task(double *ws, const PlanetC &SP, const Tables &T, const PlanesT<RT> &P,
                                              const Phys &ph, const SweepCtl &ctl, const StepIn &st, int t) {
   constexpr int C = 4;
   const int nphi = T.nphi, nrg = T.nrg, full = T.cy.loop - 1, rings = T.nr * T.nk, lane = threadIdx.x & 31;
-  int l = full, ring, lim = T.cy.lim_last;
-  // the tasks of full chunks fill whole CTAs, so that a CTA's warps take the
-  // chain's barriers together; tasks past the last ring compute and store nothing
-  const int nfull = (rings + NW - 1) / NW * NW;
-  if (t < full * nfull) {
-    // rings of one chunk side by side: the warps of an SM share its tables
-    l = t / nfull;
-    ring = t % nfull;
-    lim = ARR;
-  } else if (T.cy.stuck) {
-    ring = t - full * nfull;
+  // rings of one chunk side by side: the warps of an SM share its tables.  The
+  // tasks of full chunks fill whole CTAs, so that a CTA's warps take the
+  // barrier together; tasks past the last ring compute and store nothing.
+  const int nfull = full * T.ty[0].ng * NW;
+  const bool last = t >= nfull;
+  const Tile &M = T.ty[last];
+  int l = full, ring;
+  if (!last) {
+    const int cta = t / NW;
+    l = quot40(cta, M.ng, M.mng);
+    ring = t - l * M.ng * NW;
+  } else {
+    ring = (t - nfull) * M.P;
+  }
+  const int lim = M.lim;
+  if (last && T.cy.stuck) {
     if (ring >= rings) return;
     // ppm.cu:196 gives this chunk lim = 12: its cells keep their values and
     // only move with the ring's rotation
     const int k = ring / T.nr, row = ring % T.nr + NPAD, rk = k * nrg + row;
     const size_t base = (size_t)rk * nphi;
-    const int inc = ctl.shift ? wrapm(T.inc_j[rk], nphi) : 0;
+    const int2 sh = T.shift[rk];
+    const int inc = ctl.shift ? sh.x : 0;
     Finish<RT> F;
-    F.ring(T, ctl, st, rk, row, THREED ? k + NPAD : -1, ctl.shift ? T.inc_j[rk] : 0);
+    F.ring(T, ctl, rk, row, THREED ? k + NPAD : -1, sh.y);
     double rate = 0.0;
     bool bad = false;
 #pragma unroll 1
@@ -521,14 +515,12 @@ __device__ __forceinline__ void sweep_y_task(double *ws, const PlanetShm &SP, co
     }
     if (ctl.fuse) report(ctl, rate, bad);
     return;
-  } else {
-    ring = (t - full * nfull) * LaneMap(lim, C).P;
   }
-  const LaneMap M(lim, C);
   {
-    const int q = min(ring + min(lane / M.G, M.P - 1), rings - 1), k = q / T.nr, row = q % T.nr + NPAD, rk = k * nrg + row;
+    const int pw = min(quot16(lane, M.mG), M.P - 1);
+    const int q = min(ring + pw, rings - 1), k = quot40(q, T.nr, T.mnr), row = q - k * T.nr + NPAD, rk = k * nrg + row;
     Lane<C> L;
-    const int n0 = place_lane<C, (EOS != 0)>(L, M, lim, T.ax[1] + (size_t)l * A_COUNT * ARR, ws, ws, lane);
+    const int n0 = place_lane<C, (EOS != 0)>(L, M, pw, T.ax[1] + (size_t)l * A_COUNT * ARR, ws, ws, lane);
     // all loads in flight before the first is used; the four cells of a lane
     // share their sectors in L1
     const size_t base = (size_t)rk * nphi;
@@ -552,12 +544,12 @@ __device__ __forceinline__ void sweep_y_task(double *ws, const PlanetShm &SP, co
     const double snd = T.snd[rk], rs = T.rxc[row];
     // the planet's constants, formed meanwhile by the CTA's last warp
     __syncthreads();
-    const PlanetC pl = SP.p;
+    const PlanetC pl = SP;
     {
       L.bq = fma(rs, rs, pl.b2);         // the planet's distance sees the spherical radius in 3D
       const double a = 0.5 * st.dt * (L.vr - pl.vy);
       double s, c;
-      L.ca = SP.cy; L.sa = -SP.sy;
+      L.ca = pl.cy; L.sa = -pl.sy;
       sincos_near(a, s, c);
       L.cb = fma(L.ca, c, -(L.sa * s)); L.sb = fma(L.sa, c, L.ca * s);
       L.cc = fma(L.cb, c, -(L.sb * s)); L.sc = fma(L.sb, c, L.cb * s);
@@ -624,12 +616,13 @@ __device__ __forceinline__ void sweep_y_task(double *ws, const PlanetShm &SP, co
   const int len = lim - 2 * NPAD;
 #pragma unroll 1
   for (int b = 0; b < M.P && ring + b < rings; b++) {
-    const int q = ring + b, k = q / T.nr, row = q % T.nr + NPAD, rk = k * nrg + row;
+    const int q = ring + b, k = quot40(q, T.nr, T.mnr), row = q - k * T.nr + NPAD, rk = k * nrg + row;
     const size_t base = (size_t)rk * nphi;
-    const int inc = ctl.shift ? T.inc_j[rk] : 0, im = wrapm(inc, nphi);
+    const int2 sh = T.shift[rk];
+    const int im = ctl.shift ? sh.x : 0;
     const ColMap cm(M, b);
     Finish<RT> F;
-    F.ring(T, ctl, st, rk, row, THREED ? k + NPAD : -1, inc);
+    F.ring(T, ctl, rk, row, THREED ? k + NPAD : -1, sh.y);
 #pragma unroll 1
     for (int m = lane; m < len; m += 32) {
       const int s = cm.at<C>(m + NPAD);
@@ -649,7 +642,7 @@ __global__ void __launch_bounds__(NT, MINB) k_sweep_y(Tables T, PlanesT<RT> P, P
   YShm<EOS> &S = *reinterpret_cast<YShm<EOS> *>(shm);
   StepIn st;
   if (!load_step(ctl, st)) return;
-  planet_shm<THREED>(S.pl, st, ph);
+  planet_shm<THREED>(S.pl, ctl, st, ph);
   const int wid = threadIdx.x >> 5;
   sweep_y_task<RT, THREED, EOS>(S.ws[wid], S.pl, T, P, ph, ctl, st, blockIdx.x * NW + wid);
 }
@@ -668,40 +661,29 @@ template <class RT, int EOS, int C>
 __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const PlanesT<RT> &P, const Phys &ph,
                                              const SweepCtl &ctl, const StepIn &st, int ntop, int t) {
   const int nphi = T.nphi, nrg = T.nrg, nk = T.nk, full = T.cz.loop - 1, tid = threadIdx.x;
-  int l, i, j0;
-  const int nfull = full * ((nphi + NW - 1) / NW) * T.nr;
-  if (t < nfull) {
-    const int ng = (nphi + NW - 1) / NW;
-    j0 = (t % ng) * NW;
-    i = (t / ng) % T.nr;
-    l = t / (ng * T.nr);
-  } else {
-    const int w = NW * LaneMap(T.cz.stuck ? ARR : T.cz.lim_last, C).P, ng = (nphi + w - 1) / w;
-    t -= nfull;
-    j0 = (t % ng) * w;
-    i = t / ng;
-    l = full;
-  }
-  const int row = i + NPAD;
-  const bool last = l == full;
+  const int nfull = full * T.tz[0].ng * T.nr;
+  const bool last = t >= nfull;
+  const Tile &M = T.tz[last];
+  if (last) t -= nfull;
+  int q = quot40(t, M.ng, M.mng);
+  const int j0 = (t - q * M.ng) * M.cols;
+  const int l = last ? full : q / T.nr, i = last ? q : q - l * T.nr, row = i + NPAD;
   if (last && T.cz.stuck) {
 #pragma unroll 1
-    for (int q = tid; q < REAL * NW; q += NT) {
-      const int k = REAL * l + q / NW, j = j0 + q % NW;
+    for (int e = tid; e < REAL * NW; e += NT) {
+      const int k = REAL * l + e / NW, j = j0 + e % NW;
       if (k >= nk || j >= nphi) continue;
       const int rk = k * nrg + row;
-      int jo = j + (ctl.shift ? wrapm(T.inc_j[rk], nphi) : 0);
+      int jo = j + (ctl.shift ? T.shift[rk].x : 0);
       if (jo >= nphi) jo -= nphi;
       const size_t s = (size_t)rk * nphi + j, o = (size_t)rk * nphi + jo;
       P.ro[o] = P.r[s]; P.uo[o] = P.u[s]; P.vo[o] = P.v[s]; P.wo[o] = P.w[s];
     }
     return;
   }
-  const int lim = last ? T.cz.lim_last : ARR, k0 = REAL * l - NPAD;
-  const LaneMap M(lim, C);
-  const int cols = NW * M.P, rows = C * M.G;
+  const int lim = M.lim, k0 = REAL * l - NPAD, rows = C * M.G;
   const double rad = T.rxc[row];
-  const TileWalk W(cols, tid);
+  const TileWalk W(M, tid);
   const ColMap cm(M, W.cl);
   double *const cw = S.ws[cm.w];
   // every load of the tile in flight before the first is used; a ghost layer
@@ -711,7 +693,7 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
   double rc[4], cs2[4], bs[4], bv[4];
 #pragma unroll
   for (int i4 = 0; i4 < 4; i4++) {
-    const int n = W.n + i4 * W.step;
+    const int n = W.n + i4 * M.step;
     if (n >= rows) break;
     const int kr = min(k0 + n, nk + NPAD - 1);
     rc[i4] = (kr >= 0 && kr < nk) ? T.radc[kr * nrg + row] : rad * T.szc[kr + NPAD];
@@ -740,10 +722,10 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
     S.row[R_SH][q] = sh;
     S.row[R_NU][q] = (kr >= 0 && kr < nk) ? T.nu[rk] : T.nug[gq];
   }
-  planet_shm<true>(S.pl, st, ph);
+  planet_shm<true>(S.pl, ctl, st, ph);
 #pragma unroll
   for (int i4 = 0; i4 < 4; i4++) {
-    const int n = W.n + i4 * W.step;
+    const int n = W.n + i4 * M.step;
     if (n >= rows) break;
     const int kr = min(k0 + n, nk + NPAD - 1), s = cm.at<C>(n);
     double r, p, vt, vr, vp;
@@ -766,19 +748,19 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
   }
   __syncthreads();
   {
-    const int lane = tid & 31, wid = tid >> 5;
-    const PlanetC pl = S.pl.p;
+    const int lane = tid & 31, wid = tid >> 5, pw = min(quot16(lane, M.mG), M.P - 1);
+    const PlanetC pl = S.pl;
     Lane<C> L;
-    place_lane<C>(L, M, lim, T.ax[2] + (size_t)l * A_COUNT * ARR, S.row[0], S.ws[wid], lane);
+    place_lane<C>(L, M, pw, T.ax[2] + (size_t)l * A_COUNT * ARR, S.row[0], S.ws[wid], lane);
     L.dt = st.dt;
     L.rad = rad;
     L.irad = T.irxc[row];
     L.bq = fma(rad, rad, pl.b2);
     {
-      const int j = min(j0 + wid * M.P + min(lane / M.G, M.P - 1), nphi - 1);
+      const int j = min(j0 + wid * M.P + pw, nphi - 1);
       const double cy = T.cyc[j], sy = T.syc[j];
-      L.c0 = fma(cy, S.pl.cy, sy * S.pl.sy);
-      L.s0 = fma(sy, S.pl.cy, -(cy * S.pl.sy));
+      L.c0 = fma(cy, pl.cy, sy * pl.sy);
+      L.s0 = fma(sy, pl.cy, -(cy * pl.sy));
     }
     {
       double cs[C];
@@ -822,44 +804,22 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
   }
   __syncthreads();
   // the polar sweep is the last of a 3D step: the FARGO integer shift of each
-  // layer (rotate_rings, ppm.cu:309-322) is applied at this store.  What the
-  // epilogue needs of a layer's ring is formed once per row.
+  // layer (rotate_rings, ppm.cu:309-322) is applied at this store
   const int len = lim - 2 * NPAD;
-#pragma unroll 1
-  for (int m = tid; m < len; m += NT) {
-    const int k = k0 + m + NPAD, rk = k * nrg + row, inc = ctl.shift ? T.inc_j[rk] : 0;
-    Finish<RT> F;
-    F.ring(T, ctl, st, rk, row, k + NPAD, inc);
-    S.row[R_F][m] = F.f;
-    S.row[R_TR][m] = F.tr;
-    S.row[R_TU][m] = F.tu;
-    S.row[R_TV][m] = F.tv;
-    S.row[R_OFF][m] = F.off;
-    S.row[R_IWZ][m] = F.iwz;
-    reinterpret_cast<int2 *>(S.row[R_J])[m] = make_int2(wrapm(inc, nphi), F.rot);
-  }
-  __syncthreads();
   double rate = 0.0;
   bool bad = false;
   if (j0 + W.cl < nphi) {
-    Finish<RT> F;
-    F.irdx = T.irdx[row];
-#pragma unroll 1
-    for (int m = W.n; m < len; m += W.step) {
-      const int rk = (k0 + m + NPAD) * nrg + row, s = cm.at<C>(m + NPAD);
-      const int2 sh = reinterpret_cast<const int2 *>(S.row[R_J])[m];
-      F.f = S.row[R_F][m]; F.tr = S.row[R_TR][m]; F.tu = S.row[R_TU][m]; F.tv = S.row[R_TV][m];
-      F.off = S.row[R_OFF][m]; F.iwz = S.row[R_IWZ][m];
-      F.rot = sh.y;
-      F.cs = T.snd[rk];
-      F.cs2 = T.cs2[rk];
-      F.irc = T.irc[rk];
-      F.bs = sizeof(RT) == 4 ? T.sbg[rk] : 0.0;
-      F.bv = sizeof(RT) == 4 ? T.vbg[rk] : 0.0;
-      int jo = j0 + W.cl + sh.x;
+#pragma unroll 2
+    for (int m = W.n; m < len; m += M.step) {
+      const int k = k0 + m + NPAD, rk = k * nrg + row, s = cm.at<C>(m + NPAD);
+      const int2 sh = T.shift[rk];
+      const double rc = T.radc[rk];
+      Finish<RT> F;
+      F.ring(T, ctl, rk, row, k + NPAD, sh.y);
+      int jo = j0 + W.cl + (ctl.shift ? sh.x : 0);
       if (jo >= nphi) jo -= nphi;
       const double x = F.template cell<true, EOS>(T, P, ctl, ph, (size_t)rk * nphi + jo, jo, cw[W_R * SLOT + s],
-                                                  cw[W_V * SLOT + s], quot(cw[W_W * SLOT + s], T.radc[rk], F.irc),
+                                                  cw[W_V * SLOT + s], quot(cw[W_W * SLOT + s], rc, T.irc[rk]),
                                                   cw[W_U * SLOT + s], bad);
       rate = (x > rate || x != x) ? x : rate;
     }
@@ -897,7 +857,7 @@ __global__ void __launch_bounds__(NT, MINB) kb_sweep_x(BatchQueue q) {
     if (load_step(ctl, st)) {
       PlanesT<RT> P = batch_planes<RT>(b, 0);
       P.p0 = (sizeof(RT) == 8 && b.p0 && b.clk->ncycle == b.p0_cycle) ? b.p0 : nullptr;
-      sweep_x_tile<RT, false, 0>(*reinterpret_cast<TileShm *>(shm), b.T, P, b.ph, st, t - q.start[r]);
+      sweep_x_tile<RT, false, 0>(*reinterpret_cast<TileShm *>(shm), b.T, P, b.ph, ctl, st, t - q.start[r]);
     }
     __syncthreads();
   }
@@ -917,7 +877,7 @@ __global__ void __launch_bounds__(NT, MINB) kb_sweep_y(BatchQueue q) {
     ctl.shift = 1;
     StepIn st;
     if (load_step(ctl, st)) {
-      planet_shm<false>(S.pl, st, b.ph);
+      planet_shm<false>(S.pl, ctl, st, b.ph);
       sweep_y_task<RT, false, 0>(S.ws[wid], S.pl, b.T, batch_planes<RT>(b, 1), b.ph, ctl, st, (t - q.start[r]) * NW + wid);
     }
     __syncthreads();
@@ -931,6 +891,7 @@ namespace pgk {
 using namespace pgd;
 
 static int pencils_per_warp(int lim, int C) { return 32 / ((lim + C - 1) / C); }
+static int groups(int n, int w) { return (n + w - 1) / w; }
 
 // Cells per lane of the polar sweep: 3 or 4, whichever leaves fewer of the
 // warp's cell slots empty.  The 32-layer disk's pencils of 44 cells fill 88 of
@@ -943,20 +904,37 @@ int polar_cells(const Chunking &ch) {
   return 4 * pencils_per_warp(lim, 3) > 3 * pencils_per_warp(lim, 4) ? 3 : 4;
 }
 
-static int groups(int n, int w) { return (n + w - 1) / w; }
-static int last_group(const Chunking &ch, int C) { return NW * (ch.stuck ? 1 : pencils_per_warp(ch.lim_last, C)); }
+// tiles of a chunk of lim cells (idle: the last chunk of a multiple of 116,
+// whose cells are copied) across n pencils
+static Tile make_tile(int lim, bool idle, int C, int n) {
+  Tile t{};
+  t.lim = lim;
+  t.G = (lim + C - 1) / C;
+  t.P = idle ? 1 : 32 / t.G;
+  t.cols = NW * t.P;
+  t.step = NT / t.cols;
+  t.ng = groups(n, t.cols);
+  t.mG = 65536 / t.G + 1;
+  t.mP = 65536 / t.P + 1;
+  t.mC = 65536 / t.cols + 1;
+  t.mng = (1ull << 40) / t.ng + 1;
+  return t;
+}
+void make_tiles(Tables &T) {
+  const int rings = T.nr * T.nk, C = polar_cells(T.cz);
+  T.tx[0] = make_tile(ARR, false, 4, T.nphi);
+  T.tx[1] = make_tile(T.cx.lim_last, T.cx.stuck, 4, T.nphi);
+  T.ty[0] = make_tile(ARR, false, 4, rings);
+  T.ty[1] = make_tile(T.cy.lim_last, T.cy.stuck, 4, rings);
+  T.tz[0] = make_tile(ARR, false, 4, T.nphi);
+  T.tz[1] = make_tile(T.cz.lim_last, T.cz.stuck, C, T.nphi);
+  T.mnr = (1ull << 40) / T.nr + 1;
+}
 
 // CTAs of a run's radial, azimuthal and polar sweep
-int tiles_x(const Tables &T) {
-  return T.nk * ((T.cx.loop - 1) * groups(T.nphi, NW) + groups(T.nphi, last_group(T.cx, 4)));
-}
-int tiles_y(const Tables &T) {
-  const int rings = T.nr * T.nk;
-  return (T.cy.loop - 1) * groups(rings, NW) + groups(rings, last_group(T.cy, 4));
-}
-static int tiles_z(const Tables &T, int C) {
-  return T.nr * ((T.cz.loop - 1) * groups(T.nphi, NW) + groups(T.nphi, last_group(T.cz, C)));
-}
+int tiles_x(const Tables &T) { return T.nk * ((T.cx.loop - 1) * T.tx[0].ng + T.tx[1].ng); }
+int tiles_y(const Tables &T) { return (T.cy.loop - 1) * T.ty[0].ng + T.ty[1].ng; }
+static int tiles_z(const Tables &T) { return T.nr * ((T.cz.loop - 1) * T.tz[0].ng + T.tz[1].ng); }
 
 // the sweeps take their shared blocks (some 12 KB per warp) as dynamic shared
 // memory, above the 48 KiB default limit: set per device before a launch
@@ -1014,7 +992,7 @@ void sweep_y(const Tables &T, const PlanesT<RT> &P, const Phys &ph, const SweepC
 
 template <class RT>
 void sweep_z(const Tables &T, const PlanesT<RT> &P, const Phys &ph, const SweepCtl &c, int ntop, cudaStream_t s) {
-  const int C = polar_cells(T.cz), n = tiles_z(T, C);
+  const int C = polar_cells(T.cz), n = tiles_z(T);
   if constexpr (sizeof(RT) == 8) {
     if (ph.eos) {
       if (C == 3) k_sweep_z<RT, 1, 3><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c, ntop);

@@ -157,24 +157,17 @@ __device__ __forceinline__ void right_of(const double (&a)[C], double (&o)[C]) {
   PG_CELLS o[c] = c < C - 1 ? a[c < C - 1 ? c + 1 : 0] : r;
 }
 
-// The planet of a step as the forces use it (forces.cu:23-182): mass over
-// distance squared factors and the star's share of the mass (3D with a
-// planet: the reference's two-body reduced masses).
-struct PlanetC {
-  double m, x, ix2, b2, star;            // b2 = x^2 + rs^2
-  double y, vy;
-};
-template <bool THREED>
-__device__ __forceinline__ PlanetC planet_consts(const Body &b, const Phys &ph) {
+__device__ __forceinline__ PlanetC planet_consts(const Body &b, bool three, bool plnt) {
   PlanetC p;
-  const double stm = THREED ? 1.0 / (1.0 + b.m) : 1.0;
+  const double stm = three ? 1.0 / (1.0 + b.m) : 1.0;
   p.m = b.m * stm;
   p.x = b.x;
   p.ix2 = 1.0 / (b.x * b.x);
   p.b2 = fma(b.x, b.x, b.rs * b.rs);
-  p.star = ph.plnt ? stm : 1.0;
+  p.star = plnt ? stm : 1.0;
   p.y = b.y;
   p.vy = b.vy;
+  sincos(b.y, &p.sy, &p.cy);
   return p;
 }
 
