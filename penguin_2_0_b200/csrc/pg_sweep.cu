@@ -65,6 +65,10 @@ __device__ __forceinline__ bool load_step(const SweepCtl &c, StepIn &s) {
   return true;
 }
 
+// Keeps the loads before it ahead of what follows: a tile's loads do not wait
+// for the look at the clock.
+__device__ __forceinline__ void in_flight() { asm volatile("" ::: "memory"); }
+
 // The planet's constants into shared memory: from the clock, or (calls with a
 // planet of their own) formed by one thread while the others load.
 template <bool THREED>
@@ -371,7 +375,8 @@ __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const 
   __syncthreads();
   if (j0 + W.cl < nphi) {
 #pragma unroll 2
-    for (int n = W.n + NPAD; n < lim - NPAD; n += M.step) {
+    for (int n = W.n + 4; n < lim - NPAD; n += M.step) {
+      if (n < NPAD) continue;          // a warp's rows start with a lane's cells: different banks
       const int rk = k * nrg + row0 + n;
       const size_t o = (size_t)rk * nphi + j0 + W.cl;
       const double bs = sizeof(RT) == 4 ? T.sbg[rk] : 0.0, bv = sizeof(RT) == 4 ? T.vbg[rk] : 0.0;
@@ -474,7 +479,7 @@ struct __align__(16) YShm {
 };
 template <class RT, bool THREED, int EOS>
 __device__ __forceinline__ void sweep_y_task(double *ws, const PlanetC &SP, const Tables &T, const PlanesT<RT> &P,
-                                             const Phys &ph, const SweepCtl &ctl, const StepIn &st, int t) {
+                                             const Phys &ph, const SweepCtl &ctl, const StepIn &st, bool run, int t) {
   constexpr int C = 4;
   const int nphi = T.nphi, nrg = T.nrg, full = T.cy.loop - 1, rings = T.nr * T.nk, lane = threadIdx.x & 31;
   // rings of one chunk side by side: the warps of an SM share its tables.  The
@@ -493,7 +498,7 @@ __device__ __forceinline__ void sweep_y_task(double *ws, const PlanetC &SP, cons
   }
   const int lim = M.lim;
   if (last && T.cy.stuck) {
-    if (ring >= rings) return;
+    if (ring >= rings || !run) return;
     // ppm.cu:196 gives this chunk lim = 12: its cells keep their values and
     // only move with the ring's rotation
     const int k = ring / T.nr, row = ring % T.nr + NPAD, rk = k * nrg + row;
@@ -542,8 +547,9 @@ __device__ __forceinline__ void sweep_y_task(double *ws, const PlanetC &SP, cons
     L.vr = T.res_v[rk] * L.irad;
     L.cs2 = T.cs2[rk];
     const double snd = T.snd[rk], rs = T.rxc[row];
-    // the planet's constants, formed meanwhile by the CTA's last warp
-    __syncthreads();
+    in_flight();
+    if (!run) return;
+    __syncthreads();                     // the planet's constants
     const PlanetC pl = SP;
     {
       L.bq = fma(rs, rs, pl.b2);         // the planet's distance sees the spherical radius in 3D
@@ -641,10 +647,10 @@ __global__ void __launch_bounds__(NT, MINB) k_sweep_y(Tables T, PlanesT<RT> P, P
   extern __shared__ __align__(16) unsigned char shm[];
   YShm<EOS> &S = *reinterpret_cast<YShm<EOS> *>(shm);
   StepIn st;
-  if (!load_step(ctl, st)) return;
+  const bool run = load_step(ctl, st);
   planet_shm<THREED>(S.pl, ctl, st, ph);
   const int wid = threadIdx.x >> 5;
-  sweep_y_task<RT, THREED, EOS>(S.ws[wid], S.pl, T, P, ph, ctl, st, blockIdx.x * NW + wid);
+  sweep_y_task<RT, THREED, EOS>(S.ws[wid], S.pl, T, P, ph, ctl, st, run, blockIdx.x * NW + wid);
 }
 
 // ---------------------------------------------------------------------------
@@ -659,7 +665,7 @@ __global__ void __launch_bounds__(NT, MINB) k_sweep_y(Tables T, PlanesT<RT> P, P
 // (one layer per row) are shared by the whole CTA.
 template <class RT, int EOS, int C>
 __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const PlanesT<RT> &P, const Phys &ph,
-                                             const SweepCtl &ctl, const StepIn &st, int ntop, int t) {
+                                             const SweepCtl &ctl, const StepIn &st, bool run, int ntop, int t) {
   const int nphi = T.nphi, nrg = T.nrg, nk = T.nk, full = T.cz.loop - 1, tid = threadIdx.x;
   const int nfull = full * T.tz[0].ng * T.nr;
   const bool last = t >= nfull;
@@ -669,6 +675,7 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
   const int j0 = (t - q * M.ng) * M.cols;
   const int l = last ? full : q / T.nr, i = last ? q : q - l * T.nr, row = i + NPAD;
   if (last && T.cz.stuck) {
+    if (!run) return;
 #pragma unroll 1
     for (int e = tid; e < REAL * NW; e += NT) {
       const int k = REAL * l + e / NW, j = j0 + e % NW;
@@ -689,13 +696,11 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
   // every load of the tile in flight before the first is used; a ghost layer
   // below or a fixed one above comes from the ghost tables (no FARGO
   // residual), a mirrored one from its mirror image
-  RT a[4][4];
-  double rc[4], cs2[4], bs[4], bv[4];
+  RT a[C][4];
+  double rc[C], cs2[C], bs[C], bv[C];
 #pragma unroll
-  for (int i4 = 0; i4 < 4; i4++) {
-    const int n = W.n + i4 * M.step;
-    if (n >= rows) break;
-    const int kr = min(k0 + n, nk + NPAD - 1);
+  for (int i4 = 0; i4 < C; i4++) {
+    const int kr = min(k0 + W.n + i4 * M.step, nk + NPAD - 1);
     rc[i4] = (kr >= 0 && kr < nk) ? T.radc[kr * nrg + row] : rad * T.szc[kr + NPAD];
     if (kr >= 0 && (kr < nk || ntop == 0)) {
       const int km = kr >= nk ? 2 * nk - 1 - kr : kr, rk = km * nrg + row;
@@ -709,22 +714,31 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
       bv[i4] = sizeof(RT) == 4 ? T.vbg[rk] : 0.0;
     }
   }
+  double snd = 0.0, nu = 0.0, om = 0.0;  // of row tid: sound speed (a fixed layer: its square over gamma), viscosity, residual rotation
+  bool fixed = false;
   if (tid < rows) {
     const int kr = min(k0 + tid, nk + NPAD - 1);
-    const bool fixed = kr < 0 || (kr >= nk && ntop != 0);
+    fixed = kr < 0 || (kr >= nk && ntop != 0);
     const int km = kr >= nk ? 2 * nk - 1 - kr : kr, rk = km * nrg + row;
     const int gq = (kr < 0 ? kr + NPAD : kr - nk + NPAD) * T.nr + i;
-    const int q = table_pos(tid, C, M.G);
-    S.row[R_SND][q] = fixed ? sqrt(ph.gam * T.csg[gq]) : T.snd[rk];
-    double sh, ch;
-    sincos_near(0.5 * st.dt * ((fixed ? 0.0 : T.res_v[rk] * T.irc[rk]) - st.pl.vy), sh, ch);
-    S.row[R_CH][q] = ch;
-    S.row[R_SH][q] = sh;
-    S.row[R_NU][q] = (kr >= 0 && kr < nk) ? T.nu[rk] : T.nug[gq];
+    snd = fixed ? T.csg[gq] : T.snd[rk];
+    om = fixed ? 0.0 : T.res_v[rk] * T.irc[rk];
+    nu = (kr >= 0 && kr < nk) ? T.nu[rk] : T.nug[gq];
   }
   planet_shm<true>(S.pl, ctl, st, ph);
+  in_flight();
+  if (!run) return;
+  if (tid < rows) {
+    const int q = table_pos(tid, C, M.G);
+    double sh, ch;
+    sincos_near(0.5 * st.dt * (om - st.pl.vy), sh, ch);
+    S.row[R_SND][q] = fixed ? sqrt(ph.gam * snd) : snd;
+    S.row[R_CH][q] = ch;
+    S.row[R_SH][q] = sh;
+    S.row[R_NU][q] = nu;
+  }
 #pragma unroll
-  for (int i4 = 0; i4 < 4; i4++) {
+  for (int i4 = 0; i4 < C; i4++) {
     const int n = W.n + i4 * M.step;
     if (n >= rows) break;
     const int kr = min(k0 + n, nk + NPAD - 1), s = cm.at<C>(n);
@@ -831,8 +845,8 @@ template <class RT, int EOS, int C>
 __global__ void __launch_bounds__(NT, MINB) k_sweep_z(Tables T, PlanesT<RT> P, Phys ph, SweepCtl ctl, int ntop) {
   extern __shared__ __align__(16) unsigned char shm[];
   StepIn st;
-  if (!load_step(ctl, st)) return;
-  sweep_z_tile<RT, EOS, C>(*reinterpret_cast<TileShm *>(shm), T, P, ph, ctl, st, ntop, blockIdx.x);
+  const bool run = load_step(ctl, st);
+  sweep_z_tile<RT, EOS, C>(*reinterpret_cast<TileShm *>(shm), T, P, ph, ctl, st, run, ntop, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -876,10 +890,9 @@ __global__ void __launch_bounds__(NT, MINB) kb_sweep_y(BatchQueue q) {
     ctl.fuse = 1;
     ctl.shift = 1;
     StepIn st;
-    if (load_step(ctl, st)) {
-      planet_shm<false>(S.pl, ctl, st, b.ph);
-      sweep_y_task<RT, false, 0>(S.ws[wid], S.pl, b.T, batch_planes<RT>(b, 1), b.ph, ctl, st, (t - q.start[r]) * NW + wid);
-    }
+    const bool run = load_step(ctl, st);
+    planet_shm<false>(S.pl, ctl, st, b.ph);
+    sweep_y_task<RT, false, 0>(S.ws[wid], S.pl, b.T, batch_planes<RT>(b, 1), b.ph, ctl, st, run, (t - q.start[r]) * NW + wid);
     __syncthreads();
   }
 }
