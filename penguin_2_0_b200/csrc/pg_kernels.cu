@@ -102,6 +102,7 @@ template <class RT>
 __global__ void k_cfl(Tables T, const RT *R, const RT *U, const RT *V, const RT *W, const double *P0, Phys ph,
                       double frrot, int ndim, unsigned long long *out, DevClock *clk, int rot_pending, unsigned *counter,
                       unsigned long long *hout) {
+  after_previous();
   __shared__ double red[32];
   if (clk) {
     if (clk->halted) return;
@@ -148,6 +149,7 @@ __global__ void k_cfl(Tables T, const RT *R, const RT *U, const RT *V, const RT 
 // last sweep's epilogue
 template <class RT>
 __global__ void k_damp(Tables T, RT *R, RT *U, RT *V, RT *W, double dt, const DevClock *clk, int ndim) {
+  after_previous();
   if (clk) {
     if (clk->halted) return;
     dt = clk->dt_step;
@@ -330,13 +332,13 @@ void cfl(const Tables &T, const RT *r, const RT *u, const RT *v, const RT *w, co
          double frrot, int ndim, unsigned long long *out, DevClock *clk, int rot_pending, unsigned *counter,
          unsigned long long *hout, cudaStream_t s) {
   dim3 grid(T.nr, T.nk);
-  k_cfl<RT><<<grid, 256, 0, s>>>(T, r, u, v, w, p0, ph, frrot, ndim, out, clk, rot_pending, counter, hout);
+  launch(k_cfl<RT>, grid, 256, 0, s, T, r, u, v, w, p0, ph, frrot, ndim, out, clk, rot_pending, counter, hout);
 }
 
 template <class RT>
 void damp(const Tables &T, RT *r, RT *u, RT *v, RT *w, double dt, const DevClock *clk, int ndim, cudaStream_t s) {
   dim3 grid(T.nr, T.nk);
-  k_damp<RT><<<grid, 256, 0, s>>>(T, r, u, v, w, dt, clk, ndim);
+  launch(k_damp<RT>, grid, 256, 0, s, T, r, u, v, w, dt, clk, ndim);
 }
 #define PG_AROUND(RT)                                                                                                   \
   template void cfl<RT>(const Tables &, const RT *, const RT *, const RT *, const RT *, const double *, const Phys &,   \

@@ -63,10 +63,12 @@ __device__ __forceinline__ void finish_ring(const Tables &T, int t, double dt, d
 __device__ __forceinline__ int rotated(const Tables &T, int rk) { return wrap1(T.rot_j[rk] + T.inc_j[rk], T.nphi); }
 
 __global__ void k_index(Tables T, double dt, double frrot, int fargo) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < T.nr * T.nk) index_shift_ring(T, t, dt, frrot, fargo);
 }
 __global__ void k_rotate(Tables T) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T.nr * T.nk) return;
   const int rk = t / T.nr * T.nrg + t % T.nr + NPAD;
@@ -215,6 +217,7 @@ __device__ __forceinline__ bool last_cta(unsigned *counter, unsigned nb) {
 template <class RT>
 __global__ void __launch_bounds__(ST) k_reduce(Tables T, const RT *R, Body pl, double exclude, int mode, int plnt,
                                                double p_alpha, int ndim, double *part, unsigned *counter, double *out) {
+  after_previous();
   __shared__ double red[ST];
   const bool zero = mode != 0 && plnt && ndim != 2;     // the reference's force sums are 2D
   const RingForce F(pl, exclude, p_alpha);
@@ -443,6 +446,7 @@ __device__ __forceinline__ void between_body(StepShm &S, const Tables &T, const 
 template <class RT>
 __global__ void __launch_bounds__(ST) k_between(Tables T, const RT *R, DevClock *clk, double *part, unsigned *counter,
                                                 double p_alpha, int fargo, int torque, int ndim, int fl) {
+  after_previous();
   __shared__ StepShm S;
   between_body<RT>(S, T, R, clk, part, counter, p_alpha, fargo, torque, ndim, fl, blockIdx.x, gridDim.x);
 }
@@ -450,6 +454,7 @@ __global__ void __launch_bounds__(ST) k_between(Tables T, const RT *R, DevClock 
 // members' CTAs by the queue's prefix sums
 template <class RT>
 __global__ void __launch_bounds__(ST) kb_between(BatchQueue q, int fl) {
+  after_previous();
   __shared__ StepShm S;
   const int r = batch_find(q, blockIdx.x);
   const BatchRun &b = q.runs[r];
@@ -464,6 +469,7 @@ __global__ void __launch_bounds__(ST) kb_between(BatchQueue q, int fl) {
 template <class RT>
 __global__ void __launch_bounds__(ST) k_moving(Tables T, const RT *R, DevClock *clk, double *part, unsigned *counter,
                                                double p_alpha, int ndim) {
+  after_previous();
   __shared__ StepShm S;
   const int rings = T.nr * T.nk, tid = threadIdx.x;
   clock_in(S, clk);
@@ -518,28 +524,28 @@ int between_ctas(int rings) {
 }
 
 void index_shift(const Tables &T, double dt, double frrot, int fargo, cudaStream_t s) {
-  k_index<<<(T.nr * T.nk + 127) / 128, 128, 0, s>>>(T, dt, frrot, fargo);
+  launch(k_index, (T.nr * T.nk + 127) / 128, 128, 0, s, T, dt, frrot, fargo);
 }
-void rotate(const Tables &T, cudaStream_t s) { k_rotate<<<(T.nr * T.nk + 127) / 128, 128, 0, s>>>(T); }
+void rotate(const Tables &T, cudaStream_t s) { launch(k_rotate, (T.nr * T.nk + 127) / 128, 128, 0, s, T); }
 
 template <class RT>
 void reduce(const Tables &T, const RT *r, const Body &pl, double exclude, int mode, int plnt, double p_alpha, int ndim,
             double *part, unsigned *counter, double *out, cudaStream_t s) {
-  k_reduce<RT><<<ring_ctas(T.nr * T.nk), ST, 0, s>>>(T, r, pl, exclude, mode, plnt, p_alpha, ndim, part, counter, out);
+  launch(k_reduce<RT>, ring_ctas(T.nr * T.nk), ST, 0, s, T, r, pl, exclude, mode, plnt, p_alpha, ndim, part, counter, out);
 }
 template <class RT>
 void between(const Tables &T, const RT *r, DevClock *clk, double *part, unsigned *counter, double p_alpha, int fargo,
              int plnt, int ndim, int fl, cudaStream_t s) {
-  k_between<RT><<<between_ctas(T.nr * T.nk), ST, 0, s>>>(T, r, clk, part, counter, p_alpha, fargo, plnt && ndim == 2, ndim, fl);
+  launch(k_between<RT>, between_ctas(T.nr * T.nk), ST, 0, s, T, r, clk, part, counter, p_alpha, fargo, plnt && ndim == 2, ndim, fl);
 }
 template <class RT>
 void moving(const Tables &T, const RT *r, DevClock *clk, double *part, unsigned *counter, double p_alpha, int ndim,
             cudaStream_t s) {
-  k_moving<RT><<<ring_ctas(T.nr * T.nk), ST, 0, s>>>(T, r, clk, part, counter, p_alpha, ndim);
+  launch(k_moving<RT>, ring_ctas(T.nr * T.nk), ST, 0, s, T, r, clk, part, counter, p_alpha, ndim);
 }
 template <class RT>
 void batch_between(const BatchQueue &q, int fl, cudaStream_t s) {
-  if (q.total > 0) kb_between<RT><<<q.total, ST, 0, s>>>(q, fl);
+  if (q.total > 0) launch(kb_between<RT>, q.total, ST, 0, s, q, fl);
 }
 #define PG_STEP(RT)                                                                                                      \
   template void reduce<RT>(const Tables &, const RT *, const Body &, double, int, int, double, int, double *, unsigned *, \

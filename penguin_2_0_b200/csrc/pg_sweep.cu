@@ -392,6 +392,7 @@ __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const 
 template <class RT, bool THREED, int EOS>
 __global__ void __launch_bounds__(NT, MINB) k_sweep_x(Tables T, PlanesT<RT> P, Phys ph, SweepCtl ctl) {
   extern __shared__ __align__(16) unsigned char shm[];
+  after_previous();
   StepIn st;
   if (!load_step(ctl, st)) return;
   sweep_x_tile<RT, THREED, EOS>(*reinterpret_cast<TileShm *>(shm), T, P, ph, ctl, st, blockIdx.x);
@@ -645,6 +646,7 @@ __device__ __forceinline__ void sweep_y_task(double *ws, const PlanetC &SP, cons
 template <class RT, bool THREED, int EOS>
 __global__ void __launch_bounds__(NT, MINB) k_sweep_y(Tables T, PlanesT<RT> P, Phys ph, SweepCtl ctl) {
   extern __shared__ __align__(16) unsigned char shm[];
+  after_previous();
   YShm<EOS> &S = *reinterpret_cast<YShm<EOS> *>(shm);
   StepIn st;
   const bool run = load_step(ctl, st);
@@ -844,6 +846,7 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
 template <class RT, int EOS, int C>
 __global__ void __launch_bounds__(NT, MINB) k_sweep_z(Tables T, PlanesT<RT> P, Phys ph, SweepCtl ctl, int ntop) {
   extern __shared__ __align__(16) unsigned char shm[];
+  after_previous();
   StepIn st;
   const bool run = load_step(ctl, st);
   sweep_z_tile<RT, EOS, C>(*reinterpret_cast<TileShm *>(shm), T, P, ph, ctl, st, run, ntop, blockIdx.x);
@@ -862,6 +865,7 @@ __device__ __forceinline__ const PlanesT<RT> &batch_planes(const BatchRun &b, in
 template <class RT>
 __global__ void __launch_bounds__(NT, MINB) kb_sweep_x(BatchQueue q) {
   extern __shared__ __align__(16) unsigned char shm[];
+  after_previous();
   for (int t = blockIdx.x; t < q.total; t += gridDim.x) {
     const int r = batch_find(q, t);
     const BatchRun &b = q.runs[r];
@@ -880,6 +884,7 @@ __global__ void __launch_bounds__(NT, MINB) kb_sweep_x(BatchQueue q) {
 template <class RT>
 __global__ void __launch_bounds__(NT, MINB) kb_sweep_y(BatchQueue q) {
   extern __shared__ __align__(16) unsigned char shm[];
+  after_previous();
   YShm<0> &S = *reinterpret_cast<YShm<0> *>(shm);
   const int wid = threadIdx.x >> 5;
   for (int t = blockIdx.x; t < q.total; t += gridDim.x) {
@@ -980,13 +985,13 @@ void sweep_x(const Tables &T, const PlanesT<RT> &P, const Phys &ph, const SweepC
   const int n = tiles_x(T);
   if constexpr (sizeof(RT) == 8) {
     if (ph.eos) {
-      if (ndim == 3) k_sweep_x<RT, true, 1><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c);
-      else k_sweep_x<RT, false, 1><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c);
+      if (ndim == 3) launch(k_sweep_x<RT, true, 1>, n, NT, sizeof(TileShm), s, T, P, ph, c);
+      else launch(k_sweep_x<RT, false, 1>, n, NT, sizeof(TileShm), s, T, P, ph, c);
       return;
     }
   }
-  if (ndim == 3) k_sweep_x<RT, true, 0><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c);
-  else k_sweep_x<RT, false, 0><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c);
+  if (ndim == 3) launch(k_sweep_x<RT, true, 0>, n, NT, sizeof(TileShm), s, T, P, ph, c);
+  else launch(k_sweep_x<RT, false, 0>, n, NT, sizeof(TileShm), s, T, P, ph, c);
 }
 
 template <class RT>
@@ -994,13 +999,13 @@ void sweep_y(const Tables &T, const PlanesT<RT> &P, const Phys &ph, const SweepC
   const int n = tiles_y(T);
   if constexpr (sizeof(RT) == 8) {
     if (ph.eos) {
-      if (ndim == 3) k_sweep_y<RT, true, 1><<<n, NT, sizeof(YShm<1>), s>>>(T, P, ph, c);
-      else k_sweep_y<RT, false, 1><<<n, NT, sizeof(YShm<1>), s>>>(T, P, ph, c);
+      if (ndim == 3) launch(k_sweep_y<RT, true, 1>, n, NT, sizeof(YShm<1>), s, T, P, ph, c);
+      else launch(k_sweep_y<RT, false, 1>, n, NT, sizeof(YShm<1>), s, T, P, ph, c);
       return;
     }
   }
-  if (ndim == 3) k_sweep_y<RT, true, 0><<<n, NT, sizeof(YShm<0>), s>>>(T, P, ph, c);
-  else k_sweep_y<RT, false, 0><<<n, NT, sizeof(YShm<0>), s>>>(T, P, ph, c);
+  if (ndim == 3) launch(k_sweep_y<RT, true, 0>, n, NT, sizeof(YShm<0>), s, T, P, ph, c);
+  else launch(k_sweep_y<RT, false, 0>, n, NT, sizeof(YShm<0>), s, T, P, ph, c);
 }
 
 template <class RT>
@@ -1008,22 +1013,22 @@ void sweep_z(const Tables &T, const PlanesT<RT> &P, const Phys &ph, const SweepC
   const int C = polar_cells(T.cz), n = tiles_z(T);
   if constexpr (sizeof(RT) == 8) {
     if (ph.eos) {
-      if (C == 3) k_sweep_z<RT, 1, 3><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c, ntop);
-      else k_sweep_z<RT, 1, 4><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c, ntop);
+      if (C == 3) launch(k_sweep_z<RT, 1, 3>, n, NT, sizeof(TileShm), s, T, P, ph, c, ntop);
+      else launch(k_sweep_z<RT, 1, 4>, n, NT, sizeof(TileShm), s, T, P, ph, c, ntop);
       return;
     }
   }
-  if (C == 3) k_sweep_z<RT, 0, 3><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c, ntop);
-  else k_sweep_z<RT, 0, 4><<<n, NT, sizeof(TileShm), s>>>(T, P, ph, c, ntop);
+  if (C == 3) launch(k_sweep_z<RT, 0, 3>, n, NT, sizeof(TileShm), s, T, P, ph, c, ntop);
+  else launch(k_sweep_z<RT, 0, 4>, n, NT, sizeof(TileShm), s, T, P, ph, c, ntop);
 }
 
 template <class RT>
 void batch_sweep_x(const BatchQueue &q, int grid, cudaStream_t s) {
-  if (q.total > 0) kb_sweep_x<RT><<<grid > 0 && grid < q.total ? grid : q.total, NT, sizeof(TileShm), s>>>(q);
+  if (q.total > 0) launch(kb_sweep_x<RT>, grid > 0 && grid < q.total ? grid : q.total, NT, sizeof(TileShm), s, q);
 }
 template <class RT>
 void batch_sweep_y(const BatchQueue &q, int grid, cudaStream_t s) {
-  if (q.total > 0) kb_sweep_y<RT><<<grid > 0 && grid < q.total ? grid : q.total, NT, sizeof(YShm<0>), s>>>(q);
+  if (q.total > 0) launch(kb_sweep_y<RT>, grid > 0 && grid < q.total ? grid : q.total, NT, sizeof(YShm<0>), s, q);
 }
 
 #define PG_SWEEPS(RT)                                                                                              \
