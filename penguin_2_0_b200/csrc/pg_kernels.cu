@@ -81,6 +81,11 @@ __global__ void k_tables(Tables T, Phys ph, int ndim, double kill_rin, double ki
   cs2[t] = ph.sc2 * pow(rc, -ph.p_beta);          // get_cs2 disk_profile.cu:39-42
   const_cast<double *>(T.irc)[t] = 1.0 / rc;
   const_cast<double *>(T.snd)[t] = sqrt(ph.gam * cs2[t]);
+  RingOut &o = T.ro[t];
+  o.f = o.off = 0.0;
+  o.cs = T.snd[t]; o.irc = T.irc[t]; o.rc = rc;
+  o.irdx = 1.0 / T.rdx[row];
+  o.iwz = ndim == 3 ? __dmul_rn(1.0 / T.dz[k + NPAD], 1.0 / T.rxc[row]) : 0.0;
   nu[t] = ph.vis_nu * pow(rc, ph.p_alpha);        // get_nu disk_profile.cu:149-152
   double g = 0.0;
   bool interior = row >= NPAD && row < T.nr + NPAD;

@@ -38,6 +38,16 @@ struct Tile {
 // of the azimuth
 struct PlanetC {
   double m, x, ix2, b2, star, y, vy, cy, sy;
+  double2 turn;              // 3D: turn_of a ring with no residual velocity (fixed layers)
+};
+
+// What the last sweep of a step needs of a ring at its store, in one place: four
+// 16-byte loads where an array each took nine and their addresses.
+struct __align__(16) RingOut {
+  double f, off;             // this step's damping factor and CFL frame offset (pg_step.cu)
+  double cs, irc, rc;        // sound speed (EOS 0), 1/r_cyl, r_cyl
+  double irdx, iwz;          // 1/dr, 1/(r dtheta)
+  int2 shift;                // inc_j and rot_j + inc_j modulo nphi
 };
 
 // Geometry and per-ring tables, all device pointers.  A "row" counts radial
@@ -66,8 +76,8 @@ struct Tables {
   const double *sbg;                            // [nk*nrg] FP32 runs: Sigma background (val.r / ghost r)
   double *res_v, *rot_v;                        // [nk*nrg]
   int *inc_j, *rot_j;                           // [nk*nrg]
-  int2 *shift;                                  // [nk*nrg]: inc_j and rot_j + inc_j modulo nphi
-  double2 *fin;                                 // [nk*nrg]: this step's damping factor and CFL frame offset (pg_step.cu)
+  double2 *turn;                                // [nk*nrg], 3D: cos and sin of the planet's angle's change in dt/2 (turn_of)
+  RingOut *ro;                                  // [nk*nrg]
 };
 
 // State planes a sweep reads and writes: FP64 Sigma, v_r, v_phi, v_theta, or
@@ -195,7 +205,7 @@ __device__ __forceinline__ int quot40(int a, int d, unsigned long long m) {
 }
 // the sweeps' copy of a ring's shift
 __device__ __forceinline__ void set_shift(const Tables &T, int rk, int inc, int rot) {
-  T.shift[rk] = make_int2(wrapm(inc, T.nphi), wrapm(rot + inc, T.nphi));
+  T.ro[rk].shift = make_int2(wrapm(inc, T.nphi), wrapm(rot + inc, T.nphi));
 }
 // the run of tile t of a batch queue, by bisection in its prefix sums
 __device__ __forceinline__ int batch_find(const BatchQueue &q, int t) {

@@ -214,7 +214,7 @@ static int check_launch(pg_run *run, int n) {
 // doubles of a run's table block (pg_create lays it out)
 static size_t table_elems(size_t nr, size_t nphi, size_t nk) {
   const size_t nrg = nr + 2 * NPAD, nring = nk * nrg, nz = nk + 2 * NPAD;
-  size_t n = 7 * nrg + 13 * nring + 7 * nphi + 6 * nz + 6 * (size_t)2 * NPAD * nr;
+  size_t n = 7 * nrg + 21 * nring + 7 * nphi + 6 * nz + 6 * (size_t)2 * NPAD * nr;
   for (size_t len : {nr, nphi, nk}) n += pgk::axis_table_elems(pgd::make_chunking((int)len));
   return n;
 }
@@ -359,7 +359,7 @@ int pg_create(const pg_params *p, int device, pg_run **out) {
   size_t nz = (size_t)nk + 2 * NPAD;
   run->tab_elems = table_elems(nr, nphi, nk);
   if (cudaMalloc(&run->tab, run->tab_elems * sizeof(double)) != cudaSuccess) return bail(PG_ERR_NOMEM);
-  if (cudaMalloc(&run->itab, 4 * nring * sizeof(int)) != cudaSuccess) return bail(PG_ERR_NOMEM);
+  if (cudaMalloc(&run->itab, 2 * nring * sizeof(int)) != cudaSuccess) return bail(PG_ERR_NOMEM);
   double *t = run->tab;
   pgd::Tables &T = run->T;
   T.nr = nr; T.nphi = nphi; T.nk = nk; T.nrg = nrg;
@@ -372,7 +372,7 @@ int pg_create(const pg_params *p, int device, pg_run **out) {
     T.ax[a] = t;
     t += pgk::axis_table_elems(a == 0 ? T.cx : a == 1 ? T.cy : T.cz);
   }
-  T.fin = (double2 *)t; t += 2 * nring;
+  T.ro = (pgd::RingOut *)t; t += 8 * nring; T.turn = (double2 *)t; t += 2 * nring;
   T.rx = t; t += nrg; T.rdx = t; t += nrg; T.rxvol = t; t += nrg; T.rxc = t; t += nrg;
   T.irdx = t; t += nrg; T.irxc = t; t += nrg; T.rpa = t; t += nrg;
   T.radc = t; t += nring; T.cs2 = t; t += nring; T.nu = t; t += nring; T.irc = t; t += nring; T.snd = t; t += nring;
@@ -392,7 +392,7 @@ int pg_create(const pg_params *p, int device, pg_run **out) {
   if (cudaMalloc(&run->sbg, nring * sizeof(double)) != cudaSuccess) return bail(PG_ERR_NOMEM);
   T.sbg = run->sbg;
 
-  T.shift = (int2 *)run->itab; T.inc_j = run->itab + 2 * nring; T.rot_j = run->itab + 3 * nring;
+  T.inc_j = run->itab; T.rot_j = run->itab + nring;
   // scratch
   if (cudaMalloc(&run->ring_part, 2 * (size_t)nr * nk * sizeof(double)) != cudaSuccess) return bail(PG_ERR_NOMEM);
   if (cudaMalloc(&run->counter, sizeof(unsigned int)) != cudaSuccess) return bail(PG_ERR_NOMEM);
@@ -1216,7 +1216,7 @@ extern "C" size_t pg_run_device_bytes(const pg_params *p) {
   size_t b = 2 * (size_t)nf * up(pe * es);
   if (p->precision != 1) b += up(pe * sizeof(double));                         // p0
   b += up(table_elems(nr, nphi, nk) * sizeof(double));
-  b += up(4 * nring * sizeof(int)) + 3 * up(nring * sizeof(double));           // itab, rot_v, vbg, sbg
+  b += up(2 * nring * sizeof(int)) + 3 * up(nring * sizeof(double));           // itab, rot_v, vbg, sbg
   b += up(2 * nr * nk * sizeof(double)) + up(4) + up(8) + up(sizeof(pgd::DevClock));
   b += up((size_t)4096 * pgd::HIST_COLS * sizeof(double));
   return b;

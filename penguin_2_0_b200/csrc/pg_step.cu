@@ -53,11 +53,14 @@ __device__ __forceinline__ void index_shift_ring(const Tables &T, int t, double 
   set_shift(T, rk, T.inc_j[rk], T.rot_j[rk]);
 }
 // what the device loop's last sweep needs of a ring: this step's damping
-// factor and the frame offset of the next get_dt's azimuthal rate
-__device__ __forceinline__ void finish_ring(const Tables &T, int t, double dt, double frrot_next) {
+// factor, the frame offset of the next get_dt's azimuthal rate and (polar) the
+// planet's turn against it in half a step
+__device__ __forceinline__ void finish_ring(const Tables &T, int t, double dt, double frrot_next, double vy, int ndim) {
   const int rk = t / T.nr * T.nrg + t % T.nr + NPAD;
   const double g = T.damp_g[rk];
-  T.fin[rk] = make_double2(g > 0.0 ? g * (dt * T.damp_pw[rk]) : 0.0, fma(frrot_next, T.radc[rk], T.rot_v[rk]));
+  T.ro[rk].f = g > 0.0 ? g * (dt * T.damp_pw[rk]) : 0.0;
+  T.ro[rk].off = fma(frrot_next, T.radc[rk], T.rot_v[rk]);
+  if (ndim == 3) T.turn[rk] = turn_of(dt, T.res_v[rk], T.irc[rk], vy);
 }
 // rotate_rings ppm.cu:309-322
 __device__ __forceinline__ int rotated(const Tables &T, int rk) { return wrap1(T.rot_j[rk] + T.inc_j[rk], T.nphi); }
@@ -339,7 +342,7 @@ __device__ __forceinline__ bool step_pre(DevClock &c, double &frrot) {
   }
   c.frrot_next = fr;
   c.cfl_bits = 0ull;
-  c.pc = planet_consts(c.planet, c.ndim == 3, c.plnt_flag > 0);
+  c.pc = planet_consts(c.planet, c.ndim == 3, c.plnt_flag > 0, dt);
   return true;
 }
 
@@ -415,7 +418,7 @@ __device__ __forceinline__ void between_body(StepShm &S, const Tables &T, const 
         T.rot_j[rk] = rot;
         if (S.run) {
           index_shift_ring(T, rt, S.c.dt_step, S.frrot_pre, fargo);
-          finish_ring(T, rt, S.c.dt_step, S.c.frrot_next);
+          finish_ring(T, rt, S.c.dt_step, S.c.frrot_next, S.c.planet.vy, ndim);
         }
       }
     }
@@ -425,7 +428,7 @@ __device__ __forceinline__ void between_body(StepShm &S, const Tables &T, const 
       if (post) T.rot_j[rk] = rotated(T, rk);
       if (S.run) {
         index_shift_ring(T, rt, S.c.dt_step, S.frrot_pre, fargo);
-        finish_ring(T, rt, S.c.dt_step, S.c.frrot_next);
+        finish_ring(T, rt, S.c.dt_step, S.c.frrot_next, S.c.planet.vy, ndim);
       }
     }
   }

@@ -78,7 +78,7 @@ __device__ __forceinline__ void planet_shm(PlanetC &S, const SweepCtl &ctl, cons
   if (ctl.clk) {
     if (t >= 0 && t < N) reinterpret_cast<double *>(&S)[t] = reinterpret_cast<const double *>(&ctl.clk->pc)[t];
   } else if (t == 0) {
-    S = planet_consts(st.pl, THREED, ph.plnt);
+    S = planet_consts(st.pl, THREED, ph.plnt, st.dt);
   }
 }
 
@@ -265,7 +265,7 @@ __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const 
     const int rk = k * nrg + min(row0 + tid, nrg - 1);
     const double snd = T.snd[rk], nu = T.nu[rk], r = T.radc[rk], irc = T.irc[rk], res = T.res_v[rk];
     const int q = table_pos(tid, C, M.G);
-    S.row[R_SND][q] = snd;
+    S.row[R_SND][q] = 0.5 * st.dt * snd;
     double sh, ch;
     sincos_near(0.5 * st.dt * (res * irc - st.pl.vy), sh, ch);
     S.row[R_CH][q] = ch;
@@ -299,7 +299,7 @@ __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const 
       const int j = min(j0 + wid * M.P + pw, nphi - 1);
       const double cy = T.cyc[j], sy = T.syc[j];
       L.sp = THREED ? T.szc[k + NPAD] : 1.0;
-      L.isp2 = THREED ? 1.0 / (L.sp * L.sp) : 1.0;
+      L.isp2 = THREED ? rcp(L.sp * L.sp) : 1.0;
       L.c0 = fma(cy, pl.cy, sy * pl.sy) * L.sp;
       L.s0 = fma(sy, pl.cy, -(cy * pl.sy)) * L.sp;
     }
@@ -316,7 +316,7 @@ __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const 
       if (EOS == 0 && !P.p0) {
         double snd[C];
         ld_row<C>(L, R_SND, snd);
-        PG_CELLS cs[c] = 0.5 * st.dt * snd[c] * cs[c];
+        PG_CELLS cs[c] = snd[c] * cs[c];
       } else {
         double p[C], r[C];
         get<C>(L, W_P, p);
@@ -404,53 +404,54 @@ __global__ void __launch_bounds__(NT, MINB) k_sweep_x(Tables T, PlanesT<RT> P, P
 // Values are those that the separate kernels (k_damp, k_cfl) form.
 template <class RT>
 struct Finish {
-  double f, tr, tu, tv;                  // damping factor (0: none) and targets
-  double cs, irdx, off, irc, iwz;        // sound speed (EOS 0), 1/dr, frame offset, 1/r_cyl, 1/(r dtheta)
+  RingOut o;
+  double tr, tu, tv;                     // damping targets
   double bs, bv, cs2;
-  int rot;                               // rot_j after the step's shift
-  __device__ __forceinline__ void ring(const Tables &T, const SweepCtl &ctl, int rk, int row, int kz, int rot_new) {
+  template <bool POLAR>
+  __device__ __forceinline__ void ring(const Tables &T, const SweepCtl &ctl, int rk) {
     bs = sizeof(RT) == 4 ? T.sbg[rk] : 0.0;
     bv = sizeof(RT) == 4 ? T.vbg[rk] : 0.0;
-    f = 0.0;
-    if (!ctl.fuse) return;
-    const double2 t = T.fin[rk];
-    f = t.x;
-    off = t.y;
-    if (f > 0.0) {
+    o.shift = make_int2(0, 0);
+    if (!ctl.fuse) {
+      if (ctl.shift) o.shift = T.ro[rk].shift;
+      if (POLAR) {
+        o.rc = T.ro[rk].rc;
+        o.irc = T.ro[rk].irc;
+      }
+      return;
+    }
+    o = T.ro[rk];
+    if (o.f > 0.0) {
       tr = T.val_r[rk]; tu = T.val_u[rk]; tv = T.val_v[rk];
     }
     cs2 = T.cs2[rk];
-    cs = T.snd[rk];
-    irdx = T.irdx[row];
-    irc = T.irc[rk];
-    iwz = kz >= 0 ? T.idz[kz] * T.irxc[row] : 0.0;
-    rot = rot_new;
   }
-  // stores the cell at offset o (azimuth column jo) and returns its CFL rate
+  __device__ __forceinline__ int shift(const SweepCtl &ctl) const { return ctl.shift ? o.shift.x : 0; }
+  // stores the cell at offset at (azimuth column jo) and returns its CFL rate
   template <bool THREED, int EOS>
-  __device__ __forceinline__ double cell(const Tables &T, const PlanesT<RT> &P, const SweepCtl &ctl, const Phys &ph, size_t o,
+  __device__ __forceinline__ double cell(const Tables &T, const PlanesT<RT> &P, const SweepCtl &ctl, const Phys &ph, size_t at,
                                          int jo, double r, double u, double v, double w, bool &bad) const {
     RT sr = store_r<RT>(r, bs), su = (RT)u, sv = store_r<RT>(v, bv), sw = (RT)w;
     double rate = 0.0;
     if (ctl.fuse) {
-      if (f > 0.0) {
-        sr = store_r<RT>(damped(load_r(sr, bs), tr, f), bs);
-        su = (RT)damped((double)su, tu, f);
-        sv = store_r<RT>(damped(load_r(sv, bv), tv, f), bv);
-        if (THREED) sw = (RT)damped((double)sw, 0.0, f);
+      if (o.f > 0.0) {
+        sr = store_r<RT>(damped(load_r(sr, bs), tr, o.f), bs);
+        su = (RT)damped((double)su, tu, o.f);
+        sv = store_r<RT>(damped(load_r(sv, bv), tv, o.f), bv);
+        if (THREED) sw = (RT)damped((double)sw, 0.0, o.f);
       }
       r = load_r(sr, bs);
       v = load_r(sv, bv);
       if (!ctl.nocfl) {
-        const double a = EOS == 0 ? cs : sound_speed(r, eos_p<EOS>(r, cs2, ph), ph);
-        int js = jo - rot;
+        const double a = EOS == 0 ? o.cs : sound_speed(r, eos_p<EOS>(r, cs2, ph), ph);
+        int js = jo - o.shift.y;
         if (js < 0) js += T.nphi;
-        rate = cfl_rate<THREED>(a, (double)su, irdx, v - off, T.idy[js] * irc, (double)sw, iwz);
+        rate = cfl_rate<THREED>(a, (double)su, o.irdx, v - o.off, T.idy[js] * o.irc, (double)sw, o.iwz);
       }
       if (!(r > 0.0) || !isfinite(r) || !isfinite((double)su) || !isfinite(v)) bad = true;
     }
-    P.ro[o] = sr; P.uo[o] = su; P.vo[o] = sv;
-    if (THREED) P.wo[o] = sw;
+    P.ro[at] = sr; P.uo[at] = su; P.vo[at] = sv;
+    if (THREED) P.wo[at] = sw;
     return rate;
   }
 };
@@ -504,10 +505,9 @@ __device__ __forceinline__ void sweep_y_task(double *ws, const PlanetC &SP, cons
     // only move with the ring's rotation
     const int k = ring / T.nr, row = ring % T.nr + NPAD, rk = k * nrg + row;
     const size_t base = (size_t)rk * nphi;
-    const int2 sh = T.shift[rk];
-    const int inc = ctl.shift ? sh.x : 0;
     Finish<RT> F;
-    F.ring(T, ctl, rk, row, THREED ? k + NPAD : -1, sh.y);
+    F.template ring<false>(T, ctl, rk);
+    const int inc = F.shift(ctl);
     double rate = 0.0;
     bool bad = false;
 #pragma unroll 1
@@ -545,7 +545,8 @@ __device__ __forceinline__ void sweep_y_task(double *ws, const PlanetC &SP, cons
     L.rad = T.radc[rk];
     L.irad = T.irc[rk];
     L.sp = THREED ? T.szc[k + NPAD] : 1.0;
-    L.vr = T.res_v[rk] * L.irad;
+    const double res = T.res_v[rk];
+    L.vr = res * L.irad;
     L.cs2 = T.cs2[rk];
     const double snd = T.snd[rk], rs = T.rxc[row];
     in_flight();
@@ -554,10 +555,9 @@ __device__ __forceinline__ void sweep_y_task(double *ws, const PlanetC &SP, cons
     const PlanetC pl = SP;
     {
       L.bq = fma(rs, rs, pl.b2);         // the planet's distance sees the spherical radius in 3D
-      const double a = 0.5 * st.dt * (L.vr - pl.vy);
-      double s, c;
       L.ca = pl.cy; L.sa = -pl.sy;
-      sincos_near(a, s, c);
+      double c, s;
+      sincos_near(0.5 * st.dt * (L.vr - pl.vy), s, c);
       L.cb = fma(L.ca, c, -(L.sa * s)); L.sb = fma(L.sa, c, L.ca * s);
       L.cc = fma(L.cb, c, -(L.sb * s)); L.sc = fma(L.sb, c, L.cb * s);
     }
@@ -625,11 +625,10 @@ __device__ __forceinline__ void sweep_y_task(double *ws, const PlanetC &SP, cons
   for (int b = 0; b < M.P && ring + b < rings; b++) {
     const int q = ring + b, k = quot40(q, T.nr, T.mnr), row = q - k * T.nr + NPAD, rk = k * nrg + row;
     const size_t base = (size_t)rk * nphi;
-    const int2 sh = T.shift[rk];
-    const int im = ctl.shift ? sh.x : 0;
     const ColMap cm(M, b);
     Finish<RT> F;
-    F.ring(T, ctl, rk, row, THREED ? k + NPAD : -1, sh.y);
+    F.template ring<false>(T, ctl, rk);
+    const int im = F.shift(ctl);
 #pragma unroll 1
     for (int m = lane; m < len; m += 32) {
       const int s = cm.at<C>(m + NPAD);
@@ -683,7 +682,7 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
       const int k = REAL * l + e / NW, j = j0 + e % NW;
       if (k >= nk || j >= nphi) continue;
       const int rk = k * nrg + row;
-      int jo = j + (ctl.shift ? T.shift[rk].x : 0);
+      int jo = j + (ctl.shift ? T.ro[rk].shift.x : 0);
       if (jo >= nphi) jo -= nphi;
       const size_t s = (size_t)rk * nphi + j, o = (size_t)rk * nphi + jo;
       P.ro[o] = P.r[s]; P.uo[o] = P.u[s]; P.vo[o] = P.v[s]; P.wo[o] = P.w[s];
@@ -716,7 +715,8 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
       bv[i4] = sizeof(RT) == 4 ? T.vbg[rk] : 0.0;
     }
   }
-  double snd = 0.0, nu = 0.0, om = 0.0;  // of row tid: sound speed (a fixed layer: its square over gamma), viscosity, residual rotation
+  double snd = 0.0, nu = 0.0;            // of row tid: sound speed (a fixed layer: its square over gamma), viscosity
+  double2 turn = make_double2(0.0, 0.0);
   bool fixed = false;
   if (tid < rows) {
     const int kr = min(k0 + tid, nk + NPAD - 1);
@@ -724,7 +724,9 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
     const int km = kr >= nk ? 2 * nk - 1 - kr : kr, rk = km * nrg + row;
     const int gq = (kr < 0 ? kr + NPAD : kr - nk + NPAD) * T.nr + i;
     snd = fixed ? T.csg[gq] : T.snd[rk];
-    om = fixed ? 0.0 : T.res_v[rk] * T.irc[rk];
+    turn = !ctl.clk ? turn_call(st.dt, fixed ? 0.0 : T.res_v[rk], fixed ? 0.0 : T.irc[rk], st.pl.vy)
+           : fixed  ? ctl.clk->pc.turn
+                    : T.turn[rk];
     nu = (kr >= 0 && kr < nk) ? T.nu[rk] : T.nug[gq];
   }
   planet_shm<true>(S.pl, ctl, st, ph);
@@ -732,11 +734,9 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
   if (!run) return;
   if (tid < rows) {
     const int q = table_pos(tid, C, M.G);
-    double sh, ch;
-    sincos_near(0.5 * st.dt * (om - st.pl.vy), sh, ch);
     S.row[R_SND][q] = fixed ? sqrt(ph.gam * snd) : snd;
-    S.row[R_CH][q] = ch;
-    S.row[R_SH][q] = sh;
+    S.row[R_CH][q] = turn.x;
+    S.row[R_SH][q] = turn.y;
     S.row[R_NU][q] = nu;
   }
 #pragma unroll
@@ -828,14 +828,12 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
 #pragma unroll 2
     for (int m = W.n; m < len; m += M.step) {
       const int k = k0 + m + NPAD, rk = k * nrg + row, s = cm.at<C>(m + NPAD);
-      const int2 sh = T.shift[rk];
-      const double rc = T.radc[rk];
       Finish<RT> F;
-      F.ring(T, ctl, rk, row, k + NPAD, sh.y);
-      int jo = j0 + W.cl + (ctl.shift ? sh.x : 0);
+      F.template ring<true>(T, ctl, rk);
+      int jo = j0 + W.cl + F.shift(ctl);
       if (jo >= nphi) jo -= nphi;
       const double x = F.template cell<true, EOS>(T, P, ctl, ph, (size_t)rk * nphi + jo, jo, cw[W_R * SLOT + s],
-                                                  cw[W_V * SLOT + s], quot(cw[W_W * SLOT + s], rc, T.irc[rk]),
+                                                  cw[W_V * SLOT + s], quot(cw[W_W * SLOT + s], F.o.rc, F.o.irc),
                                                   cw[W_U * SLOT + s], bad);
       rate = (x > rate || x != x) ? x : rate;
     }

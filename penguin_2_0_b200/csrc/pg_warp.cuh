@@ -54,8 +54,8 @@ namespace pgd {
 
 // Series coefficients as operands from the constant bank: as immediates each
 // takes two moves before its use.
-__constant__ double kSin[5] = {-1.0 / 39916800.0, 1.0 / 362880.0, -1.0 / 5040.0, 1.0 / 120.0, -1.0 / 6.0};
-__constant__ double kCos[4] = {-1.0 / 3628800.0, 1.0 / 40320.0, -1.0 / 720.0, 1.0 / 24.0};
+__constant__ double kSin[4] = {1.0 / 362880.0, -1.0 / 5040.0, 1.0 / 120.0, -1.0 / 6.0};
+__constant__ double kCos[3] = {1.0 / 40320.0, -1.0 / 720.0, 1.0 / 24.0};
 __constant__ double kLog[8] = {1.0 / 17.0, 1.0 / 15.0, 1.0 / 13.0, 1.0 / 11.0, 1.0 / 9.0, 1.0 / 7.0, 1.0 / 5.0, 1.0 / 3.0};
 __constant__ double kExp[8] = {1.0 / 3628800.0, 1.0 / 362880.0, 1.0 / 40320.0, 1.0 / 5040.0,
                                1.0 / 720.0,     1.0 / 120.0,    1.0 / 24.0,    1.0 / 6.0};
@@ -88,9 +88,9 @@ __device__ __forceinline__ double quot(double a, double b, double ib) {
   return fma(fma(-q, b, a), ib, q);
 }
 
-// sin(x) = x q(x^2) and cos(x) for the small angles of a step.  Taylor to
-// x^11 and x^10: for |x| <= 0.2 the first omitted terms are below 1e-18
-// relative.  Larger angles take sincos.
+// sin(x) and cos(x) for the small angles of a step (fractions of a cell).
+// Taylor to x^9 and x^8: for |x| <= 0.05 the first omitted terms are below 1e-19
+// of sin's x and of cos's 1.  Larger angles take sincos.
 static __device__ __noinline__ double2 sincos_call(double x) {
   double s, c;
   sincos(x, &s, &c);
@@ -98,17 +98,9 @@ static __device__ __noinline__ double2 sincos_call(double x) {
 }
 __device__ __forceinline__ void sincos_near(double x, double &s, double &c) {
   const double z = x * x;
-  double q = fma(z, kSin[0], kSin[1]);
-  q = fma(z, q, kSin[2]);
-  q = fma(z, q, kSin[3]);
-  q = fma(z, q, kSin[4]);
-  s = fma(x * z, q, x);
-  double k = fma(z, kCos[0], kCos[1]);
-  k = fma(z, k, kCos[2]);
-  k = fma(z, k, kCos[3]);
-  k = fma(z, k, -0.5);
-  c = fma(z, k, 1.0);
-  if (fabs(x) > 0.2) {
+  s = fma(x * z, fma(z, fma(z, fma(z, kSin[0], kSin[1]), kSin[2]), kSin[3]), x);
+  c = fma(z, fma(z, fma(z, fma(z, kCos[0], kCos[1]), kCos[2]), -0.5), 1.0);
+  if (fabs(x) > 0.05) {
     const double2 t = sincos_call(x);
     s = t.x;
     c = t.y;
@@ -117,13 +109,9 @@ __device__ __forceinline__ void sincos_near(double x, double &s, double &c) {
 
 // sin(x) / x of such an angle
 __device__ __forceinline__ double sinc_near(double x) {
-  if (fabs(x) > 0.2) return sincos_call(x).x / x;
+  if (fabs(x) > 0.05) return sincos_call(x).x / x;
   const double z = x * x;
-  double q = fma(z, kSin[0], kSin[1]);
-  q = fma(z, q, kSin[2]);
-  q = fma(z, q, kSin[3]);
-  q = fma(z, q, kSin[4]);
-  return fma(z, q, 1.0);
+  return fma(z, fma(z, fma(z, fma(z, kSin[0], kSin[1]), kSin[2]), kSin[3]), 1.0);
 }
 static __device__ __noinline__ double pow_call(double x, double y) { return pow(x, y); }
 
@@ -157,7 +145,18 @@ __device__ __forceinline__ void right_of(const double (&a)[C], double (&o)[C]) {
   PG_CELLS o[c] = c < C - 1 ? a[c < C - 1 ? c + 1 : 0] : r;
 }
 
-__device__ __forceinline__ PlanetC planet_consts(const Body &b, bool three, bool plnt) {
+// cos and sin of the planet's angle's change against a ring in half a step
+// (res_v and 1/r_cyl of the ring)
+__device__ __forceinline__ double2 turn_of(double dt, double res, double irc, double vy) {
+  double2 t;
+  sincos_near(0.5 * dt * (res * irc - vy), t.y, t.x);
+  return t;
+}
+static __device__ __noinline__ double2 turn_call(double dt, double res, double irc, double vy) {
+  return turn_of(dt, res, irc, vy);
+}
+
+__device__ __forceinline__ PlanetC planet_consts(const Body &b, bool three, bool plnt, double dt) {
   PlanetC p;
   const double stm = three ? 1.0 / (1.0 + b.m) : 1.0;
   p.m = b.m * stm;
@@ -168,6 +167,7 @@ __device__ __forceinline__ PlanetC planet_consts(const Body &b, bool three, bool
   p.y = b.y;
   p.vy = b.vy;
   sincos(b.y, &p.sy, &p.cy);
+  p.turn = three ? turn_of(dt, 0.0, 0.0, b.vy) : make_double2(1.0, 0.0);
   return p;
 }
 
