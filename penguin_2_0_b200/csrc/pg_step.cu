@@ -242,7 +242,8 @@ __device__ double d_set_M_p(const DevClock &c, double t) {
 }
 __device__ void d_kick(Body &pl, double &FrRot, double dt, int frflag) {
   pl.vx += dt * pl.fx;
-  pl.vy += FrRot + dt * pl.fy / pl.x / pl.x;
+  // without a force (fixed planet) the quotients are the same zero
+  pl.vy += FrRot + (pl.fy == 0.0 && pl.x > 0.0 ? dt * pl.fy : dt * pl.fy / pl.x / pl.x);
   FrRot = (frflag == 1) ? pl.vy : 0.0;
   pl.vy -= FrRot;
 }
@@ -281,9 +282,9 @@ __device__ void d_forces_fixed(Body &pl, double FrRot) {
 }
 
 // ---------------------------------------------------------------------------
-// The scalar parts of a step, on a CTA's copy of the clock.
-// End of a step (main.cu:378-412) with a fixed planet; with a moving one in
-// two parts around the disk's force sums (planet.cu:54-93).
+// The scalar parts of a step, on a CTA's copy of the clock: its end
+// (main.cu:378-412) with a moving planet, in two parts around the disk's force
+// sums (planet.cu:54-93); with a fixed one see step_scalars.
 __device__ __forceinline__ void step_time(DevClock &c) {
   c.simtime += c.dt_step;
   c.timem += c.dt_step;
@@ -299,51 +300,6 @@ __device__ __forceinline__ void step_books(DevClock &c) {
     c.halted = 1;   // the host dumps before continuing
   }
   if (c.done) c.halted = 1;
-}
-__device__ __forceinline__ void step_post(DevClock &c) {
-  step_time(c);
-  if (c.plnt_flag > 0) {
-    d_drift(c.planet, c.frrot, c.dt_step, c);
-    c.planet.m = d_set_M_p(c, c.simtime);
-    d_forces_fixed(c.planet, c.frrot);
-    d_kick(c.planet, c.frrot, 0.5 * c.dt_step, c.frrot_flag);
-  }
-  step_books(c);
-}
-// get_dt's host part, the dt clipping and the half kick (main.cu:345-370).
-// False: the run has halted.  frrot: FrRot before the kick, as Index_Shift sees it.
-__device__ __forceinline__ bool step_pre(DevClock &c, double &frrot) {
-  if (c.halted || c.done) return false;
-  if (c.status != 0) { c.halted = 1; return false; }
-  const double rate = __longlong_as_double((long long)c.cfl_bits);
-  const double hdt = c.courant / rate;         // dt_lv3 timestep.cu:105
-  double dt = 1.1 * c.dt;                      // timestep.cu:135-141
-  dt = (hdt < dt) ? hdt : dt;
-  if (dt / c.endtime < 1.0e-12 || !(dt > 0.0)) { c.status = 4; c.halted = 1; return false; }
-  c.prin = 0;
-  if (c.ncycle == c.ncycend) { c.prin = 1; c.done = 1; }
-  if (c.simtime + dt >= c.endtime) {
-    c.old_dt = dt; dt = c.endtime - c.simtime; c.prin = 1; c.make_pict = 1; c.done = 1;
-  }
-  if (c.timem + dt >= c.tmovie) { c.old_dt = dt; dt = c.tmovie - c.timem; c.make_pict = 1; }
-  c.dt = dt;
-  c.dt_step = dt;
-  frrot = c.frrot;
-  // kick_drift_kick(planet, FrRot, ..., 0.5*dt, true) main.cu:370
-  if (c.plnt_flag > 0) d_kick(c.planet, c.frrot, 0.5 * dt, c.frrot_flag);
-  // FrRot at the next get_dt, for the fused CFL: replay drift, forces and kick
-  // on copies (fixed planet: forces are analytic)
-  Body b = c.planet;
-  double fr = c.frrot;
-  if (c.plnt_flag > 0) {
-    d_drift(b, fr, dt, c);
-    d_forces_fixed(b, fr);
-    d_kick(b, fr, 0.5 * dt, c.frrot_flag);
-  }
-  c.frrot_next = fr;
-  c.cfl_bits = 0ull;
-  c.pc = planet_consts(c.planet, c.ndim == 3, c.plnt_flag > 0, dt);
-  return true;
 }
 
 // a diagnostics row (main.cu:414-428) of the finished step's planet and time
@@ -382,6 +338,152 @@ __device__ __forceinline__ void clock_out(StepShm &S, DevClock *clk) {
     reinterpret_cast<unsigned long long *>(clk)[threadIdx.x] = reinterpret_cast<const unsigned long long *>(&S.c)[threadIdx.x];
 }
 
+// drift's new place of the planet (planet.cu:54-60)
+__device__ __forceinline__ double drift_y(const Body &p, double dt) {
+  double y = p.y + dt * p.vy;
+  if (y < 0.0) y += 6.283185307179586476925286766559;
+  if (y >= 6.283185307179586476925286766559) y -= 6.283185307179586476925286766559;
+  return y;
+}
+// The end of a step with a fixed planet (post; main.cu:378-412: time, drift,
+// forces, kick, books) and the start of the next (BETWEEN_PRE; get_dt's host
+// part, the dt clipping and the half kick, main.cu:345-370), by a whole warp:
+// the divisions that do not wait for one another are done side by side, a lane
+// each, so that the chain has four of them one after another instead of
+// seventeen at some 200 cycles each.  The planet's cos and sin come from
+// another warp.  Every operation is the scalar code's, so are the bits.
+__device__ __forceinline__ void step_scalars(StepShm &S, int fl, bool post) {
+  DevClock &c = S.c;
+  const int lane = threadIdx.x & 31;
+  const bool pln = c.plnt_flag > 0;
+  const double ds = c.dt_step, courant = c.courant, endtime = c.endtime, tmovie = c.tmovie;
+  Body p = c.planet;
+  double fr = c.frrot, simtime = c.simtime, timem = c.timem, cdt = c.dt, old_dt = c.old_dt;
+  long long ncycle = c.ncycle, ncycp = c.ncycp;
+  int prin = c.prin, make_pict = c.make_pict, done = c.done, halted = c.halted, status = c.status;
+  double x1 = p.x, y1 = p.y;
+  if (post) {
+    simtime += ds;
+    timem += ds;
+    ncycle += 1;
+    ncycp += 1;
+    if (pln) {
+      x1 = p.x + ds * p.vx;
+      y1 = drift_y(p, ds);
+      p.m = d_set_M_p(c, simtime);
+    }
+  }
+  double n = 1.0, d1 = 1.0, d2 = 1.0;
+  if (lane == 0) { n = (p.vy + fr) * p.x * p.x; d1 = d2 = x1; }             // drift's v_phi
+  if (lane == 1) { n = -1.0; d1 = d2 = x1; }                                // the star's pull
+  if (lane == 2) { n = courant; d1 = __longlong_as_double((long long)c.cfl_bits); }   // dt_lv3 timestep.cu:105
+  if (lane == 3) d1 = x1 * x1;
+  if (lane == 4 && c.ndim == 3) d1 = 1.0 + p.m;
+  double q = n / d1 / d2;
+  const double hdt = __shfl_sync(0xffffffffu, q, 2), ix2 = __shfl_sync(0xffffffffu, q, 3), stm = __shfl_sync(0xffffffffu, q, 4);
+  {
+    const double v = __shfl_sync(0xffffffffu, q, 0), g = __shfl_sync(0xffffffffu, q, 1);
+    if (post && pln) {
+      p.x = x1;
+      p.y = y1;
+      p.vy = v - fr;
+      p.fx = g + p.x * pow_host_form(p.vy + fr, 2.0);
+      p.fy = 0.0;
+      d_kick(p, fr, 0.5 * ds, c.frrot_flag);
+    }
+  }
+  if (post) {                              // step_books
+    if (ncycp == c.nprin) { ncycp = 0; prin = 1; }
+    if (make_pict) {
+      timem = 0.0;
+      make_pict = 0;
+      cdt = old_dt;
+      halted = 1;
+    }
+    if (done) halted = 1;
+  }
+  const bool print = (fl & BETWEEN_DIAG) && prin;
+  if (print) prin = 0;
+  if (print && lane == 0) {
+    S.planet = p;
+    S.frrot = fr;
+    S.simtime = simtime;
+  }
+  bool run = (fl & BETWEEN_PRE) && !halted && !done;
+  if (run && status != 0) {
+    halted = 1;
+    run = false;
+  }
+  double dt = 1.1 * cdt;                   // timestep.cu:135-141
+  dt = (hdt < dt) ? hdt : dt;
+  const double dt0 = dt;
+  bool last = false, out = false;
+  if (ncycle == c.ncycend) last = true;
+  double od = old_dt;
+  bool end = false, pict = false;
+  if (simtime + dt >= endtime) { od = dt; dt = endtime - simtime; end = pict = true; }
+  if (timem + dt >= tmovie) { od = dt; dt = tmovie - timem; pict = true; }
+  out = last || end;
+  // kick_drift_kick(planet, FrRot, ..., 0.5*dt, true) main.cu:370
+  Body k = p;
+  double fk = fr;
+  if (pln) d_kick(k, fk, 0.5 * dt, c.frrot_flag);
+  // FrRot at the next get_dt, for the fused CFL: drift and kick replayed on
+  // copies (fixed planet: its forces are analytic and leave v_phi alone)
+  n = 1.0; d1 = 1.0; d2 = 1.0;
+  if (lane == 0) { n = (k.vy + fk) * k.x * k.x; d1 = d2 = k.x + dt * k.vx; }
+  if (lane == 1) { n = dt0; d1 = endtime; }
+  q = n / d1 / d2;
+  double frn = fk;
+  {
+    const double v = __shfl_sync(0xffffffffu, q, 0), rel = __shfl_sync(0xffffffffu, q, 1);
+    if (pln) frn = c.frrot_flag == 1 ? (v - fk) + (fk + 0.0) : 0.0;
+    if (run && (rel < 1.0e-12 || !(dt0 > 0.0))) {
+      status = 4;
+      halted = 1;
+      run = false;
+    }
+  }
+  if (lane == 0) {
+    c.simtime = simtime;
+    c.timem = timem;
+    c.ncycle = ncycle;
+    c.ncycp = ncycp;
+    c.halted = halted;
+    c.status = status;
+    S.print = print;
+    S.run = run;
+    if (run) {
+      S.frrot_pre = fr;                    // as Index_Shift sees it
+      c.prin = out;
+      if (out) done = 1;
+      if (pict) make_pict = 1;
+      c.old_dt = od;
+      c.dt = c.dt_step = dt;
+      c.planet = k;
+      c.frrot = fk;
+      c.frrot_next = frn;
+      c.cfl_bits = 0ull;
+      PlanetC &e = c.pc;                   // planet_consts; cy, sy: between_body
+      e.m = k.m * stm;
+      e.x = k.x;
+      e.ix2 = ix2;
+      e.b2 = fma(k.x, k.x, k.rs * k.rs);
+      e.star = pln ? stm : 1.0;
+      e.y = k.y;
+      e.vy = k.vy;
+      e.turn = c.ndim == 3 ? turn_of(dt, 0.0, 0.0, k.vy) : make_double2(1.0, 0.0);
+    } else {
+      c.prin = prin;
+      c.dt = cdt;
+      c.planet = p;
+      c.frrot = fr;
+    }
+    c.done = done;
+    c.make_pict = make_pict;
+  }
+}
+
 // CTA b of a run's nb.  fl: BETWEEN_POST the end of a step with a fixed planet,
 // BETWEEN_DIAG its diagnostics, BETWEEN_PRE the start of the next.
 template <class RT>
@@ -393,19 +495,16 @@ __device__ __forceinline__ void between_body(StepShm &S, const Tables &T, const 
   const bool off = S.c.halted && !(fl & BETWEEN_DIAG && S.c.prin);
   if (off) return;                       // every CTA of the run alike
   const bool post = (fl & BETWEEN_POST) && !S.c.halted;
+  const double py = post && S.c.plnt_flag > 0 ? drift_y(S.c.planet, S.c.dt_step) : S.c.planet.y;
+  double sy = 0.0, cy = 1.0;
   __syncthreads();
-  if (tid == 0) {
-    if (post) step_post(S.c);
-    S.print = (fl & BETWEEN_DIAG) && S.c.prin;
-    if (S.print) {
-      S.c.prin = 0;
-      S.planet = S.c.planet;
-      S.frrot = S.c.frrot;
-      S.simtime = S.c.simtime;
-    }
-    S.run = (fl & BETWEEN_PRE) && step_pre(S.c, S.frrot_pre);
+  if (tid < 32) step_scalars(S, fl, post);
+  else if (tid == 32) sincos(py, &sy, &cy);
+  __syncthreads();
+  if (tid == 32 && S.run) {
+    S.c.pc.sy = sy;
+    S.c.pc.cy = cy;
   }
-  __syncthreads();
   if (S.print) {
     const RingForce F(S.planet, 0.0, p_alpha);
     for (int rt = b; rt < rings; rt += nb) {
