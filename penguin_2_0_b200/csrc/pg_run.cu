@@ -123,10 +123,13 @@ static int fail(pg_run *run, int code, const std::string &msg) {
 
 // Device memory that dumps pass through on their way in and out.  One block
 // per device is kept while the device has runs, grown to the largest dump up to
-// kStageKeep; a larger dump, or a second one at the same time (another thread's
-// run), gets memory of its own for the call.  With a cudaMalloc and cudaFree in
-// each, the 256x768 disk's load took 1165 us and its save 1060; without, 337
-// and 283, which its host tables and PCIe (22 MB, some 400 us) account for.
+// kStageKeep (0.3 % of the GPU's memory); a larger dump, or a second one at the
+// same time (another thread's run), gets memory of its own for the call, and an
+// allocation that fails gives the idle block back and tries again.  With a
+// cudaMalloc and cudaFree in each, the 256x768 disk's load took 1165 us and its
+// save 1060; without, 337 and 283, which its host tables and PCIe (22 MB, some
+// 400 us) account for.  For the 302 MB dump of the 128x1024x32 disk such a free
+// now and then took half a second: jobs of 200 steps 0.22-1.8 s, without 0.212.
 struct DumpStage {
   std::mutex m;
   void *p = nullptr;
@@ -134,10 +137,20 @@ struct DumpStage {
   bool busy = false;
   int runs = 0;
 };
-static constexpr size_t kStageKeep = (size_t)64 << 20;
+static constexpr size_t kStageKeep = (size_t)512 << 20;
 static DumpStage &dump_stage(int dev) {
   static DumpStage d[64];
   return d[dev & 63];
+}
+// gives an idle block back; true if there was one
+static bool stage_drop(int dev) {
+  DumpStage &d = dump_stage(dev);
+  std::lock_guard<std::mutex> l(d.m);
+  if (d.busy || !d.p) return false;
+  cudaFree(d.p);
+  d.p = nullptr;
+  d.n = 0;
+  return true;
 }
 static void *stage_take(int dev, size_t bytes) {
   DumpStage &d = dump_stage(dev);
@@ -158,7 +171,8 @@ static void *stage_take(int dev, size_t bytes) {
     }
   }
   void *p = nullptr;
-  return cudaMalloc(&p, bytes) == cudaSuccess ? p : nullptr;
+  if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+  return stage_drop(dev) && cudaMalloc(&p, bytes) == cudaSuccess ? p : nullptr;
 }
 // after the work on it is complete
 static void stage_give(int dev, void *p) {
@@ -320,9 +334,15 @@ const char *pg_last_error(const pg_run *run) { return run ? run->err.c_str() : "
 
 int64_t pg_launch_count(const pg_run *run) { return run ? run->launches : 0; }
 
+static int create(const pg_params *p, int device, pg_run **out);
 int pg_create(const pg_params *p, int device, pg_run **out) {
   if (!p || !out) return PG_ERR_ARG;
   *out = nullptr;
+  int st = create(p, device, out);
+  if (st == PG_ERR_NOMEM && stage_drop(device)) st = create(p, device, out);
+  return st;
+}
+static int create(const pg_params *p, int device, pg_run **out) {
   std::string why;
   int st = pg::check_params(p, why);
   if (st) {
@@ -1160,7 +1180,8 @@ int pg_history(pg_run *run, double *rows, int max, int *rows_out) {
 // ---------------------------------------------------------------------------
 // post-processing of the current state (read/ tools)
 static int post_buffer(pg_run *run, size_t n, double **buf) {
-  if (cudaMalloc(buf, n * sizeof(double)) != cudaSuccess) return fail(run, PG_ERR_NOMEM, "post-processing buffer");
+  if (cudaMalloc(buf, n * sizeof(double)) == cudaSuccess) return PG_OK;
+  if (!stage_drop(run->dev) || cudaMalloc(buf, n * sizeof(double)) != cudaSuccess) return fail(run, PG_ERR_NOMEM, "post-processing buffer");
   return PG_OK;
 }
 

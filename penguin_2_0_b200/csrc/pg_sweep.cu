@@ -23,18 +23,22 @@
 // contiguous bytes.
 //
 // What bounds them and what they measured (B200, event-timed per sweep, FP64):
-// instruction issue at 2.1-2.3 of 4 per cycle and SM, FP64 pipe 40-45 %, DRAM
-// below 20 %.  Against one thread per cell, the chain through shared memory
-// and 22 CTA barriers per chunk:
-//   128x1024x32  radial 628 -> 284 us, azimuthal 554 -> 207, polar 698 -> 470
-//   1536x4608    radial 836 -> 369 us, azimuthal 906 -> 338
-//   256x768      radial  46 ->  22 us, azimuthal  37 ->  21
+// instruction issue (pg_warp.cuh) at 2.2-2.4 of 4 per cycle and SM, FP64 pipe
+// 43-51 %, DRAM below 15 %.  Against one thread per cell, the chain through
+// shared memory and 22 CTA barriers per chunk:
+//   128x1024x32  radial 628 -> 265 us, azimuthal 554 -> 194, polar 698 -> 423
+//   1536x4608    radial 836 -> 345 us, azimuthal 906 -> 311
+//   256x768      radial  46 ->  21 us, azimuthal  37 ->  21
+// Of the radial sweep's 162 M instructions on the 3D disk 26 M are the tile's
+// loads and stores and what they need, of the azimuthal one's 131 M 17 M, of
+// the polar one's 285 M some 55 M.
 // 4 warps per CTA, 4 CTAs per SM at 128 registers (some 100 bytes of spills):
-// 3 CTAs at 168 registers without spills ran 0-13 % longer, 2 CTAs at 230
-// registers 25-50 %; 8 warps per CTA 5 %, 16 warps 30 %.  Loading the tile in
-// one go before the first use took the radial sweep from 344 to 328 us, cutting
-// the workspace from 11 to 9 slots (which leaves L1 room for the axis tables)
-// from 308 to 284.
+// 3 CTAs ran 2-13 % longer but on the smallest grids, 5 CTAs 5-25 %, 8 warps per
+// CTA 5 %, 16 warps 30 %.  Loading the tile in one go before the first use took
+// the radial sweep from 344 to 328 us, cutting the workspace from 11 to 9 slots
+// (which leaves L1 room for the axis tables) from 308 to 284, planet constants
+// from the clock and quotients by multiplication (tiles formed on the host) to
+// 268.
 #include "pg_warp.cuh"
 
 namespace pgd {

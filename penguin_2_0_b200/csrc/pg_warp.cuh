@@ -9,15 +9,19 @@
 // value; between stages the fields rest in the warp's slots of shared memory
 // (each lane on its own cells, so without bank conflicts or barriers).
 //
-// What bounds it: instruction issue and the FP64 pipe.  The sweeps read and
-// write each field once (DRAM far from its limit), so what counts is the
-// number of instructions per cell, and that they come from the SM's
-// instruction cache: straight-line code of more than 2048 instructions
+// What bounds it: instruction issue.  The sweeps read and write each field once
+// (DRAM far from its limit).  Measured with 16 warps per SM: an FP64
+// instruction keeps a scheduler from issuing for two cycles, any other for one
+// (32 DFMA take 64 cycles, with 32 LOP3 between them 97), and with that the
+// sweeps run at 78-85 % of what their instructions allow.  So what counts is
+// the number of instructions per cell, FP64 ones twice, and that they come from
+// the SM's instruction cache: straight-line code of more than 2048 instructions
 // (32 KB) was measured to issue at 1.2-1.9 instructions per cycle and SM
 // against 3.85 below that, whatever the number of warps, and the chain with
 // every stage unrolled over 4 cells and all fields is 4700 instructions long.
-// So the stages that repeat per field (edges, fluxes) are loops over fields,
-// and the faces (forces, Riemann problem) a loop over pairs of cells.
+// So the stages that repeat per field (edges, fluxes) are loops over fields.
+// The faces (forces, Riemann problem) as a loop over pairs of cells as well were
+// 3 % slower: the moves that it takes cost more than the shorter code gains.
 // The number of operations is kept down by
 //   * edge values as differences from the cell value (edges below): the
 //     monotonicity rules of parabola.cu:70-133 become comparisons of the two
@@ -250,12 +254,10 @@ __device__ __forceinline__ void put(const Lane<C> &L, int slot, const double (&o
     PG_CELLS q[c * PIECE<C>] = o[c];
   }
 }
-// per-row values of a radial or polar tile (one ring of one layer per row):
-// before the chain those it reads, after it those of the polar epilogue
+// per-row values of a radial or polar tile (one ring of one layer per row)
 enum RowEntry {
   R_SND, R_CH, R_SH, R_NU, R_RC, R_IRC,   // R_CH, R_SH: cos and sin of the planet's angle's change in dt/2
-  R_F = 0, R_TR, R_TU, R_TV, R_OFF, R_IWZ, R_J,
-  R_COUNT = 7
+  R_COUNT
 };
 // the lane's entries of one array of the axis table, and of the per-row values
 template <int C>

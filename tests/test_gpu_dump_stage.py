@@ -20,8 +20,8 @@ def _fields(buf, p):
     return a[:, : 32 * p.jmax].copy().view(np.float64)
 
 
-# small, larger (the block grows), smaller again, above what is kept (64 MiB)
-@pytest.mark.parametrize("sizes", [[(64, 130), (200, 600), (64, 130)], [(480, 2000), (64, 130)]])
+# small, larger (the block grows), smaller again, above what is kept (512 MiB)
+@pytest.mark.parametrize("sizes", [[(64, 130), (200, 600), (64, 130)], [(1700, 4700), (64, 130)]])
 def test_a_dump_comes_back_as_it_went_in(sizes):
     for nr, nphi in sizes:
         p = _p(nr, nphi)
