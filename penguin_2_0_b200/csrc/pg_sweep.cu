@@ -917,6 +917,8 @@ static int groups(int n, int w) { return (n + w - 1) / w; }
 // warp's cell slots empty.  The 32-layer disk's pencils of 44 cells fill 88 of
 // 96 slots with 3 (two pencils of 15 lanes) and 88 of 128 with 4; 28 and 36
 // cells fill 112 and 108 of 128 with 4.  Grids of more than one chunk take 4.
+// Polar sweep with 3 and 4 cells, us: 128x1024x32 424, 578; 128x512 of 40 layers
+// 422, 305; 24: 223, 209; 20: 214, 150; 16: 152, 154; 12: 114, 127.
 int polar_cells(const Chunking &ch) {
   if (ch.loop > 1 || ch.stuck) return 4;
   const int lim = ch.lim_last;
