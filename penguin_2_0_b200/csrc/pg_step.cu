@@ -514,21 +514,18 @@ __device__ __forceinline__ void between_body(StepShm &S, const Tables &T, const 
       if (tid == 0) {
         part[rt] = m;
         part[rings + rt] = t;
-        T.rot_j[rk] = rot;
-        if (S.run) {
-          index_shift_ring(T, rt, S.c.dt_step, S.frrot_pre, fargo);
-          finish_ring(T, rt, S.c.dt_step, S.c.frrot_next, S.c.planet.vy, ndim);
-        }
       }
     }
-  } else {
-    for (int rt = b * ST + tid; rt < rings; rt += nb * ST) {
-      const int rk = rt / T.nr * T.nrg + rt % T.nr + NPAD;
-      if (post) T.rot_j[rk] = rotated(T, rk);
-      if (S.run) {
-        index_shift_ring(T, rt, S.c.dt_step, S.frrot_pre, fargo);
-        finish_ring(T, rt, S.c.dt_step, S.c.frrot_next, S.c.planet.vy, ndim);
-      }
+  }
+  // a thread per ring; in a step that sums the CTA's own rings, which it alone
+  // has read
+  const int first = S.print ? b + tid * nb : b * ST + tid, by = nb * ST;
+  for (int rt = first; rt < rings; rt += by) {
+    const int rk = rt / T.nr * T.nrg + rt % T.nr + NPAD;
+    if (post) T.rot_j[rk] = rotated(T, rk);
+    if (S.run) {
+      index_shift_ring(T, rt, S.c.dt_step, S.frrot_pre, fargo);
+      finish_ring(T, rt, S.c.dt_step, S.c.frrot_next, S.c.planet.vy, ndim);
     }
   }
   if (nb > 1 && !last_cta(counter, nb)) return;
@@ -616,10 +613,16 @@ __global__ void __launch_bounds__(ST) k_moving(Tables T, const RT *R, DevClock *
 namespace pgk {
 using namespace pgd;
 
-// Sums on every call (k_reduce, k_moving): a CTA per ring up to four per SM of
-// a B200, then each several.  Between steps, of which one in nprin sums: a
-// thread per ring, but enough CTAs that a summing step takes few rings each.
+// A CTA per ring up to four per SM of a B200, then each several: for the sums of
+// k_reduce and k_moving, and between steps, where a step that prints sums (one
+// in nprin) and one that does not takes as long with 16 CTAs as with 592.  With
+// a CTA per 8 rings, at most 148, and Index_Shift by the thread that stored the
+// sum, a printing step took, us: 128x384 54.6, now 35.1; 1536x4608 895, 776;
+// 128x1024x32 1019, 943 (without printing 30, 655 and 893 both ways).  k_reduce
+// with at most 296 and 1184 CTAs instead of 592: 1536x4608 torque 76 and 54 us
+// for 52.
 static int ring_ctas(int rings) { return rings < 592 ? rings : 592; }
+// of a batch member, whose fellows fill the GPU
 int between_ctas(int rings) {
   const int n = (rings + SWARPS - 1) / SWARPS;
   return n < 148 ? n : 148;
@@ -638,7 +641,7 @@ void reduce(const Tables &T, const RT *r, const Body &pl, double exclude, int mo
 template <class RT>
 void between(const Tables &T, const RT *r, DevClock *clk, double *part, unsigned *counter, double p_alpha, int fargo,
              int plnt, int ndim, int fl, cudaStream_t s) {
-  launch(k_between<RT>, between_ctas(T.nr * T.nk), ST, 0, s, T, r, clk, part, counter, p_alpha, fargo, plnt && ndim == 2, ndim, fl);
+  launch(k_between<RT>, ring_ctas(T.nr * T.nk), ST, 0, s, T, r, clk, part, counter, p_alpha, fargo, plnt && ndim == 2, ndim, fl);
 }
 template <class RT>
 void moving(const Tables &T, const RT *r, DevClock *clk, double *part, unsigned *counter, double p_alpha, int ndim,
