@@ -727,9 +727,14 @@ __device__ __forceinline__ void warp_chain(const Lane<C> &L, const PlanetC &P, c
       double a = dm * (pr[c] - pm[c]);
       if (AXIS != 1) a *= 0.5 * (vr[c] + vf[c]);
       u[c] = u[c] + fma(hdt, f1[c] + f2[c], -a);
-      m[c] = r[c] * vol[c];               // the cell's mass, which the Lagrangian step keeps
+      // the cell's mass, which the Lagrangian step keeps but for a density that
+      // the bound replaces (an emptied cell, or one whose faces crossed): there
+      // it is the bound's times the moved volume (evolve.cu:137, remap.cu:94-99)
+      m[c] = r[c] * vol[c];
       const double q = m[c] * rcp(dvol[c]);
-      r[c] = q > kSmallr ? q : kSmallr;
+      const bool held = q > kSmallr;
+      r[c] = held ? q : kSmallr;
+      m[c] = held ? m[c] : kSmallr * dvol[c];
     }
     put<C>(L, W_R, r);
     put<C>(L, W_U, u);
