@@ -770,8 +770,13 @@ __device__ __forceinline__ void warp_chain(const Lane<C> &L, const PlanetC &P, c
       e[c] = 0.5 * del[c] * rcp(del[c] >= 0.0 ? xm[c] : dx[c]);
     }
   }
-  double im[C], mf[C];                    // 1 / mass after the remap (per dvol's unit, as m); mass flux
-  PG_CELLS mf[c] = lvol[c];
+  // 1 / mass after the remap (per dvol's unit, as m), whose sign says which way
+  // the left face moved: e's own turns around with a crossed donor's width; mass flux
+  double im[C], mf[C];
+  PG_CELLS {
+    im[c] = del[c];
+    mf[c] = lvol[c];
+  }
   // 2D leaves out the slot that stays zero: w of the radial sweep, v of the
   // azimuthal one
   constexpr int NF = THREED ? 4 : 3;
@@ -785,7 +790,7 @@ __device__ __forceinline__ void warp_chain(const Lane<C> &L, const PlanetC &P, c
     left_of<C>(d1, l1);
     left_of<C>(d2, l2);
     PG_CELLS {
-      const bool up = __double2hiint(e[c]) >= 0;
+      const bool up = __double2hiint(im[c]) >= 0;
       const double q = up ? al[c] : a[c], x1 = up ? l1[c] : d1[c], x2 = up ? l2[c] : d2[c];
       // t = edge - e (da - s a6), s = 1 - 4/3 e from the left cell, -(1 + 4/3 e) from the right one
       const double s3 = fma(-4.0, e[c], up ? 3.0 : -3.0);
@@ -801,12 +806,12 @@ __device__ __forceinline__ void warp_chain(const Lane<C> &L, const PlanetC &P, c
         double q = quot(m[c] + fl[c] - fr[c], vol[c], ivol[c]);
         q = q > kSmallr ? q : kSmallr;
         a[c] = L.in(c, NPAD, NPAD) ? q : a[c];
-        im[c] = rcp(a[c] * vol[c]);
+        im[c] = copysign(rcp(a[c] * vol[c]), im[c]);
         mf[c] = fl[c];
       }
     } else {
       PG_CELLS {
-        const double q = fma(a[c], m[c], fl[c] - fr[c]) * im[c];
+        const double q = fma(a[c], m[c], fl[c] - fr[c]) * fabs(im[c]);
         a[c] = L.in(c, NPAD, NPAD) ? q : a[c];
       }
     }
