@@ -327,7 +327,7 @@ __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const 
         get<C>(L, W_R, r);
         PG_CELLS {
           const double x = ph.gam * p[c] * rcp(r[c]);
-          cs[c] = 0.5 * st.dt * (x * rsq(x)) * cs[c];
+          cs[c] = 0.5 * st.dt * root(x) * cs[c];
         }
       }
       warp_chain<0, THREED, EOS, C>(L, pl, ph, cs);
@@ -592,7 +592,7 @@ __device__ __forceinline__ void sweep_y_task(double *ws, const PlanetC &SP, cons
         PG_CELLS {
           p[c] = L.cs2 * pow_call(r[c], ph.gam) / ph.gam;
           const double x2 = ph.gam * p[c] * rcp(r[c]);
-          cs[c] *= 0.5 * st.dt * (x2 * rsq(x2)) * L.irad;
+          cs[c] *= 0.5 * st.dt * root(x2) * L.irad;
         }
         put<C>(L, W_P, p);
       }
@@ -796,7 +796,7 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
         get<C>(L, W_R, r);
         PG_CELLS {
           const double x = ph.gam * p[c] * rcp(r[c]);
-          cs[c] = a * (x * rsq(x)) * cs[c];
+          cs[c] = a * root(x) * cs[c];
         }
       }
       warp_chain<2, true, EOS, C>(L, pl, ph, cs);

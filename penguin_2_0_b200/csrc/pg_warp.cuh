@@ -82,6 +82,12 @@ __device__ __forceinline__ double rsq(double x) {
   const double e = fma(-(x * y), y, 1.0);
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
+// sqrt(x) by rsq where x is positive and normal, else (zero, as where a dump holds
+// no pressure) by CUDA's, out of line
+static __device__ __noinline__ double sqrt_call(double x) { return sqrt(x); }
+__device__ __forceinline__ double root(double x) {
+  return (unsigned)(__double2hiint(x) - 0x00100000) < 0x7fe00000u ? x * rsq(x) : sqrt_call(x);
+}
 
 // a / b from ib = 1 / b to rounding: the quotient corrected by its remainder
 // (Markstein).  Where the same b divides step after step (a cell's volume, a
