@@ -279,6 +279,7 @@ int pg_batch_advance(pg_batch *b, int nsteps, int chunk) {
   if (b->runs.empty() || nsteps == 0) return PG_OK;
   if (b->dirty)
     if (int e = rebuild(b)) return e;
+  for (pg_run *r : b->runs) pgi::run_stepped(r);     // every member, replayed or queued, also where this call fails
   if (!b->solo.empty() && (chunk & 1)) chunk += 1;   // 3D steps alternate the plane copies
   int done = 0;
   // a 3D member with a freshly loaded dump reads its p0 plane in its first
@@ -342,7 +343,7 @@ int pg_batch_advance(pg_batch *b, int nsteps, int chunk) {
     b->launches += nk;
   }
   for (auto &g : b->g)
-    for (pg_run *r : g.members) pgi::run_batched(r, 0);
+    for (pg_run *r : g.members) pgi::run_batched(r);
   return PG_OK;
 }
 
@@ -384,6 +385,7 @@ int pg_batch_tune(pg_batch *b, int trial_steps) {
   BK(cudaEventCreate(&e0));
   BK(cudaEventCreate(&e1));
   int rc = PG_OK;
+  for (pg_run *r : b->runs) pgi::run_stepped(r);
   for (int gi = 0; gi < 2 && rc == PG_OK; gi++) {
     Group &g = b->g[gi];
     if (g.members.empty()) continue;
@@ -419,7 +421,7 @@ int pg_batch_tune(pg_batch *b, int trial_steps) {
   if (rc) return bfail(b, rc, "tuning launches failed");
   drop_graph(b);
   for (auto &g : b->g)
-    for (pg_run *r : g.members) pgi::run_batched(r, 0);
+    for (pg_run *r : g.members) pgi::run_batched(r);
   return PG_OK;
 }
 

@@ -21,8 +21,10 @@ int run_shape(const pg_run *run, RunShape *out);
 
 // Device descriptor of a 2D run whose clock is set (pg_clock_reset).
 int run_batch_desc(pg_run *run, pgd::BatchRun *d);
-// The batch enqueued steps of this run: the p0 plane is used up, count launches.
-void run_batched(pg_run *run, int64_t launches);
+// The batch enqueued steps of this run: the p0 plane is used up.
+void run_batched(pg_run *run);
+// The batch is about to step this run: its step count is the device's to tell.
+void run_stepped(pg_run *run);
 // One step of the device-resident loop of this run, enqueued on stream s
 // (first, last: of the sequence being queued).
 int run_enqueue_on(pg_run *run, cudaStream_t s, bool first, bool last, int64_t *launches);

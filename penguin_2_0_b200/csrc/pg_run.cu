@@ -76,7 +76,7 @@ struct pg_run {
     pgd::DevClock clk;
   };
   HostPage *page = nullptr;
-  int64_t ncycle = -1;             // clk->ncycle as far as the host knows it (-1: it does not)
+  int64_t ncycle = -1;             // clk->ncycle after the run's own last advance or reset (-1: others have stepped it)
   cudaEvent_t halt_ev[4] = {};
   // event timing
   bool timing = false;
@@ -211,7 +211,16 @@ static int read_clock(pg_run *run) {
   if (int e = host_page(run)) return e;
   CK(cudaMemcpyAsync(&run->page->clk, run->clk, sizeof(pgd::DevClock), cudaMemcpyDeviceToHost, run->stream));
   CK(cudaStreamSynchronize(run->stream));
-  run->ncycle = run->page->clk.ncycle;
+  return PG_OK;
+}
+// the step count an advance starts from
+static int steps_before(pg_run *run, int64_t *before) {
+  if (run->ncycle < 0) {
+    if (int e = read_clock(run)) return e;
+    run->ncycle = run->page->clk.ncycle;
+  }
+  *before = run->ncycle;
+  run->ncycle = -1;                // until finish_advance has seen the end
   return PG_OK;
 }
 
@@ -1047,6 +1056,7 @@ struct HaltProbe {
 static int finish_advance(pg_run *run, int64_t before, int *taken) {
   if (int e = read_clock(run)) return e;
   const pgd::DevClock &c = run->page->clk;
+  run->ncycle = c.ncycle;
   if (taken) *taken = (int)(c.ncycle - before);
   if (c.status != 0) {
     return fail(run, c.status, c.status == PG_ERR_NONFINITE ? "non-finite or non-positive state"
@@ -1065,9 +1075,8 @@ int pg_advance(pg_run *run, int nsteps, int *taken) {
   if (!run) return PG_ERR_ARG;
   if (!run->clock_ready) return fail(run, PG_ERR_STATE, "call pg_clock_reset first");
   CK(cudaSetDevice(run->dev));
-  if (run->ncycle < 0)
-    if (int e = read_clock(run)) return e;
-  const int64_t before = run->ncycle;
+  int64_t before;
+  if (int e = steps_before(run, &before)) return e;
   HaltProbe hp{run};
   if (int e = hp.init()) return fail(run, e, "halt probe set-up");
   const int group = 16;
@@ -1086,9 +1095,8 @@ int pg_advance_graph(pg_run *run, int nsteps, int chunk, int *taken) {
   if (chunk < 1) return fail(run, PG_ERR_ARG, "chunk must be >= 1");
   CK(cudaSetDevice(run->dev));
   if (run->P.ndim == 3 && (chunk & 1)) chunk += 1;   // 3D steps alternate the plane copies
-  if (run->ncycle < 0)
-    if (int e = read_clock(run)) return e;
-  const int64_t before = run->ncycle;
+  int64_t before;
+  if (int e = steps_before(run, &before)) return e;
   int done = 0;
   if (run->p0_live && nsteps > 0) {
     if (int e = enqueue_step(run, true, true, true)) return e;
@@ -1291,18 +1299,14 @@ int run_batch_desc(pg_run *run, pgd::BatchRun *d) {
   return PG_OK;
 }
 
-void run_batched(pg_run *run, int64_t launches) {
-  run->p0_live = false;
-  run->ncycle = -1;
-  run->launches += launches;
-}
+void run_batched(pg_run *run) { run->p0_live = false; }
+void run_stepped(pg_run *run) { run->ncycle = -1; }
 
 int run_enqueue_on(pg_run *run, cudaStream_t s, bool first, bool last, int64_t *launches) {
   cudaStream_t own = run->stream;
   int64_t l0 = run->launches;
   run->stream = s;
   int st = enqueue_step(run, run->p0_live, first, last);
-  run->ncycle = -1;
   run->stream = own;
   run->p0_live = false;
   if (launches) *launches += run->launches - l0;
