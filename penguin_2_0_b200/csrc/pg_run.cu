@@ -76,6 +76,7 @@ struct pg_run {
     pgd::DevClock clk;
   };
   HostPage *page = nullptr;
+  std::mutex page_m;               // its making and its clock: another thread may look at the clock of a run that advances
   int64_t ncycle = -1;             // clk->ncycle after the run's own last advance or reset (-1: others have stepped it)
   cudaEvent_t halt_ev[4] = {};
   // event timing
@@ -199,6 +200,7 @@ static void stage_runs(int dev, int by) {
 }
 
 static int host_page(pg_run *run) {
+  std::lock_guard<std::mutex> l(run->page_m);
   if (run->page) return PG_OK;
   if (cudaHostAlloc(&run->page, sizeof(pg_run::HostPage), cudaHostAllocDefault) != cudaSuccess) {
     run->page = nullptr;
@@ -206,18 +208,21 @@ static int host_page(pg_run *run) {
   }
   return PG_OK;
 }
-// the run's clock, copied to the page; waits for the stream
-static int read_clock(pg_run *run) {
+// the run's clock, by way of the page; waits for the stream
+static int read_clock(pg_run *run, pgd::DevClock *c) {
   if (int e = host_page(run)) return e;
+  std::lock_guard<std::mutex> l(run->page_m);
   CK(cudaMemcpyAsync(&run->page->clk, run->clk, sizeof(pgd::DevClock), cudaMemcpyDeviceToHost, run->stream));
   CK(cudaStreamSynchronize(run->stream));
+  *c = run->page->clk;
   return PG_OK;
 }
 // the step count an advance starts from
 static int steps_before(pg_run *run, int64_t *before) {
   if (run->ncycle < 0) {
-    if (int e = read_clock(run)) return e;
-    run->ncycle = run->page->clk.ncycle;
+    pgd::DevClock c;
+    if (int e = read_clock(run, &c)) return e;
+    run->ncycle = c.ncycle;
   }
   *before = run->ncycle;
   run->ncycle = -1;                // until finish_advance has seen the end
@@ -1002,8 +1007,8 @@ int pg_clock_get(pg_run *run, pg_clock *out, pg_body *planet) {
   if (!run) return PG_ERR_ARG;
   if (!run->clock_ready) return fail(run, PG_ERR_STATE, "clock not reset");
   CK(cudaSetDevice(run->dev));
-  if (int e = read_clock(run)) return e;
-  const pgd::DevClock &c = run->page->clk;
+  pgd::DevClock c;
+  if (int e = read_clock(run, &c)) return e;
   if (out) {
     out->simtime = c.simtime; out->timem = c.timem; out->dt = c.dt; out->dt_used = c.dt_step;
     out->frrot = c.frrot; out->ncycle = c.ncycle; out->make_pict = c.make_pict; out->done = c.done;
@@ -1054,8 +1059,8 @@ struct HaltProbe {
 };
 
 static int finish_advance(pg_run *run, int64_t before, int *taken) {
-  if (int e = read_clock(run)) return e;
-  const pgd::DevClock &c = run->page->clk;
+  pgd::DevClock c;
+  if (int e = read_clock(run, &c)) return e;
   run->ncycle = c.ncycle;
   if (taken) *taken = (int)(c.ncycle - before);
   if (c.status != 0) {
@@ -1172,8 +1177,8 @@ int pg_history(pg_run *run, double *rows, int max, int *rows_out) {
   if (!run || !rows_out) return PG_ERR_ARG;
   if (!run->clock_ready) return fail(run, PG_ERR_STATE, "clock not reset");
   CK(cudaSetDevice(run->dev));
-  if (int e = read_clock(run)) return e;
-  const pgd::DevClock &c = run->page->clk;
+  pgd::DevClock c;
+  if (int e = read_clock(run, &c)) return e;
   int n = c.hist_count < max ? c.hist_count : max;
   if (n > 0 && rows)
     CK(cudaMemcpy(rows, run->hist, (size_t)n * pgd::HIST_COLS * sizeof(double), cudaMemcpyDeviceToHost));
