@@ -153,6 +153,20 @@ static bool stage_drop(int dev) {
   d.n = 0;
   return true;
 }
+// cudaMalloc that gives an idle block back where memory is short.  A failure that
+// is tried again or told by its result does not stay the thread's last error.
+static cudaError_t dev_malloc(int dev, void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess && stage_drop(dev)) {
+    (void)cudaGetLastError();
+    e = cudaMalloc(p, bytes);
+  }
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    *p = nullptr;
+  }
+  return e;
+}
 static void *stage_take(int dev, size_t bytes) {
   DumpStage &d = dump_stage(dev);
   if (bytes <= kStageKeep) {
@@ -172,8 +186,8 @@ static void *stage_take(int dev, size_t bytes) {
     }
   }
   void *p = nullptr;
-  if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
-  return stage_drop(dev) && cudaMalloc(&p, bytes) == cudaSuccess ? p : nullptr;
+  dev_malloc(dev, &p, bytes);
+  return p;
 }
 // after the work on it is complete
 static void stage_give(int dev, void *p) {
@@ -1193,9 +1207,8 @@ int pg_history(pg_run *run, double *rows, int max, int *rows_out) {
 // ---------------------------------------------------------------------------
 // post-processing of the current state (read/ tools)
 static int post_buffer(pg_run *run, size_t n, double **buf) {
-  if (cudaMalloc(buf, n * sizeof(double)) == cudaSuccess) return PG_OK;
-  if (!stage_drop(run->dev) || cudaMalloc(buf, n * sizeof(double)) != cudaSuccess) return fail(run, PG_ERR_NOMEM, "post-processing buffer");
-  return PG_OK;
+  if (dev_malloc(run->dev, (void **)buf, n * sizeof(double)) == cudaSuccess) return PG_OK;
+  return fail(run, PG_ERR_NOMEM, "post-processing buffer");
 }
 
 extern "C" int pg_post_harmonic(pg_run *run, double m, double *an, double *bn) {
