@@ -111,8 +111,8 @@ static int rebuild(pg_batch *b) {
       g.d_runs = nullptr;
       g.d_start = nullptr;
       size_t cap = std::max<size_t>(n, 16);
-      BK(cudaMalloc(&g.d_runs, cap * sizeof(pgd::BatchRun)));
-      BK(cudaMalloc(&g.d_start, 3 * (cap + 1) * sizeof(int)));
+      BK(pgi::device_malloc(b->dev, (void **)&g.d_runs, cap * sizeof(pgd::BatchRun)));
+      BK(pgi::device_malloc(b->dev, (void **)&g.d_start, 3 * (cap + 1) * sizeof(int)));
       g.cap = cap;
     }
     std::vector<pgd::BatchRun> h(n);
@@ -142,8 +142,8 @@ static int rebuild(pg_batch *b) {
     if (b->h_status) cudaFreeHost(b->h_status);
     b->d_clks = nullptr; b->d_status = nullptr; b->h_status = nullptr;
     size_t cap = std::max<size_t>(n, 16);
-    BK(cudaMalloc(&b->d_clks, cap * sizeof(pgd::DevClock *)));
-    BK(cudaMalloc(&b->d_status, cap * sizeof(pg_batch_member)));
+    BK(pgi::device_malloc(b->dev, (void **)&b->d_clks, cap * sizeof(pgd::DevClock *)));
+    BK(pgi::device_malloc(b->dev, (void **)&b->d_status, cap * sizeof(pg_batch_member)));
     BK(cudaHostAlloc(&b->h_status, cap * sizeof(pg_batch_member), cudaHostAllocDefault));
     b->status_cap = cap;
   }
@@ -200,7 +200,7 @@ int pg_batch_create(int device, pg_batch **out) {
   pg_batch *b = new pg_batch();
   b->dev = device;
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc(&b->d_halted, sizeof(int)) != cudaSuccess ||
+      pgi::device_malloc(device, (void **)&b->d_halted, sizeof(int)) != cudaSuccess ||
       cudaHostAlloc(&b->h_halted, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
     pg_batch_destroy(b);
     (void)cudaGetLastError();

@@ -28,6 +28,8 @@ void run_stepped(pg_run *run);
 // One step of the device-resident loop of this run, enqueued on stream s
 // (first, last: of the sequence being queued).
 int run_enqueue_on(pg_run *run, cudaStream_t s, bool first, bool last, int64_t *launches);
+// cudaMalloc that gives the dumps' idle block back where memory is short.
+cudaError_t device_malloc(int dev, void **p, size_t bytes);
 // Device clock of the run.
 pgd::DevClock *run_clock(pg_run *run);
 // which of the two plane copies is current (3D steps flip it)

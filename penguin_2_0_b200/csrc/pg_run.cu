@@ -1331,6 +1331,7 @@ int run_enqueue_on(pg_run *run, cudaStream_t s, bool first, bool last, int64_t *
   return st;
 }
 
+cudaError_t device_malloc(int dev, void **p, size_t bytes) { return dev_malloc(dev, p, bytes); }
 pgd::DevClock *run_clock(pg_run *run) { return run->clk; }
 int run_cur(const pg_run *run) { return run->cur; }
 cudaStream_t run_stream(pg_run *run) { return run->stream; }

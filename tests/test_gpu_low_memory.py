@@ -63,13 +63,18 @@ def test_a_dump_larger_than_what_is_free(idle_block):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("what", ["graph", "harmonic", "load", "create"])
+@pytest.mark.parametrize("what", ["batch", "graph", "harmonic", "load", "create"])
 def test_calls_with_no_memory_free(idle_block, what):
     p = _p(64, 130)
     ic = pg.build_ic(p)
 
-    def call(r):
-        if what == "graph":
+    def call(r, b):
+        if what == "batch":
+            b.add(r)
+            b.advance(4, chunk=2)
+            b.sync()
+            b.remove(r)
+        elif what == "graph":
             r.advance(5, graph_chunk=2)
         elif what == "harmonic":
             r.harmonic(2.0)
@@ -83,15 +88,15 @@ def test_calls_with_no_memory_free(idle_block, what):
 
     out = []
     for full in (False, True):               # the first loads every kernel
-        with pg.Run(p, 0) as r:
+        with pg.Run(p, 0) as r, pg.Batch(0) as b:
             r.load(ic)
             r.clock_reset(0)
             r.advance(1)
             idle_block.save()
             if full:
                 with _memory_taken(0):
-                    call(r)
+                    call(r, b)
             else:
-                call(r)
+                call(r, b)
             out.append(bytes(r.save()))
     assert out[0] == out[1]
