@@ -62,8 +62,12 @@ __device__ __forceinline__ void finish_ring(const Tables &T, int t, double dt, d
   T.ro[rk].off = fma(frrot_next, T.radc[rk], T.rot_v[rk]);
   if (ndim == 3) T.turn[rk] = turn_of(dt, T.res_v[rk], T.irc[rk], vy);
 }
-// rotate_rings ppm.cu:309-322
-__device__ __forceinline__ int rotated(const Tables &T, int rk) { return wrap1(T.rot_j[rk] + T.inc_j[rk], T.nphi); }
+// rotate_rings ppm.cu:309-322, and also where a ring turns more than once in a
+// step (a cold disk of few rings): dumps and sums index by rot_j
+__device__ __forceinline__ int rotated(const Tables &T, int rk) {
+  const int j = wrap1(T.rot_j[rk] + T.inc_j[rk], T.nphi);
+  return (unsigned)j < (unsigned)T.nphi ? j : wrapm(j, T.nphi);
+}
 
 __global__ void k_index(Tables T, double dt, double frrot, int fargo) {
   after_previous();
