@@ -373,8 +373,8 @@ typedef struct pg_batch_member {
 typedef struct pg_batch_shape {
   int grid_x, grid_y;          /* CTAs of the batched radial / azimuthal
                                   sweeps (0: one CTA per tile)              */
-  int minb;                    /* 4 or 8: CTAs per SM of the tuner's
-                                  persistent grids                          */
+  int minb;                    /* 4 or 8; the sweeps keep 4 CTAs per SM
+                                  either way                                */
   int pad;
 } pg_batch_shape;
 int pg_batch_create(int device, pg_batch **out);

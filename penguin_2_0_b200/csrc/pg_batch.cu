@@ -199,6 +199,7 @@ int pg_batch_create(int device, pg_batch **out) {
   if (cudaSetDevice(device) != cudaSuccess) return PG_ERR_CUDA;
   pg_batch *b = new pg_batch();
   b->dev = device;
+  b->g[1].shape.minb = 4;
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
       pgi::device_malloc(device, (void **)&b->d_halted, sizeof(int)) != cudaSuccess ||
       cudaHostAlloc(&b->h_halted, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
@@ -389,14 +390,10 @@ int pg_batch_tune(pg_batch *b, int trial_steps) {
   for (int gi = 0; gi < 2 && rc == PG_OK; gi++) {
     Group &g = b->g[gi];
     if (g.members.empty()) continue;
-    // candidates: one CTA per tile, or a persistent grid of 1 or 2 times 8 or
-    // 4 CTAs per SM walking the tile queue
+    // candidates: one CTA per tile, or a persistent grid of 1, 2, 3, 4 or 6
+    // times the CTAs that are resident (4 per SM) walking the tile queue
     std::vector<pg_batch_shape> cand;
-    for (int minb : {8, 4})
-      for (int waves : {0, 1, 2}) {
-        int grid = waves ? waves * minb * sms : 0;
-        cand.push_back(pg_batch_shape{grid, grid, minb, 0});
-      }
+    for (int waves : {0, 1, 2, 3, 4, 6}) cand.push_back(pg_batch_shape{waves * 4 * sms, waves * 4 * sms, g.shape.minb, 0});
     float best = 1e30f;
     pg_batch_shape keep = g.shape;
     for (const pg_batch_shape &c : cand) {
