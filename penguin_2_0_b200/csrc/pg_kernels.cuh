@@ -141,7 +141,6 @@ struct BatchRun {
   long long p0_cycle;     //   read by the radial sweep of the step with ncycle == p0_cycle
   double *ring_part;
   unsigned int *counter;
-  double p_alpha;
   int fargo, plnt;
 };
 
@@ -273,15 +272,15 @@ void rotate(const Tables &T, cudaStream_t s);
 // disk mass (mode 0), radial force (8) or torque (9) on the planet into *out;
 // part: 2 nr nk doubles, counter: 0 between launches
 template <class RT>
-void reduce(const Tables &T, const RT *r, const Body &pl, double exclude, int mode, int plnt, double p_alpha, int ndim,
+void reduce(const Tables &T, const RT *r, const Body &pl, double exclude, int mode, int plnt, int ndim,
             double *part, unsigned *counter, double *out, cudaStream_t s);
 // between two steps: any of the parts BETWEEN_*
 template <class RT>
-void between(const Tables &T, const RT *r, DevClock *clk, double *part, unsigned *counter, double p_alpha, int fargo,
+void between(const Tables &T, const RT *r, DevClock *clk, double *part, unsigned *counter, int fargo,
              int plnt, int ndim, int fl, cudaStream_t s);
 // moving planet (plnt_flag 2): a step's end up to the kick
 template <class RT>
-void moving(const Tables &T, const RT *r, DevClock *clk, double *part, unsigned *counter, double p_alpha, int ndim,
+void moving(const Tables &T, const RT *r, DevClock *clk, double *part, unsigned *counter, int ndim,
             cudaStream_t s);
 // between() of every member of a batch; CTAs of a member
 template <class RT>

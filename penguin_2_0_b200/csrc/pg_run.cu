@@ -306,7 +306,7 @@ static int enqueue_step_t(pg_run *run, bool first_p0, bool first, bool last) {
   if (tm && ev_pair(run, 3, e_step)) return fail(run, PG_ERR_CUDA, "event record");
   const bool moving = P.plnt_flag == 2;
   auto between = [&](int fl) {
-    pgk::between<RT>(run->T, planes_of<RT>(run, run->cur)[0], run->clk, run->ring_part, run->counter, P.p_alpha,
+    pgk::between<RT>(run->T, planes_of<RT>(run, run->cur)[0], run->clk, run->ring_part, run->counter,
                      P.FARGO_flag, P.plnt_flag > 0, P.ndim, fl, s);
     n++;
   };
@@ -347,7 +347,7 @@ static int enqueue_step_t(pg_run *run, bool first_p0, bool first, bool last) {
     // drifted planet (reductions 8 and 9), kick; FrRot is then known and the
     // next get_dt's CFL runs on the stored state
     RT **cp = planes_of<RT>(run, run->cur);
-    pgk::moving<RT>(run->T, cp[0], run->clk, run->ring_part, run->counter, P.p_alpha, P.ndim, s); n++;
+    pgk::moving<RT>(run->T, cp[0], run->clk, run->ring_part, run->counter, P.ndim, s); n++;
     pgk::cfl<RT>(run->T, cp[0], cp[1], cp[2], cp[3], nullptr, run->ph, 0.0, P.ndim, nullptr, run->clk, 0, nullptr,
                  nullptr, s); n++;
   }
@@ -890,10 +890,10 @@ int pg_reduce(pg_run *run, const pg_body *planet, double exclude, int mode, doub
   double *h = &run->page->sum;     // the kernel writes it
   const int plnt = run->P.plnt_flag > 0;
   if (run->fp32)
-    pgk::reduce<float>(run->T, run->p32[run->cur][0], b, exclude, mode, plnt, run->P.p_alpha, run->P.ndim,
+    pgk::reduce<float>(run->T, run->p32[run->cur][0], b, exclude, mode, plnt, run->P.ndim,
                        run->ring_part, run->counter, h, run->stream);
   else
-    pgk::reduce<double>(run->T, run->planes[run->cur][0], b, exclude, mode, plnt, run->P.p_alpha, run->P.ndim,
+    pgk::reduce<double>(run->T, run->planes[run->cur][0], b, exclude, mode, plnt, run->P.ndim,
                         run->ring_part, run->counter, h, run->stream);
   if (int e = check_launch(run, 1)) return e;
   CK(cudaStreamSynchronize(run->stream));
@@ -1144,7 +1144,6 @@ int pg_advance_graph(pg_run *run, int nsteps, int chunk, int *taken) {
     run->launches = l0;
     run->cur = cur0;
   }
-  int64_t per = 0;
   HaltProbe hp{run};
   if (int e = hp.init()) return fail(run, e, "halt probe set-up");
   for (; done + chunk <= nsteps; done += chunk) {
@@ -1154,13 +1153,11 @@ int pg_advance_graph(pg_run *run, int nsteps, int chunk, int *taken) {
     CK(cudaGraphLaunch(run->gexec, run->stream));
     if (run->timing && ev_close(run, e)) return fail(run, PG_ERR_CUDA, "event record");
     run->launches += run->graph_kernels;
-    per++;
     if (hp.post()) return fail(run, PG_ERR_CUDA, "halt probe");
   }
   for (bool first = true; done < nsteps; done++, first = false) {
     if (int e = enqueue_step(run, false, first, done == nsteps - 1)) return e;
   }
-  (void)per;
   return finish_advance(run, before, taken);
 }
 
@@ -1311,7 +1308,6 @@ int run_batch_desc(pg_run *run, pgd::BatchRun *d) {
   }
   d->ring_part = run->ring_part;
   d->counter = run->counter;
-  d->p_alpha = run->P.p_alpha;
   d->fargo = run->P.FARGO_flag;
   d->plnt = run->P.plnt_flag > 0;
   return PG_OK;

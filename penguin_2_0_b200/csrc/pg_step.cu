@@ -116,14 +116,13 @@ __device__ __forceinline__ double cta_tree1024(double (&v)[4], double *red) {
 
 // What a ring's sum needs of the planet (modes 8 and 9)
 struct RingForce {
-  double m, x, y, ix2, b2, cy, sy, exclude2, p_alpha;
-  __device__ __forceinline__ RingForce(const Body &b, double exclude, double alpha) {
+  double m, x, y, ix2, b2, cy, sy, exclude2;
+  __device__ __forceinline__ RingForce(const Body &b, double exclude) {
     m = b.m; x = b.x; y = b.y;
     ix2 = 1.0 / (b.x * b.x);
     b2 = fma(b.x, b.x, b.rs * b.rs);
     sincos(b.y, &sy, &cy);
     exclude2 = exclude * exclude;
-    p_alpha = alpha;
   }
 };
 
@@ -223,11 +222,11 @@ __device__ __forceinline__ bool last_cta(unsigned *counter, unsigned nb) {
 
 template <class RT>
 __global__ void __launch_bounds__(ST) k_reduce(Tables T, const RT *R, Body pl, double exclude, int mode, int plnt,
-                                               double p_alpha, int ndim, double *part, unsigned *counter, double *out) {
+                                               int ndim, double *part, unsigned *counter, double *out) {
   after_previous();
   __shared__ double red[ST];
   const bool zero = mode != 0 && plnt && ndim != 2;     // the reference's force sums are 2D
-  const RingForce F(pl, exclude, p_alpha);
+  const RingForce F(pl, exclude);
   for (int rt = blockIdx.x; rt < T.nr * T.nk; rt += gridDim.x) {
     const int rk = rt / T.nr * T.nrg + rt % T.nr + NPAD;
     const double x = zero ? 0.0 : ring_sum<RT>(T, R, rt, T.rot_j[rk], plnt ? mode : 0, ndim, F, red);
@@ -262,27 +261,17 @@ __device__ __forceinline__ double pow_host_form(double x, double y) {
   if (y == 2.0) return x * x;
   return pow(x, y);
 }
-__device__ void d_drift(Body &pl, double FrRot, double dt, const DevClock &c) {
+// moving planet: the drift moves x, and the softening follows it as
+// kick_drift_kick does on the host, rs = rs_fac h(x), h = sqrt(cs2(x) x^3)
+// with cs2 = sc_h^2 x^-p_beta (disk_profile.cu:39-52)
+__device__ void d_drift_moving(Body &pl, double FrRot, double dt, const DevClock &c) {
   double old_rad = pl.x;
   pl.x += dt * pl.vx;
   pl.y += dt * pl.vy;
   pl.vy = ((pl.vy + FrRot) * old_rad * old_rad / pl.x / pl.x) - FrRot;
   if (pl.y < 0.0) pl.y += 6.283185307179586476925286766559;
   if (pl.y >= 6.283185307179586476925286766559) pl.y -= 6.283185307179586476925286766559;
-  // rs = rs_fac*get_h(x), get_h = sqrt(cs2(x) x^3); cs2 = sc2 * x^-p_beta is
-  // evaluated on the host for the fixed-orbit case and never changes there
-  (void)c;
-}
-// moving planet: the drift moves x, and the softening follows it as
-// kick_drift_kick does on the host, rs = rs_fac h(x), h = sqrt(cs2(x) x^3)
-// with cs2 = sc_h^2 x^-p_beta (disk_profile.cu:39-52)
-__device__ void d_drift_moving(Body &pl, double FrRot, double dt, const DevClock &c) {
-  d_drift(pl, FrRot, dt, c);
   pl.rs = c.rs_fac * sqrt(c.sc2 * pow_host_form(pl.x, -c.p_beta) * pl.x * pl.x * pl.x);
-}
-__device__ void d_forces_fixed(Body &pl, double FrRot) {
-  pl.fx = -1.0 / pl.x / pl.x + pl.x * pow_host_form(pl.vy + FrRot, 2.0);
-  pl.fy = 0.0;
 }
 
 // ---------------------------------------------------------------------------
@@ -492,7 +481,7 @@ __device__ __forceinline__ void step_scalars(StepShm &S, int fl, bool post) {
 // BETWEEN_DIAG its diagnostics, BETWEEN_PRE the start of the next.
 template <class RT>
 __device__ __forceinline__ void between_body(StepShm &S, const Tables &T, const RT *R, DevClock *clk, double *part,
-                                             unsigned *counter, double p_alpha, int fargo, int torque, int ndim, int fl, int b,
+                                             unsigned *counter, int fargo, int torque, int ndim, int fl, int b,
                                              int nb) {
   const int rings = T.nr * T.nk, tid = threadIdx.x;
   clock_in(S, clk);
@@ -510,7 +499,7 @@ __device__ __forceinline__ void between_body(StepShm &S, const Tables &T, const 
     S.c.pc.cy = cy;
   }
   if (S.print) {
-    const RingForce F(S.planet, 0.0, p_alpha);
+    const RingForce F(S.planet, 0.0);
     for (int rt = b; rt < rings; rt += nb) {
       const int rk = rt / T.nr * T.nrg + rt % T.nr + NPAD, rot = post ? rotated(T, rk) : T.rot_j[rk];
       const double m = ring_sum<RT>(T, R, rt, rot, 0, ndim, F, S.red);
@@ -548,10 +537,10 @@ __device__ __forceinline__ void between_body(StepShm &S, const Tables &T, const 
 
 template <class RT>
 __global__ void __launch_bounds__(ST) k_between(Tables T, const RT *R, DevClock *clk, double *part, unsigned *counter,
-                                                double p_alpha, int fargo, int torque, int ndim, int fl) {
+                                                int fargo, int torque, int ndim, int fl) {
   after_previous();
   __shared__ StepShm S;
-  between_body<RT>(S, T, R, clk, part, counter, p_alpha, fargo, torque, ndim, fl, blockIdx.x, gridDim.x);
+  between_body<RT>(S, T, R, clk, part, counter, fargo, torque, ndim, fl, blockIdx.x, gridDim.x);
 }
 
 // members' CTAs by the queue's prefix sums
@@ -564,14 +553,14 @@ __global__ void __launch_bounds__(ST) kb_between(BatchQueue q, int fl) {
   const RT *R;
   if constexpr (sizeof(RT) == 4) R = (const RT *)b.QX.r;   // a 2D step ends in its first planes
   else R = (const RT *)b.PX.r;
-  between_body<RT>(S, b.T, R, b.clk, b.ring_part, b.counter, b.p_alpha, b.fargo, b.plnt, 2, fl, blockIdx.x - q.start[r],
+  between_body<RT>(S, b.T, R, b.clk, b.ring_part, b.counter, b.fargo, b.plnt, 2, fl, blockIdx.x - q.start[r],
                    q.start[r + 1] - q.start[r]);
 }
 
 // moving planet: the step's end up to the kick
 template <class RT>
 __global__ void __launch_bounds__(ST) k_moving(Tables T, const RT *R, DevClock *clk, double *part, unsigned *counter,
-                                               double p_alpha, int ndim) {
+                                               int ndim) {
   after_previous();
   __shared__ StepShm S;
   const int rings = T.nr * T.nk, tid = threadIdx.x;
@@ -584,7 +573,7 @@ __global__ void __launch_bounds__(ST) k_moving(Tables T, const RT *R, DevClock *
     S.c.planet.m = d_set_M_p(S.c, S.c.simtime);
   }
   __syncthreads();
-  const RingForce F(S.c.planet, 0.0, p_alpha);
+  const RingForce F(S.c.planet, 0.0);
   for (int rt = blockIdx.x; rt < rings; rt += gridDim.x) {
     const int rk = rt / T.nr * T.nrg + rt % T.nr + NPAD, rot = rotated(T, rk);
     const double f8 = ndim == 2 ? ring_sum<RT>(T, R, rt, rot, 8, ndim, F, S.red) : 0.0;
@@ -638,30 +627,30 @@ void index_shift(const Tables &T, double dt, double frrot, int fargo, cudaStream
 void rotate(const Tables &T, cudaStream_t s) { launch(k_rotate, (T.nr * T.nk + 127) / 128, 128, 0, s, T); }
 
 template <class RT>
-void reduce(const Tables &T, const RT *r, const Body &pl, double exclude, int mode, int plnt, double p_alpha, int ndim,
+void reduce(const Tables &T, const RT *r, const Body &pl, double exclude, int mode, int plnt, int ndim,
             double *part, unsigned *counter, double *out, cudaStream_t s) {
-  launch(k_reduce<RT>, ring_ctas(T.nr * T.nk), ST, 0, s, T, r, pl, exclude, mode, plnt, p_alpha, ndim, part, counter, out);
+  launch(k_reduce<RT>, ring_ctas(T.nr * T.nk), ST, 0, s, T, r, pl, exclude, mode, plnt, ndim, part, counter, out);
 }
 template <class RT>
-void between(const Tables &T, const RT *r, DevClock *clk, double *part, unsigned *counter, double p_alpha, int fargo,
+void between(const Tables &T, const RT *r, DevClock *clk, double *part, unsigned *counter, int fargo,
              int plnt, int ndim, int fl, cudaStream_t s) {
-  launch(k_between<RT>, ring_ctas(T.nr * T.nk), ST, 0, s, T, r, clk, part, counter, p_alpha, fargo, plnt && ndim == 2, ndim, fl);
+  launch(k_between<RT>, ring_ctas(T.nr * T.nk), ST, 0, s, T, r, clk, part, counter, fargo, plnt && ndim == 2, ndim, fl);
 }
 template <class RT>
-void moving(const Tables &T, const RT *r, DevClock *clk, double *part, unsigned *counter, double p_alpha, int ndim,
+void moving(const Tables &T, const RT *r, DevClock *clk, double *part, unsigned *counter, int ndim,
             cudaStream_t s) {
-  launch(k_moving<RT>, ring_ctas(T.nr * T.nk), ST, 0, s, T, r, clk, part, counter, p_alpha, ndim);
+  launch(k_moving<RT>, ring_ctas(T.nr * T.nk), ST, 0, s, T, r, clk, part, counter, ndim);
 }
 template <class RT>
 void batch_between(const BatchQueue &q, int fl, cudaStream_t s) {
   if (q.total > 0) launch(kb_between<RT>, q.total, ST, 0, s, q, fl);
 }
 #define PG_STEP(RT)                                                                                                      \
-  template void reduce<RT>(const Tables &, const RT *, const Body &, double, int, int, double, int, double *, unsigned *, \
+  template void reduce<RT>(const Tables &, const RT *, const Body &, double, int, int, int, double *, unsigned *, \
                            double *, cudaStream_t);                                                                      \
-  template void between<RT>(const Tables &, const RT *, DevClock *, double *, unsigned *, double, int, int, int, int,    \
+  template void between<RT>(const Tables &, const RT *, DevClock *, double *, unsigned *, int, int, int, int,    \
                             cudaStream_t);                                                                               \
-  template void moving<RT>(const Tables &, const RT *, DevClock *, double *, unsigned *, double, int, cudaStream_t);     \
+  template void moving<RT>(const Tables &, const RT *, DevClock *, double *, unsigned *, int, cudaStream_t);     \
   template void batch_between<RT>(const BatchQueue &, int, cudaStream_t);
 PG_STEP(double)
 PG_STEP(float)

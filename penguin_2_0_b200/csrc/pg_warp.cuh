@@ -198,8 +198,7 @@ enum Slot {
 };
 // Place of cell c of a lane in a slot, from the lane's own base (ws_lane):
 // pairs of cells (C = 4) or single cells (C = 3) of all lanes side by side,
-// PIECE apart.  c = -1 and c = C are the neighbour lanes' cells (in the slot
-// for any lane).  Pieces, slots and warps are padded so that a tile's loads
+// PIECE apart.  Pieces, slots and warps are padded so that a tile's loads
 // and stores (neighbouring threads on neighbouring columns, that is warps)
 // fall in different banks.
 constexpr int SLOT = 132;
@@ -209,11 +208,6 @@ template <int C>
 constexpr int PIECE = C == 4 ? 66 : 34;
 template <int C>
 __device__ __forceinline__ constexpr int ws_lane(int lane) { return C == 4 ? 2 * lane : lane; }
-template <int C>
-__device__ __forceinline__ constexpr int ws_cell(int c) {
-  return C == 4 ? (c < 0 ? PIECE<4> - 1 : c < 4 ? (c >> 1) * PIECE<4> + (c & 1) : 2)
-                : (c < 0 ? 2 * PIECE<3> - 1 : c < 3 ? c * PIECE<3> : 1);
-}
 
 // What a lane knows of its pencil and its cells.
 template <int C>
@@ -237,7 +231,6 @@ struct Lane {
   __device__ __forceinline__ bool in(int c, int lo, int hi) const {
     return (unsigned)(n0 + c - lo) < (unsigned)(lim - hi - lo);
   }
-  __device__ __forceinline__ double get(int slot, int c) const { return ws[slot * SLOT + ws_cell<C>(c)]; }
 };
 
 template <int C>
