@@ -75,7 +75,7 @@ __device__ __forceinline__ double rcp(double b) {
   return fma(y, fma(e, e, e), y);
 }
 // 1 / sqrt(x), x > 0 and normal: rsqrt.approx.ftz.f64 and one third-order
-// step, y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2
+// step of the same kind (Householder), y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2
 __device__ __forceinline__ double rsq(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
