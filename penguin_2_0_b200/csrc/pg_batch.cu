@@ -7,9 +7,10 @@
 //     step is one launch per phase: radial sweep and azimuthal sweep (a tile
 //     queue over the pencil chunks of every member; CTA b takes tiles b,
 //     b + grid, ...) and what lies between two steps (a few CTAs per member).
-//   * 3D members, members with a moving planet (plnt_flag 2) and isentropic
-//     members (EOS 1) take their own launch sequence (the per-run fused
-//     step) in the same stream order; the queue kernels are isothermal 2D.
+//   * 3D members, members with a moving planet (plnt_flag 2), isentropic
+//     members (EOS 1) and members whose ghost rings lack a state take their own
+//     launch sequence (the per-run fused step) in the same stream order; the
+//     queue kernels are isothermal 2D.
 // The step sequence of `chunk` steps is captured once as a CUDA graph and
 // replayed; membership changes rebuild the descriptors and the graph.
 #include <cuda_runtime.h>
@@ -100,7 +101,7 @@ static int rebuild(pg_batch *b) {
   for (pg_run *r : b->runs) {
     pgi::RunShape sh;
     pgi::run_shape(r, &sh);
-    if (sh.ndim == 3 || sh.moving || sh.eos) b->solo.push_back(r);
+    if (sh.ndim == 3 || sh.moving || sh.eos || sh.odd) b->solo.push_back(r);
     else b->g[sh.fp32].members.push_back(r);
   }
   for (auto &g : b->g) {

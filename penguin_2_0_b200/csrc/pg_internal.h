@@ -13,6 +13,7 @@ struct RunShape {
   int dev, ndim, fp32, loaded, clock_ready, p0_live;
   int moving;              // plnt_flag 2: the planet feels the disk (own step sequence)
   int eos;                 // EOS 1: isentropic sweeps (own step sequence)
+  int odd;                 // ghost rings without a state (own step sequence)
   int nr, nphi, nk;
   int tiles_x, tiles_y;    // CTAs of the radial and azimuthal sweeps
   int ctas_b;              // CTAs between two steps

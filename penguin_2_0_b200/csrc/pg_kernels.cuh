@@ -55,6 +55,7 @@ struct __align__(16) RingOut {
 // "ring" index rk = k*nrg + row.
 struct Tables {
   int nr, nphi, nk, nrg;
+  int odd;                                      // ghost cells without a state: 1 of the radial sweep, 2 of the polar one
   Chunking cx, cy, cz;
   Tile tx[2], ty[2], tz[2];                     // per axis: full chunks, last chunk (pgk::tiles)
   unsigned long long mnr;                       // 2^40 / nr rounded up

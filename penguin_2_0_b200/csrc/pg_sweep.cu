@@ -216,7 +216,7 @@ __device__ __forceinline__ int place_lane(Lane<C> &L, const Tile &M, int pw, con
 
 // ---------------------------------------------------------------------------
 // radial sweep: tile t of the run
-template <class RT, bool THREED, int EOS>
+template <class RT, bool THREED, int EOS, bool ODD>
 __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const PlanesT<RT> &P, const Phys &ph,
                                              const SweepCtl &ctl, const StepIn &st, int t) {
   constexpr int C = 4;
@@ -317,7 +317,7 @@ __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const 
     {
       double cs[C];
       ld<C>(L, A_IW, cs);
-      if (EOS == 0 && !P.p0) {
+      if (EOS == 0 && !P.p0 && !ODD) {
         double snd[C];
         ld_row<C>(L, R_SND, snd);
         PG_CELLS cs[c] = snd[c] * cs[c];
@@ -330,7 +330,7 @@ __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const 
           cs[c] = 0.5 * st.dt * root(x) * cs[c];
         }
       }
-      warp_chain<0, THREED, EOS, C>(L, pl, ph, cs);
+      warp_chain<0, THREED, EOS, ODD, C>(L, pl, ph, cs);
     }
     // device_viscosity_r viscosity.cu:370-421; the stored v_phi is v / r_cyl
     double irc[C], rc[C], v[C];
@@ -393,13 +393,13 @@ __device__ __forceinline__ void sweep_x_tile(TileShm &S, const Tables &T, const 
   }
 }
 
-template <class RT, bool THREED, int EOS>
+template <class RT, bool THREED, int EOS, bool ODD>
 __global__ void __launch_bounds__(NT, MINB) k_sweep_x(Tables T, PlanesT<RT> P, Phys ph, SweepCtl ctl) {
   extern __shared__ __align__(16) unsigned char shm[];
   after_previous();
   StepIn st;
   if (!load_step(ctl, st)) return;
-  sweep_x_tile<RT, THREED, EOS>(*reinterpret_cast<TileShm *>(shm), T, P, ph, ctl, st, blockIdx.x);
+  sweep_x_tile<RT, THREED, EOS, ODD>(*reinterpret_cast<TileShm *>(shm), T, P, ph, ctl, st, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -597,7 +597,7 @@ __device__ __forceinline__ void sweep_y_task(double *ws, const PlanetC &SP, cons
         put<C>(L, W_P, p);
       }
     }
-    warp_chain<1, THREED, EOS, C>(L, pl, ph, cs);
+    warp_chain<1, THREED, EOS, false, C>(L, pl, ph, cs);
     // device_viscosity_p viscosity.cu:423-472 on x = r_cyl phi
     if (ph.visc) {
       const double nu = T.nu[rk], ir = L.irad;
@@ -668,7 +668,7 @@ __global__ void __launch_bounds__(NT, MINB) k_sweep_y(Tables T, PlanesT<RT> P, P
 // centrifugal term); viscosity follows device_viscosity_p's pattern on the
 // arc length r*theta.  A tile is 4 P columns of one ring, so its row values
 // (one layer per row) are shared by the whole CTA.
-template <class RT, int EOS, int C>
+template <class RT, int EOS, bool ODD, int C>
 __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const PlanesT<RT> &P, const Phys &ph,
                                              const SweepCtl &ctl, const StepIn &st, bool run, int ntop, int t) {
   const int nphi = T.nphi, nrg = T.nrg, nk = T.nk, full = T.cz.loop - 1, tid = threadIdx.x;
@@ -786,7 +786,7 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
       double cs[C];
       ld<C>(L, A_IW, cs);
       const double a = 0.5 * st.dt * L.irad;
-      if (EOS == 0) {
+      if (EOS == 0 && !ODD) {
         double snd[C];
         ld_row<C>(L, R_SND, snd);
         PG_CELLS cs[c] = a * snd[c] * cs[c];
@@ -799,7 +799,7 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
           cs[c] = a * root(x) * cs[c];
         }
       }
-      warp_chain<2, true, EOS, C>(L, pl, ph, cs);
+      warp_chain<2, true, EOS, ODD, C>(L, pl, ph, cs);
     }
     if (ph.visc) {
       double a[C], nr[C], n1[C], d1[C], d2[C], dtr[C];
@@ -845,13 +845,13 @@ __device__ __forceinline__ void sweep_z_tile(TileShm &S, const Tables &T, const 
   if (ctl.fuse) report(ctl, rate, bad);
 }
 
-template <class RT, int EOS, int C>
+template <class RT, int EOS, bool ODD, int C>
 __global__ void __launch_bounds__(NT, MINB) k_sweep_z(Tables T, PlanesT<RT> P, Phys ph, SweepCtl ctl, int ntop) {
   extern __shared__ __align__(16) unsigned char shm[];
   after_previous();
   StepIn st;
   const bool run = load_step(ctl, st);
-  sweep_z_tile<RT, EOS, C>(*reinterpret_cast<TileShm *>(shm), T, P, ph, ctl, st, run, ntop, blockIdx.x);
+  sweep_z_tile<RT, EOS, ODD, C>(*reinterpret_cast<TileShm *>(shm), T, P, ph, ctl, st, run, ntop, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -877,7 +877,7 @@ __global__ void __launch_bounds__(NT, MINB) kb_sweep_x(BatchQueue q) {
     if (load_step(ctl, st)) {
       PlanesT<RT> P = batch_planes<RT>(b, 0);
       P.p0 = (sizeof(RT) == 8 && b.p0 && b.clk->ncycle == b.p0_cycle) ? b.p0 : nullptr;
-      sweep_x_tile<RT, false, 0>(*reinterpret_cast<TileShm *>(shm), b.T, P, b.ph, ctl, st, t - q.start[r]);
+      sweep_x_tile<RT, false, 0, false>(*reinterpret_cast<TileShm *>(shm), b.T, P, b.ph, ctl, st, t - q.start[r]);
     }
     __syncthreads();
   }
@@ -958,24 +958,56 @@ int tiles_x(const Tables &T) { return T.nk * ((T.cx.loop - 1) * T.tx[0].ng + T.t
 int tiles_y(const Tables &T) { return (T.cy.loop - 1) * T.ty[0].ng + T.ty[1].ng; }
 static int tiles_z(const Tables &T) { return T.nr * ((T.cz.loop - 1) * T.tz[0].ng + T.tz[1].ng); }
 
-// the sweeps take their shared blocks (some 12 KB per warp) as dynamic shared
-// memory, above the 48 KiB default limit: set per device before a launch
-int setup_device() {
-  const void *k[] = {(const void *)k_sweep_x<double, false, 0>, (const void *)k_sweep_x<double, true, 0>,
-                     (const void *)k_sweep_x<double, false, 1>, (const void *)k_sweep_x<double, true, 1>,
-                     (const void *)k_sweep_x<float, false, 0>,  (const void *)k_sweep_x<float, true, 0>,
-                     (const void *)k_sweep_z<double, 0, 3>,     (const void *)k_sweep_z<double, 0, 4>,
-                     (const void *)k_sweep_z<double, 1, 3>,     (const void *)k_sweep_z<double, 1, 4>,
-                     (const void *)k_sweep_z<float, 0, 3>,      (const void *)k_sweep_z<float, 0, 4>,
-                     (const void *)kb_sweep_x<double>,          (const void *)kb_sweep_x<float>,
-                     (const void *)k_sweep_y<double, false, 0>, (const void *)k_sweep_y<double, true, 0>,
-                     (const void *)k_sweep_y<double, false, 1>, (const void *)k_sweep_y<double, true, 1>,
-                     (const void *)k_sweep_y<float, false, 0>,  (const void *)k_sweep_y<float, true, 0>,
-                     (const void *)kb_sweep_y<double>,          (const void *)kb_sweep_y<float>};
-  for (const void *f : k)
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileShm)) != cudaSuccess) return 1;
-  return 0;
+// The sweeps' kernels, by plane type, dimension, equation of state, cells per lane
+// and whether ghost cells hold no state (Tables::odd).
+template <class RT>
+using SweepK = void (*)(Tables, PlanesT<RT>, Phys, SweepCtl);
+template <class RT>
+using SweepZK = void (*)(Tables, PlanesT<RT>, Phys, SweepCtl, int);
+template <class RT, bool ODD>
+static SweepK<RT> kernel_x(bool three, int eos) {
+  if constexpr (sizeof(RT) == 8) {
+    if (eos) return three ? k_sweep_x<RT, true, 1, ODD> : k_sweep_x<RT, false, 1, ODD>;
+  }
+  return three ? k_sweep_x<RT, true, 0, ODD> : k_sweep_x<RT, false, 0, ODD>;
 }
+template <class RT>
+static SweepK<RT> kernel_y(bool three, int eos) {
+  if constexpr (sizeof(RT) == 8) {
+    if (eos) return three ? k_sweep_y<RT, true, 1> : k_sweep_y<RT, false, 1>;
+  }
+  return three ? k_sweep_y<RT, true, 0> : k_sweep_y<RT, false, 0>;
+}
+template <class RT, bool ODD>
+static SweepZK<RT> kernel_z(int C, int eos) {
+  if constexpr (sizeof(RT) == 8) {
+    if (eos) return C == 3 ? k_sweep_z<RT, 1, ODD, 3> : k_sweep_z<RT, 1, ODD, 4>;
+  }
+  return C == 3 ? k_sweep_z<RT, 0, ODD, 3> : k_sweep_z<RT, 0, ODD, 4>;
+}
+
+// The sweeps take their shared blocks as dynamic shared memory, 44.8 KB for a tile
+// of 4 warps, below the default limit of 48 KiB.  Naming the kernels to the runtime
+// here loads the module in a process's first pg_create (7.5-9 ms of it for 3.4-4.5);
+// the first load then takes that much less, 6.5-8.5 ms for 9.5-12.
+static_assert(sizeof(TileShm) <= 48 * 1024 && sizeof(YShm<1>) <= sizeof(TileShm), "within the default limit");
+template <class RT>
+static bool name_kernels() {
+  bool ok = true;
+  auto name = [&](const void *f) {
+    ok = ok && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileShm)) == cudaSuccess;
+  };
+  for (int eos = 0; eos < (sizeof(RT) == 8 ? 2 : 1); eos++)
+    for (bool three : {false, true}) {
+      name((const void *)kernel_x<RT, false>(three, eos));
+      name((const void *)kernel_y<RT>(three, eos));
+      name((const void *)kernel_z<RT, false>(three ? 3 : 4, eos));
+    }
+  name((const void *)kb_sweep_x<RT>);
+  name((const void *)kb_sweep_y<RT>);
+  return ok;
+}
+int setup_device() { return name_kernels<double>() && name_kernels<float>() ? 0 : 1; }
 
 void axis_tables(const Tables &T, int ndim, cudaStream_t s) {
   k_axis_table<<<T.cx.loop, ARR, 0, s>>>(T, 0, 4, const_cast<double *>(T.ax[0]));
@@ -986,44 +1018,21 @@ size_t axis_table_elems(const Chunking &ch) { return (size_t)ch.loop * A_COUNT *
 
 template <class RT>
 void sweep_x(const Tables &T, const PlanesT<RT> &P, const Phys &ph, const SweepCtl &c, int ndim, cudaStream_t s) {
-  const int n = tiles_x(T);
-  if constexpr (sizeof(RT) == 8) {
-    if (ph.eos) {
-      if (ndim == 3) launch(k_sweep_x<RT, true, 1>, n, NT, sizeof(TileShm), s, T, P, ph, c);
-      else launch(k_sweep_x<RT, false, 1>, n, NT, sizeof(TileShm), s, T, P, ph, c);
-      return;
-    }
-  }
-  if (ndim == 3) launch(k_sweep_x<RT, true, 0>, n, NT, sizeof(TileShm), s, T, P, ph, c);
-  else launch(k_sweep_x<RT, false, 0>, n, NT, sizeof(TileShm), s, T, P, ph, c);
+  launch(T.odd & 1 ? kernel_x<RT, true>(ndim == 3, ph.eos) : kernel_x<RT, false>(ndim == 3, ph.eos), tiles_x(T), NT,
+         sizeof(TileShm), s, T, P, ph, c);
 }
 
 template <class RT>
 void sweep_y(const Tables &T, const PlanesT<RT> &P, const Phys &ph, const SweepCtl &c, int ndim, cudaStream_t s) {
-  const int n = tiles_y(T);
-  if constexpr (sizeof(RT) == 8) {
-    if (ph.eos) {
-      if (ndim == 3) launch(k_sweep_y<RT, true, 1>, n, NT, sizeof(YShm<1>), s, T, P, ph, c);
-      else launch(k_sweep_y<RT, false, 1>, n, NT, sizeof(YShm<1>), s, T, P, ph, c);
-      return;
-    }
-  }
-  if (ndim == 3) launch(k_sweep_y<RT, true, 0>, n, NT, sizeof(YShm<0>), s, T, P, ph, c);
-  else launch(k_sweep_y<RT, false, 0>, n, NT, sizeof(YShm<0>), s, T, P, ph, c);
+  launch(kernel_y<RT>(ndim == 3, ph.eos), tiles_y(T), NT, sizeof(RT) == 8 && ph.eos ? sizeof(YShm<1>) : sizeof(YShm<0>), s, T, P,
+         ph, c);
 }
 
 template <class RT>
 void sweep_z(const Tables &T, const PlanesT<RT> &P, const Phys &ph, const SweepCtl &c, int ntop, cudaStream_t s) {
-  const int C = polar_cells(T.cz), n = tiles_z(T);
-  if constexpr (sizeof(RT) == 8) {
-    if (ph.eos) {
-      if (C == 3) launch(k_sweep_z<RT, 1, 3>, n, NT, sizeof(TileShm), s, T, P, ph, c, ntop);
-      else launch(k_sweep_z<RT, 1, 4>, n, NT, sizeof(TileShm), s, T, P, ph, c, ntop);
-      return;
-    }
-  }
-  if (C == 3) launch(k_sweep_z<RT, 0, 3>, n, NT, sizeof(TileShm), s, T, P, ph, c, ntop);
-  else launch(k_sweep_z<RT, 0, 4>, n, NT, sizeof(TileShm), s, T, P, ph, c, ntop);
+  const int C = polar_cells(T.cz);
+  launch(T.odd & 2 ? kernel_z<RT, true>(C, ph.eos) : kernel_z<RT, false>(C, ph.eos), tiles_z(T), NT, sizeof(TileShm), s, T, P, ph,
+         c, ntop);
 }
 
 template <class RT>

@@ -295,7 +295,9 @@ __device__ __forceinline__ double twice(double x, bool zero) {
 // an extremum has d1 and d2 of opposite sign and takes both zero; u2 < u1 is
 // |d2| > 2 |d1| and sets d2 = 2 d1; u2 < -u1 is |d1| > 2 |d2| and sets
 // d1 = 2 d2.  flat: whether a cell of the warp is flattened (W_OMF is set).
-template <int C>
+// ODD: some ghost cells hold no state (NaN), and the slopes beside them are
+// parabola's by its own comparisons (min3 of simple_func.cu:1-14).
+template <bool ODD, int C>
 __device__ __forceinline__ void edges(const Lane<C> &L, const double (&a)[C], const ParC<C> &k, bool flat, double (&d1)[C],
                                       double (&d2)[C]) {
   double dr[C], dl[C], t[C], tr[C], s[C];
@@ -304,10 +306,17 @@ __device__ __forceinline__ void edges(const Lane<C> &L, const double (&a)[C], co
   left_of<C>(dr, dl);
   PG_CELLS {
     const double x = fma(k.c3[c], dr[c], k.c4[c] * dl[c]);
-    double q = fabs(dl[c]) < fabs(dr[c]) ? fabs(dl[c]) : fabs(dr[c]);
-    q = twice(q, opposite(dl[c], dr[c]));
-    q = fabs(x) < q ? fabs(x) : q;
-    t[c] = copysign(q, x);
+    if (ODD) {
+      const double l2 = 2.0 * fabs(dl[c]), r2 = 2.0 * fabs(dr[c]), q = fabs(x) < l2 ? fabs(x) : l2;
+      t[c] = r2 < q ? r2 : q;
+      t[c] = x < 0.0 ? -t[c] : t[c];
+      if (dl[c] * dr[c] < 0.0) t[c] = 0.0;
+    } else {
+      double q = fabs(dl[c]) < fabs(dr[c]) ? fabs(dl[c]) : fabs(dr[c]);
+      q = twice(q, opposite(dl[c], dr[c]));
+      q = fabs(x) < q ? fabs(x) : q;
+      t[c] = copysign(q, x);
+    }
   }
   right_of<C>(t, tr);
   PG_CELLS s[c] = fma(k.c0[c], dr[c], fma(k.c1[c], tr[c], k.c2[c] * t[c]));
@@ -336,12 +345,13 @@ __device__ __forceinline__ void edges(const Lane<C> &L, const double (&a)[C], co
 // Planet (and star) acceleration along the radius (forces.cu:185-264): radius
 // x and 1/x, cf = cos(phi - phi_p) sin(theta), angular momentum v and w = r
 // v_theta
-template <bool THREED>
+template <bool THREED, bool ODD>
 __device__ __forceinline__ double force_r(double x, double ix, double cf, double v, double w, const PlanetC &P, int plnt,
                                           double isp2) {
   double t = v * v;
   if (THREED) t = fma(w, w, t * isp2);
-  const double f = (ix * ix) * fma(ix, t, -P.star);
+  // ODD: a ghost face at radius 0 has no force (inf - inf), as the reference's terms
+  const double f = ODD ? t * (ix * ix * ix) - P.star * (ix * ix) : (ix * ix) * fma(ix, t, -P.star);
   if (!plnt) return f;
   const double xc = P.x * cf;
   const double y = rsq(fma(x, fma(-2.0, xc, x), P.b2));
@@ -443,7 +453,7 @@ static __device__ __noinline__ double2 riemann_isen(double pl, double rl, double
 // 6 <= n < lim - 6 hold the remapped values, the others the Lagrangian ones,
 // which is what the viscosity's stencil reads at the chunk's ends
 // (remap.cu:94, viscosity.cu:370-472).  All lanes of the warp call it.
-template <int AXIS, bool THREED, int EOS, int C>
+template <int AXIS, bool THREED, int EOS, bool ODD, int C>
 __device__ __forceinline__ void warp_chain(const Lane<C> &L, const PlanetC &P, const Phys &ph, const double (&cs)[C]) {
   constexpr bool PAR_P = !(AXIS == 1 && EOS == 0);      // p has a parabola of its own
   const int lim = L.lim;
@@ -480,7 +490,7 @@ __device__ __forceinline__ void warp_chain(const Lane<C> &L, const PlanetC &P, c
       const double small = PAR_P ? kSmallp : kSmallp / L.cs2;
       PG_CELLS {
         const double m = pr[c] < pl[c] ? pr[c] : pl[c];
-        const bool shock = fabs(pr[c] - pl[c]) > 0.33 * m && !(ul[c] < ur[c]) && L.in(c, 2, 2);
+        const bool shock = fabs(pr[c] - pl[c]) > 0.33 * m && m >= 0.0 && !(ul[c] < ur[c]) && L.in(c, 2, 2);
         double dp2 = prr[c] - pll[c];
         if (fabs(dp2) < small) dp2 = small;
         const double x = ((pr[c] - pl[c]) / dp2 - 0.75) * 5.0;
@@ -516,7 +526,7 @@ __device__ __forceinline__ void warp_chain(const Lane<C> &L, const PlanetC &P, c
       for (int f = PAR_P ? 0 : 1; f < 3; f++) {
         double a[C], d1[C], d2[C], e[C];
         get<C>(L, f == 0 ? (int)W_P : f == 1 ? (int)W_R : (int)W_U, a);
-        edges<C>(L, a, k, flat, d1, d2);
+        edges<ODD, C>(L, a, k, flat, d1, d2);
         PG_CELLS {
           const double d = d1[c] + d2[c], a6 = 3.0 * (d2[c] - d1[c]), fac = fma(-kFourthd, cs[c], 1.0);
           e[c] = a[c] + fma(-cs[c], fma(-fac, a6, d), d1[c]);          // at the right face
@@ -544,7 +554,7 @@ __device__ __forceinline__ void warp_chain(const Lane<C> &L, const PlanetC &P, c
         get<C>(L, W_W, w);
         left_of<C>(w, wl);
       }
-      PG_CELLS f[c] = force_r<THREED>(x[c], ix[c], fma(L.c0, ch[c], -(L.s0 * sh[c])), 0.5 * (v[c] + vl[c]),
+      PG_CELLS f[c] = force_r<THREED, ODD>(x[c], ix[c], fma(L.c0, ch[c], -(L.s0 * sh[c])), 0.5 * (v[c] + vl[c]),
                                       THREED ? 0.5 * (w[c] + wl[c]) : 0.0, P, ph.plnt, L.isp2);
     } else if (AXIS == 1) {
       PG_CELLS f[c] = 0.0;
@@ -646,8 +656,8 @@ __device__ __forceinline__ void warp_chain(const Lane<C> &L, const PlanetC &P, c
       PG_CELLS {
         const double s = 2.0 * sh[c] * ch[c], k = fma(-2.0 * sh[c], sh[c], 1.0);    // the change in dt
         const double xn = fma(0.5, dx[c], xa[c]), wc = THREED ? w[c] : 0.0;
-        f1[c] = force_r<THREED>(xc[c], ixc[c], L.c0, v[c], wc, P, ph.plnt, L.isp2);
-        f2[c] = force_r<THREED>(xn, rcp(xn), fma(L.c0, k, -(L.s0 * s)), v[c], wc, P, ph.plnt, L.isp2);
+        f1[c] = force_r<THREED, ODD>(xc[c], ixc[c], L.c0, v[c], wc, P, ph.plnt, L.isp2);
+        f2[c] = force_r<THREED, ODD>(xn, rcp(xn), fma(L.c0, k, -(L.s0 * s)), v[c], wc, P, ph.plnt, L.isp2);
         const double d = xa[c] - xf[c];
         const double xe = L.n(c) < lim - 3 ? xa[c] : xf[c];         // the last face keeps its start (evolve.cu:36-44)
         if (!THREED) {
@@ -784,7 +794,7 @@ __device__ __forceinline__ void warp_chain(const Lane<C> &L, const PlanetC &P, c
     const int slot = (AXIS == 1 && !THREED && f == 2) ? (int)W_W : f;
     double a[C], d1[C], d2[C], al[C], l1[C], l2[C], fl[C], fr[C];
     get<C>(L, slot, a);
-    edges<C>(L, a, k, flat, d1, d2);
+    edges<ODD, C>(L, a, k, flat, d1, d2);
     left_of<C>(a, al);
     left_of<C>(d1, l1);
     left_of<C>(d2, l2);

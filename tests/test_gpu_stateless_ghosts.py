@@ -1,0 +1,104 @@
+"""Grids so coarse that ghost rings lie at no positive radius, against the CPU
+oracle.  The profiles have no value there: ghost densities, pressures and
+velocities are NaN or negative, and what the first rings get depends on how each
+comparison of the reference treats those (fmin, min3, flatten's quotient).  Two
+steps; bound relative 1e-12 as for the other comparisons (a change of the input's
+last bit moves the oracle's results by at most 4e-14), with FP32 planes six
+roundings to 24 bits, 4e-7.  Members of a batch equal the run alone bit for bit."""
+import math
+
+import numpy as np
+import pytest
+
+import penguin_2_0_b200 as pg
+from tests._lockstep import OracleLoop, rel_linf
+
+CASES = [
+    dict(which=0, imax=6, jmax=123, visc_flag=0, p_beta=1.0, p_alpha=0.0, noise_amp=0.0),
+    dict(which=0, imax=7, jmax=122, p_beta=0.5),
+    dict(which=0, imax=9, jmax=130, p_beta=0.0, visc_flag=0, plnt_flag=0),
+    dict(which=0, imax=33, jmax=123, EOS=1, gam=1.4, p_beta=0.0, noise_amp=0.6, grspx=6, dx_min=0.5 / 33, dx_max=3.0 / 33,
+         dz_min=0.5 / 33, dz_max=3.0 / 33),
+    dict(which=1, imax=6, jmax=122, kmax=33, ntop=3, visc_flag=0, p_alpha=0.0, p_beta=0.5, noise_amp=0.9),
+    dict(which=1, imax=20, jmax=122, kmax=6, EOS=1, gam=3.0, sc_h=0.15, flat_flag=0, visc_flag=0, grspx=4, dx_min=0.025,
+         dx_max=0.15, dz_min=0.025, dz_max=0.15),
+    # ghost layers beyond the axis
+    dict(which=1, imax=12, jmax=125, kmax=6, visc_flag=0, p_alpha=0.0, p_beta=1.0, sc_h=0.2, zmin=0.74, noise_amp=0.3),
+    dict(which=1, imax=21, jmax=124, kmax=8, ntop=3, EOS=1, gam=1.1, p_alpha=0.0, p_beta=0.0, sc_h=0.6, zmin=0.59, plnt_flag=0),
+    dict(which=1, imax=7, jmax=122, kmax=7, ntop=3, visc_flag=0, p_alpha=0.5, p_beta=0.5, noise_amp=0.6, precision=1),
+]
+
+
+def _params(case):
+    c = dict(case)
+    return pg.params(c.pop("which"), nprin=1, endtime=1e6, tmovie=1e6, **c)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", CASES, ids=range(len(CASES)))
+def test_rings_beside_ghosts_without_a_state(gpu, case):
+    p = _params(case)
+    tol = 4e-7 if p.precision else 1e-12
+    ic = pg.build_ic(p)
+    ref = OracleLoop(p, ic)
+    got = []
+    with pg.Run(p, 0) as run:
+        run.load(ic)
+        run.kernel_loop(2, record=lambda s, t, dt, pl, fr: got.append((dt, pg.dump_fields(run.save(), p))))
+        run.load(ic)
+        run.clock_reset(0)
+        assert run.advance(2) == 2
+        loop = pg.dump_fields(run.save(), p)
+    for gdt, g in got:
+        dt, _, _ = ref.step()
+        f = ref.fields()
+        speed = max(np.max(np.abs(f[k])) for k in "uvw")
+        for h in (g, loop) if g is got[-1][1] else (g,):
+            np.testing.assert_array_equal(h["rot_j"], f["rot_j"])
+            assert rel_linf(h["r"], f["r"]) <= tol
+            assert max(np.max(np.abs(h[k] - f[k])) / speed for k in "uvw") <= tol
+        assert abs(gdt - dt) <= tol * dt
+
+
+@pytest.mark.gpu
+def test_batch_member_with_such_ghosts(gpu):
+    cases = [CASES[1], dict(which=0, imax=72, jmax=150)]
+    params = [_params(c) for c in cases]
+    ics = [pg.build_ic(p) for p in params]
+    alone, together = [], [pg.Run(p, 0).load(ic) for p, ic in zip(params, ics)]
+    for p, ic in zip(params, ics):
+        with pg.Run(p, 0) as r:
+            r.load(ic)
+            r.clock_reset(0)
+            r.advance(6)
+            alone.append(bytes(r.save()))
+    with pg.Batch(0) as b:
+        for r in together:
+            r.clock_reset(0)
+            b.add(r)
+        b.advance(6, chunk=2)
+        b.sync()
+        for r in together:
+            b.remove(r)
+    assert [bytes(r.save()) for r in together] == alone
+    for r in together:
+        r.close()
+
+
+@pytest.mark.gpu
+def test_a_graph_follows_the_loaded_grid(gpu):
+    """A dump brings its own grid: of two with the same sizes, one has such ghosts."""
+    a = pg.params(0, imax=8, jmax=122, endtime=1e6, tmovie=1e6, kill_rin=0.0, kill_rout=0.0)
+    b = pg.params(0, imax=8, jmax=122, xmin=2.0, xmax=2.4, endtime=1e6, tmovie=1e6, kill_rin=0.0,
+                  kill_rout=0.0)
+    ics = [pg.build_ic(p) for p in (a, b)]
+    with pg.Run(a, 0) as r:
+        for ic in (ics[0], ics[1], ics[0]):
+            r.load(ic)
+            r.clock_reset(0)
+            r.advance(5, graph_chunk=2)
+            with pg.Run(a, 0) as f:
+                f.load(ic)
+                f.clock_reset(0)
+                f.advance(5)
+                assert bytes(r.save()) == bytes(f.save())
