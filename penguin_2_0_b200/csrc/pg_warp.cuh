@@ -490,7 +490,8 @@ __device__ __forceinline__ void warp_chain(const Lane<C> &L, const PlanetC &P, c
       const double small = PAR_P ? kSmallp : kSmallp / L.cs2;
       PG_CELLS {
         const double m = pr[c] < pl[c] ? pr[c] : pl[c];
-        const bool shock = fabs(pr[c] - pl[c]) > 0.33 * m && m >= 0.0 && !(ul[c] < ur[c]) && L.in(c, 2, 2);
+        // velocities that the limiter left at 1e-308 for zero are equal
+        const bool shock = fabs(pr[c] - pl[c]) > 0.33 * m && m >= 0.0 && !(ul[c] + 1.0e-290 < ur[c]) && L.in(c, 2, 2);
         double dp2 = prr[c] - pll[c];
         if (fabs(dp2) < small) dp2 = small;
         const double x = ((pr[c] - pl[c]) / dp2 - 0.75) * 5.0;
