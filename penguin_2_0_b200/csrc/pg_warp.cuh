@@ -295,8 +295,8 @@ __device__ __forceinline__ double twice(double x, bool zero) {
 // an extremum has d1 and d2 of opposite sign and takes both zero; u2 < u1 is
 // |d2| > 2 |d1| and sets d2 = 2 d1; u2 < -u1 is |d1| > 2 |d2| and sets
 // d1 = 2 d2.  flat: whether a cell of the warp is flattened (W_OMF is set).
-// ODD: some ghost cells hold no state (NaN), and the slopes beside them are
-// parabola's by its own comparisons (min3 of simple_func.cu:1-14).
+// ODD: some ghost cells hold no state (NaN, or beyond 1e154), and the slopes beside
+// them are parabola's by its own comparisons (min3 of simple_func.cu:1-14).
 template <bool ODD, int C>
 __device__ __forceinline__ void edges(const Lane<C> &L, const double (&a)[C], const ParC<C> &k, bool flat, double (&d1)[C],
                                       double (&d2)[C]) {
@@ -335,6 +335,13 @@ __device__ __forceinline__ void edges(const Lane<C> &L, const double (&a)[C], co
   }
   PG_CELLS {
     const double x1 = d1[c], x2 = d2[c];
+    if (ODD) {
+      const double j = x1 + x2, jj = j * j, j6 = j * (3.0 * (x2 - x1));
+      if (x1 * x2 <= 0.0) d1[c] = d2[c] = 0.0;
+      if (jj < j6) d2[c] = 2.0 * d1[c];
+      if (jj < -j6) d1[c] = 2.0 * d2[c];
+      continue;
+    }
     const bool ext = opposite(x1, x2);
     const double y1 = twice(x1, ext), y2 = twice(x2, ext);
     d1[c] = fabs(x1) > fabs(y2) ? y2 : x1;
@@ -350,8 +357,10 @@ __device__ __forceinline__ double force_r(double x, double ix, double cf, double
                                           double isp2) {
   double t = v * v;
   if (THREED) t = fma(w, w, t * isp2);
-  // ODD: a ghost face at radius 0 has no force (inf - inf), as the reference's terms
-  const double f = ODD ? t * (ix * ix * ix) - P.star * (ix * ix) : (ix * ix) * fma(ix, t, -P.star);
+  // ODD: a ghost face at radius 0 has no force (inf - inf), as the reference's terms;
+  // without a planet its 2D star pulls towards radius 0 from either side
+  const double i2 = ODD && !THREED && !plnt ? ix * fabs(ix) : ix * ix;
+  const double f = ODD ? t * (ix * ix * ix) - P.star * i2 : i2 * fma(ix, t, -P.star);
   if (!plnt) return f;
   const double xc = P.x * cf;
   const double y = rsq(fma(x, fma(-2.0, xc, x), P.b2));

@@ -22,6 +22,9 @@ CASES = [
     dict(which=1, imax=6, jmax=122, kmax=33, ntop=3, visc_flag=0, p_alpha=0.0, p_beta=0.5, noise_amp=0.9),
     dict(which=1, imax=20, jmax=122, kmax=6, EOS=1, gam=3.0, sc_h=0.15, flat_flag=0, visc_flag=0, grspx=4, dx_min=0.025,
          dx_max=0.15, dz_min=0.025, dz_max=0.15),
+    dict(which=0, imax=36, jmax=232, plnt_flag=0, FrRot_flag=0, visc_flag=0, p_alpha=0.5, p_beta=1.0, sc_h=0.03, noise_amp=0.9,
+         grspx=6, dx_min=0.5 / 36, dx_max=3.0 / 36, dz_min=0.5 / 36, dz_max=3.0 / 36, seed=423789),
+    dict(which=1, imax=6, jmax=122, kmax=8, zmin=1.2425, p_alpha=1.0, p_beta=0.0, sc_h=0.2, R_p=1.3, M_p=1e-6, FARGO_flag=1),
     # ghost layers beyond the axis
     dict(which=1, imax=12, jmax=125, kmax=6, visc_flag=0, p_alpha=0.0, p_beta=1.0, sc_h=0.2, zmin=0.74, noise_amp=0.3),
     dict(which=1, imax=21, jmax=124, kmax=8, ntop=3, EOS=1, gam=1.1, p_alpha=0.0, p_beta=0.0, sc_h=0.6, zmin=0.59, plnt_flag=0),
