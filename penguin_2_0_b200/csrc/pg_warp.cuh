@@ -418,6 +418,10 @@ __device__ __forceinline__ bool riemann_near(double a, double b, double s, doubl
 // a double's high word as an integer grows with it; kTiny: that of 1e-14, an
 // order of magnitude above the bounds kSmallp and kSmallr
 constexpr int kTiny = 0x3d06849b;
+// x above kSmallr (by its high word: false from 1e-15 (1 + 1e-6) down, and for what is not finite)
+__device__ __forceinline__ bool above_bound(double x) {
+  return (unsigned)(__double2hiint(x) - 0x3cd203b0) < 0x7ff00000u - 0x3cd203b0u;
+}
 
 // Isentropic Riemann problem (riemann.cu:75-111): van Leer's (1979) Newton
 // iteration for the contact pressure, at most 10 passes, relative tolerance
@@ -741,19 +745,24 @@ __device__ __forceinline__ void warp_chain(const Lane<C> &L, const PlanetC &P, c
     get<C>(L, W_U, u);
     right_of<C>(pm, pr);
     if (AXIS != 1) right_of<C>(vf, vr);
+    bool low = false;                     // a density below its bound: an emptied cell, or one whose faces crossed
     PG_CELLS {
       const double dm = dt * ivol[c] * (AXIS == 0 ? 1.0 : L.irad) * rcp(r[c]);     // dt / (r dvol0)
       double a = dm * (pr[c] - pm[c]);
       if (AXIS != 1) a *= 0.5 * (vr[c] + vf[c]);
       u[c] = u[c] + fma(hdt, f1[c] + f2[c], -a);
-      // the cell's mass, which the Lagrangian step keeps but for a density that
-      // the bound replaces (an emptied cell, or one whose faces crossed): there
-      // it is the bound's times the moved volume (evolve.cu:137, remap.cu:94-99)
-      m[c] = r[c] * vol[c];
-      const double q = m[c] * rcp(dvol[c]);
-      const bool held = q > kSmallr;
-      r[c] = held ? q : kSmallr;
-      m[c] = held ? m[c] : kSmallr * dvol[c];
+      m[c] = r[c] * vol[c];               // the cell's mass, which the Lagrangian step keeps
+      r[c] = m[c] * rcp(dvol[c]);
+      low = low || (!above_bound(r[c]) && L.n(c) < lim - 3);
+    }
+    if (low) {
+      // the bound takes its place, and its mass is the bound's times the moved
+      // volume (evolve.cu:137, remap.cu:94-99)
+      PG_CELLS {
+        const bool held = r[c] > kSmallr;
+        m[c] = held ? m[c] : kSmallr * dvol[c];
+        r[c] = held ? r[c] : kSmallr;
+      }
     }
     put<C>(L, W_R, r);
     put<C>(L, W_U, u);

@@ -41,6 +41,7 @@ __global__ void k(int what, int n, const double *a, const double *b, const doubl
   }
   if (what == 5) q[i] = riemann_near(a[i], b[i], 1.0, c[i], d[i], e[i], o[i], p[i]);
   if (what == 6) o[i] = quot16((int)a[i], 65536 / (int)b[i] + 1);
+  if (what == 8) o[i] = above_bound(a[i]);
   if (what == 7) o[i] = quot40((int)a[i], (int)b[i], (1ull << 40) / (unsigned long long)b[i] + 1);
 }
 extern "C" int run(int what, int n, const double *const *in, double *const *out) {
@@ -161,3 +162,15 @@ def test_quotients_by_multiplication(device):
         a = np.maximum(q * d + off, 0)
         a = np.minimum(a, 2 ** 31 - 2)
         assert np.array_equal(device(7, a, d)[0], a // d)
+
+
+@pytest.mark.gpu
+def test_density_bound_by_its_high_word(device):
+    r = np.random.default_rng(6)
+    b = 1e-15
+    x = np.concatenate([_spread(r, 200000, -1000, 1000), b * (1 + r.uniform(-4e-6, 4e-6, 200000)), [b, np.nextafter(b, 0), np.nextafter(b, 1)]])
+    x = np.concatenate([x, -x])
+    got = device(8, x)[0]
+    assert np.all(x[got == 1] > b)                       # never where the bound replaces a density
+    assert np.all(x[got == 0] <= b * (1 + 2e-6))         # and not far above it does it ask for the exact look
+    assert np.all(device(8, np.array([0.0, -0.0, 5e-324, np.inf, -np.inf, np.nan, -np.nan]))[0] == 0)
