@@ -44,9 +44,7 @@ __device__ __forceinline__ double eos_p_rt(double r, double cs2, const Phys &ph)
 }
 
 // ---- star + planet gravity, forces.cu:23-182 (non-barycentric frame) ------
-// The *_cf forms take cosfac = cos(azi - (p.y + dt p.vy)) from the caller
-// (shared by the cells of a pencil at dt = 0); the arithmetic after it is
-// the same as in the forms that evaluate it.
+// as pg_noalloc.cu's sums take it; the sweeps' form is in pg_warp.cuh
 __device__ __forceinline__ double planet_cosfac(double azi, const Body &p, double dt) {
   return cos(azi - (p.y + dt * p.vy));
 }

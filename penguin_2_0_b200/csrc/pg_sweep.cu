@@ -26,15 +26,17 @@
 // instruction issue (pg_warp.cuh) at 2.2-2.4 of 4 per cycle and SM, FP64 pipe
 // 43-51 %, DRAM below 15 %.  Against one thread per cell, the chain through
 // shared memory and 22 CTA barriers per chunk:
-//   128x1024x32  radial 628 -> 265 us, azimuthal 554 -> 194, polar 698 -> 423
-//   1536x4608    radial 836 -> 345 us, azimuthal 906 -> 311
+//   128x1024x32  radial 628 -> 268 us, azimuthal 554 -> 194, polar 698 -> 422
+//   1536x4608    radial 836 -> 346 us, azimuthal 906 -> 312
 //   256x768      radial  46 ->  21 us, azimuthal  37 ->  21
 // Of the radial sweep's 162 M instructions on the 3D disk 26 M are the tile's
 // loads and stores and what they need, of the azimuthal one's 131 M 17 M, of
 // the polar one's 285 M some 55 M.
-// 4 warps per CTA, 4 CTAs per SM at 128 registers (some 100 bytes of spills):
-// 3 CTAs ran 2-13 % longer but on the smallest grids, 5 CTAs 5-25 %, 8 warps per
-// CTA 5 %, 16 warps 30 %.  Loading the tile in one go before the first use took
+// 4 warps per CTA, 4 CTAs per SM at 128 registers.  A thread reloads 44-96 bytes of
+// spills in the radial sweep, 120-160 in the azimuthal one, 24-32 in the polar one
+// with 3 cells per lane and 156-244 with 4, 284-320 in the batch's kernels, whose
+// tables are behind a pointer.  3 CTAs ran 2-13 % longer but on the smallest grids,
+// 5 CTAs 5-25 %, 8 warps per CTA 5 %, 16 warps 30 %.  Loading the tile in one go before the first use took
 // the radial sweep from 344 to 328 us, cutting the workspace from 11 to 9 slots
 // (which leaves L1 room for the axis tables) from 308 to 284, planet constants
 // from the clock and quotients by multiplication (tiles formed on the host) to
