@@ -55,6 +55,8 @@ struct pg_batch {
   cudaStream_t stream = nullptr;
   std::string err;
   std::vector<pg_run *> runs;      // in the order added
+  struct Anchor { int cur; int64_t ncycle; };
+  std::vector<Anchor> anchors;     // per run: plane copy and step count when it was added
   Group g[2];                      // 2D members: FP64, FP32
   std::vector<pg_run *> solo;      // members with their own step sequence
   bool dirty = true;
@@ -181,6 +183,35 @@ static int enqueue_batch_step(pg_batch *b, bool first, bool last, int64_t *nk) {
   return PG_OK;
 }
 
+static int steps_of(pg_batch *b, pg_run *run, int64_t *n) {
+  long long c;
+  BK(cudaMemcpy(&c, &pgi::run_clock(run)->ncycle, sizeof(c), cudaMemcpyDeviceToHost));
+  *n = c;
+  return PG_OK;
+}
+// The plane copy that holds member i's state, once the stream is done: a 3D step swaps
+// the copies, and one that was queued behind the member's halt does not.
+static int settle(pg_batch *b, size_t i) {
+  pgi::RunShape sh;
+  pgi::run_shape(b->runs[i], &sh);
+  if (sh.ndim != 3) return PG_OK;
+  int64_t n;
+  if (int e = steps_of(b, b->runs[i], &n)) return e;
+  pgi::run_set_cur(b->runs[i], b->anchors[i].cur ^ (int)((n - b->anchors[i].ncycle) & 1));
+  return PG_OK;
+}
+static void drop_member(pg_batch *b, size_t i) {
+  pgi::run_set_batch(b->runs[i], nullptr);
+  b->runs.erase(b->runs.begin() + i);
+  b->anchors.erase(b->anchors.begin() + i);
+  b->dirty = true;
+}
+static int settle(pg_batch *b) {
+  for (size_t i = 0; i < b->runs.size(); i++)
+    if (int e = settle(b, i)) return e;
+  return PG_OK;
+}
+
 // count of halted members, read back through pinned memory
 static int snapshot(pg_batch *b) {
   int n = (int)b->runs.size();
@@ -221,6 +252,8 @@ int pg_batch_destroy(pg_batch *b) {
   if (!b) return PG_OK;
   cudaSetDevice(b->dev);
   if (b->stream) cudaStreamSynchronize(b->stream);
+  settle(b);
+  for (pg_run *r : b->runs) pgi::run_set_batch(r, nullptr);
   drop_graph(b);
   for (auto &g : b->g) {
     cudaFree(g.d_runs);
@@ -249,7 +282,11 @@ int pg_batch_add(pg_batch *b, pg_run *run) {
     return bfail(b, PG_ERR_ARG, "run is already in the batch");
   BK(cudaSetDevice(b->dev));
   BK(cudaStreamSynchronize(pgi::run_stream(run)));
+  int64_t n;
+  if (int e = steps_of(b, run, &n)) return e;
   b->runs.push_back(run);
+  b->anchors.push_back({pgi::run_cur(run), n});
+  pgi::run_set_batch(run, b);
   b->dirty = true;
   return PG_OK;
 }
@@ -260,8 +297,8 @@ int pg_batch_remove(pg_batch *b, pg_run *run) {
   if (it == b->runs.end()) return bfail(b, PG_ERR_ARG, "run is not in the batch");
   BK(cudaSetDevice(b->dev));
   BK(cudaStreamSynchronize(b->stream));
-  b->runs.erase(it);
-  b->dirty = true;
+  if (int e = settle(b, it - b->runs.begin())) return e;
+  drop_member(b, it - b->runs.begin());
   return PG_OK;
 }
 
@@ -271,7 +308,7 @@ int pg_batch_sync(pg_batch *b) {
   if (!b) return PG_ERR_ARG;
   BK(cudaSetDevice(b->dev));
   BK(cudaStreamSynchronize(b->stream));
-  return PG_OK;
+  return settle(b);
 }
 
 int pg_batch_advance(pg_batch *b, int nsteps, int chunk) {
@@ -356,6 +393,7 @@ int pg_batch_status(pg_batch *b, pg_batch_member *out, int n) {
     if (int e = rebuild(b)) return e;
   if (int e = snapshot(b)) return e;
   BK(cudaStreamSynchronize(b->stream));
+  if (int e = settle(b)) return e;
   int m = std::min(n, (int)b->runs.size());
   for (int i = 0; i < m; i++) out[i] = b->h_status[i];
   return PG_OK;
@@ -428,3 +466,12 @@ int64_t pg_batch_launch_count(const pg_batch *b) { return b ? b->launches : 0; }
 void *pg_batch_stream(const pg_batch *b) { return b ? (void *)b->stream : nullptr; }
 
 }  // extern "C"
+
+namespace pgi {
+void batch_forget(pg_batch *b, pg_run *run) {
+  auto it = std::find(b->runs.begin(), b->runs.end(), run);
+  if (it == b->runs.end()) return;
+  cudaStreamSynchronize(b->stream);
+  drop_member(b, it - b->runs.begin());
+}
+}  // namespace pgi

@@ -35,6 +35,10 @@ cudaError_t device_malloc(int dev, void **p, size_t bytes);
 pgd::DevClock *run_clock(pg_run *run);
 // which of the two plane copies is current (3D steps flip it)
 int run_cur(const pg_run *run);
+void run_set_cur(pg_run *run, int cur);
+// The batch a run is in (null: none), which is told when the run is destroyed.
+void run_set_batch(pg_run *run, pg_batch *b);
+void batch_forget(pg_batch *b, pg_run *run);
 cudaStream_t run_stream(pg_run *run);
 
 }  // namespace pgi

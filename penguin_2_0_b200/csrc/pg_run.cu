@@ -61,6 +61,7 @@ struct pg_run {
   bool clock_ready = false;
   bool counted = false;            // among its device's runs (stage_runs)
   int64_t launches = 0;
+  pg_batch *batch = nullptr;       // the batch it is in
   // captured step graphs
   cudaGraphExec_t gexec = nullptr;
   int gsteps = 0;
@@ -470,6 +471,7 @@ static int create(const pg_params *p, int device, pg_run **out) {
 int pg_destroy(pg_run *run) {
   if (!run) return PG_OK;
   cudaSetDevice(run->dev);
+  if (run->batch) pgi::batch_forget(run->batch, run);
   if (run->stream) cudaStreamSynchronize(run->stream);
   if (run->gexec) cudaGraphExecDestroy(run->gexec);
   for (auto e : run->ev_pool) cudaEventDestroy(e);
@@ -1090,10 +1092,13 @@ struct HaltProbe {
   }
 };
 
-static int finish_advance(pg_run *run, int64_t before, int *taken) {
+// cur0: the plane copy that was current at the call's start
+static int finish_advance(pg_run *run, int64_t before, int cur0, int *taken) {
   pgd::DevClock c;
   if (int e = read_clock(run, &c)) return e;
   run->ncycle = c.ncycle;
+  // a 3D step swaps the plane copies, one that was queued behind the halt does not
+  if (run->P.ndim == 3) run->cur = cur0 ^ (int)((c.ncycle - before) & 1);
   if (taken) *taken = (int)(c.ncycle - before);
   if (c.status != 0) {
     return fail(run, c.status, c.status == PG_ERR_NONFINITE ? "non-finite or non-positive state"
@@ -1114,6 +1119,7 @@ int pg_advance(pg_run *run, int nsteps, int *taken) {
   CK(cudaSetDevice(run->dev));
   int64_t before;
   if (int e = steps_before(run, &before)) return e;
+  const int cur_before = run->cur;
   HaltProbe hp{run};
   if (int e = hp.init()) return fail(run, e, "halt probe set-up");
   const int group = 16;
@@ -1123,7 +1129,7 @@ int pg_advance(pg_run *run, int nsteps, int *taken) {
     run->p0_live = false;
     if ((i + 1) % group == 0 && hp.post()) return fail(run, PG_ERR_CUDA, "halt probe");
   }
-  return finish_advance(run, before, taken);
+  return finish_advance(run, before, cur_before, taken);
 }
 
 int pg_advance_graph(pg_run *run, int nsteps, int chunk, int *taken) {
@@ -1134,6 +1140,7 @@ int pg_advance_graph(pg_run *run, int nsteps, int chunk, int *taken) {
   if (run->P.ndim == 3 && (chunk & 1)) chunk += 1;   // 3D steps alternate the plane copies
   int64_t before;
   if (int e = steps_before(run, &before)) return e;
+  const int cur_before = run->cur;
   int done = 0;
   if (run->p0_live && nsteps > 0) {
     if (int e = enqueue_step(run, true, true, true)) return e;
@@ -1176,7 +1183,7 @@ int pg_advance_graph(pg_run *run, int nsteps, int chunk, int *taken) {
   for (bool first = true; done < nsteps; done++, first = false) {
     if (int e = enqueue_step(run, false, first, done == nsteps - 1)) return e;
   }
-  return finish_advance(run, before, taken);
+  return finish_advance(run, before, cur_before, taken);
 }
 
 int pg_timing(pg_run *run, int on) {
@@ -1349,6 +1356,8 @@ int run_enqueue_on(pg_run *run, cudaStream_t s, bool first, bool last, int64_t *
 cudaError_t device_malloc(int dev, void **p, size_t bytes) { return dev_malloc(dev, p, bytes); }
 pgd::DevClock *run_clock(pg_run *run) { return run->clk; }
 int run_cur(const pg_run *run) { return run->cur; }
+void run_set_cur(pg_run *run, int cur) { run->cur = cur; }
+void run_set_batch(pg_run *run, pg_batch *b) { run->batch = b; }
 cudaStream_t run_stream(pg_run *run) { return run->stream; }
 
 }  // namespace pgi
