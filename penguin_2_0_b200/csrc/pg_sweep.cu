@@ -427,7 +427,7 @@ struct Finish {
       return;
     }
     o = T.ro[rk];
-    if (o.f > 0.0) {
+    if (o.f != 0.0) {
       tr = T.val_r[rk]; tu = T.val_u[rk]; tv = T.val_v[rk];
     }
     cs2 = T.cs2[rk];
@@ -440,7 +440,7 @@ struct Finish {
     RT sr = store_r<RT>(r, bs), su = (RT)u, sv = store_r<RT>(v, bv), sw = (RT)w;
     double rate = 0.0;
     if (ctl.fuse) {
-      if (o.f > 0.0) {
+      if (o.f != 0.0) {
         sr = store_r<RT>(damped(load_r(sr, bs), tr, o.f), bs);
         su = (RT)damped((double)su, tu, o.f);
         sv = store_r<RT>(damped(load_r(sv, bv), tv, o.f), bv);
