@@ -569,7 +569,7 @@ __device__ __forceinline__ void warp_chain(const Lane<C> &L, const PlanetC &P, c
         left_of<C>(w, wl);
       }
       PG_CELLS f[c] = force_r<THREED, ODD>(x[c], ix[c], fma(L.c0, ch[c], -(L.s0 * sh[c])), 0.5 * (v[c] + vl[c]),
-                                      THREED ? 0.5 * (w[c] + wl[c]) : 0.0, P, ph.plnt, L.isp2);
+                                           THREED ? 0.5 * (w[c] + wl[c]) : 0.0, P, ph.plnt, L.isp2);
     } else if (AXIS == 1) {
       PG_CELLS f[c] = 0.0;
       if (ph.plnt) {
